@@ -568,7 +568,7 @@ def gpu_arm(args):
                 "lf_choice": list(choice),
                 "lf_layout": {"passes_per_cta": lf_layout[0], "threads_per_cta": lf_layout[1],
                               "prefetch": bool(lf_layout[2]), "ctas_per_sm": lf_layout[3],
-                              "chosen_by": "autotune (timed on the first sweep of this picture shape)"},
+                              "chosen_by": "rule (picture size and candidates)"},
             },
             "e2e": {"value": round(e2e, 1), "unit": "MB/s", "h2d_bytes_per_step": int(ps.h2d),
                     "d2h_bytes_per_step": int(ps.d2h),
@@ -1088,7 +1088,7 @@ def batch_arm(args):
     # stage's algorithmic GB/s (per MB: ARNR 6 frames x 384 B in + 384 out;
     # analysis source 256 + 2 refs x 256 + decision 104; reconstruction
     # 1264; LF sweep 774 read once), with the launch shape the sweep's
-    # autotuner picked for that batch.
+    # rule picked for that batch.
     per_alg = {"arnr": (BATCH_LOOKAHEAD + 1) * 384, "analysis": 256 + 2 * 256 + 104, "recon": 1264, "lf": 774}
     per_res = {}
     del bs
@@ -1140,7 +1140,7 @@ def batch_arm(args):
             "warmup": args.warmup, "streams": args.streams, "mbs_per_step": n_mb, "per_resolution": per_res,
             "lf_layout_mixed": {"passes_per_cta": mixed_layout[0], "threads_per_cta": mixed_layout[1],
                                 "prefetch": bool(mixed_layout[2]), "ctas_per_sm": mixed_layout[3],
-                                "chosen_by": "autotune (timed on the first batch of these picture shapes)"},
+                                "chosen_by": "rule (picture sizes and candidates; the last launch of the batch)"},
             "stage_ms": stages, "step_ms": [round(x, 3) for x in ts],
             "config": {"workload": "%d streams from {176x144, 640x360, 1280x720, 1920x1080, 3840x2160}: "
                                    "P frame vs LAST/ALTREF, ARNR(5, centre), qi-44 reconstruction, LF 64x8 sweep"

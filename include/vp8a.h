@@ -268,11 +268,9 @@ uint64_t vp8a_ctx_launch_count(const vp8a_ctx* ctx);
  * hanging or faulting anything. Applies to calls issued after it. */
 vp8a_status vp8a_ctx_set_wait_limit(vp8a_ctx* ctx, uint64_t polls);
 /* No counterpart in the reference (launch shapes of the device kernels).
- * With autotune on (the default) the loop-filter sweep times every launch
- * shape that fits — passes per CTA, threads per CTA, next-MB prefetch — on
- * the first scored sweep of each picture shape and keeps the fastest for
- * that shape in the context (the first call takes longer); off, a cost
- * model picks. Results never depend on the shape. */
+ * The loop-filter sweep's launch shape follows rules on the picture's size
+ * and the number of candidates, so there is nothing left to time on a first
+ * call: accepted, and without effect. Results never depend on the shape. */
 vp8a_status vp8a_ctx_set_autotune(vp8a_ctx* ctx, uint32_t on);
 /* No counterpart in the reference. On, the inter analysis first builds
  * each reference's 16 quarter-pel sub-pel planes (every §18.3 sample at
@@ -299,7 +297,7 @@ vp8a_status vp8a_ctx_set_trellis_strength(vp8a_ctx* ctx, double strength);
  * VP8A_E_INVALID_ARGUMENT. */
 vp8a_status vp8a_ctx_force_sweep_layout(vp8a_ctx* ctx, uint32_t passes, uint32_t threads, uint32_t prefetch);
 /* The last sweep's launch shape: out[0] passes per CTA, out[1] threads per
- * CTA, out[2] prefetch, out[3] CTAs per SM (0: rings in global memory). */
+ * CTA, out[2] prefetch, out[3] CTAs per SM. */
 vp8a_status vp8a_ctx_last_sweep_layout(const vp8a_ctx* ctx, uint32_t out[4]);
 /* Text of the last error on this thread ("" if none). */
 const char* vp8a_last_error(void);
@@ -546,7 +544,7 @@ vp8a_status vp8a_filter_sweep(vp8a_ctx* ctx, const vp8a_planes* planes,
  *    `ssd_out`) must already be device memory of the context's GPU
  *    (VP8A_E_INVALID_ARGUMENT otherwise);
  *  - its scratch (candidate list and step schedule) is one fixed array of
- *    about 72 KiB compiled into the library, which every GPU that loads the
+ *    about 80 KiB compiled into the library, which every GPU that loads the
  *    library holds until the process exits; it bounds the picture to at most
  *    256 x 136 MBs (4096 x 2176 pixels), larger grids return
  *    VP8A_E_INVALID_DIMENSIONS;

@@ -6,7 +6,6 @@
 #include <array>
 #include <cstdint>
 #include <cstring>
-#include <map>
 #include <string>
 #include <vector>
 
@@ -36,12 +35,9 @@ struct vp8a_ctx {
   uint8_t* up_host = nullptr;
   cudaEvent_t up_ev[UP_SLOTS] = {};
   unsigned up_next = 0;
-  // Launch-shape choice of the loop-filter sweep: measured on first use
-  // per picture shape (autotune) or by the cost model; a forced layout
-  // (tests) overrides both. Cache: shape key -> (passes per CTA, threads,
-  // prefetch). last_layout: the last sweep's (passes, threads, prefetch,
-  // CTAs per SM).
-  bool autotune = true;
+  // The loop-filter sweep's launch shape is chosen by rule (lf.cu); a forced
+  // layout (tests) overrides it. last_layout: the last sweep's (passes per
+  // CTA, threads, prefetch, CTAs per SM).
   // The analysis reads its half- and quarter-pel predictions from planes
   // precomputed per call (vp8a_ctx_set_subpel_planes; off by default: the
   // SPLITMV warps, not the refinements, bound each MB's latency).
@@ -50,8 +46,6 @@ struct vp8a_ctx {
   // 0 = plain rounding).
   double trellis_strength = 0.0;
   int force_layout[3] = {0, 0, 0};
-  std::map<std::array<int64_t, 6>, std::array<int, 3>> lf_tuned;
-  std::map<std::vector<int64_t>, std::array<int, 3>> lf_tuned_batch;  // batched sweeps: job shapes -> layout
   int last_layout[4] = {0, 0, 0, 0};
 };
 

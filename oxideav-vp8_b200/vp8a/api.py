@@ -63,7 +63,7 @@ class Context:
         check(self._lib.vp8a_ctx_set_subpel_planes(self.handle, int(bool(on))), "vp8a_ctx_set_subpel_planes")
 
     def set_autotune(self, on):
-        """Measured (True, the default) or modelled launch shapes."""
+        """Accepted, without effect: the launch shapes follow rules."""
         check(self._lib.vp8a_ctx_set_autotune(self.handle, int(bool(on))), "vp8a_ctx_set_autotune")
 
     def force_sweep_layout(self, passes, threads=0, prefetch=0):
