@@ -9,24 +9,34 @@
 // census record feeds later MBs.
 //
 // Scheduling. The census makes MB (r, c) depend on (r, c-1), (r-1, c) and
-// (r-1, c-1); the reference's wavefront lets row r run while row r-1 is two
-// MBs ahead (src/encoder/inter.rs:376-379). Here a persistent grid of
-// co-resident CTAs owns MB rows round-robin; a CTA processes its rows left
-// to right and, before MB (r, c), waits until row r-1 has published
-// min(c+2, mb_cols) MBs. Rows are claimed in increasing order and every
-// waited-on row belongs to a resident CTA, so the wait always ends; it is
-// still bounded, and a wait that runs out sets the device status word and
-// the whole grid returns (VP8A_E_DEVICE_TIMEOUT on the host).
+// (r-1, c-1). A persistent grid of co-resident clusters, one CTA a reference,
+// owns MB rows round-robin; a cluster takes its rows left to right, MB (r, c)
+// once row r-1 has published c + 1 MBs. Rows are claimed in increasing order
+// and every waited-on row belongs to a resident cluster, so the wait always
+// ends; it is still bounded, and a wait that runs out sets the device status
+// word and the whole grid returns (VP8A_E_DEVICE_TIMEOUT on the host).
 //
-// Per MB, one staging phase fetches (edge-clamped, all loads in flight
-// together) everything the searches read: per reference the search window
-// around the predictor, the NEAREST/NEAR six-tap halos and the 16x16
-// blocks at the ZERO and neighbour vectors. Then each reference gets one
-// "main" warp (ZEROMV, diamond, half via shared half-pel planes, quarter,
-// NEAREST, NEAR) and four SPLITMV warps (one per partition, groups in
-// parallel across lanes). The f64 RD decision runs on one thread with the
-// reference's operation order; the library is built with -fmad=false so no
-// multiply-add is fused.
+// What bounds it: the chain of mb_cols + mb_rows MB steps, each a chain of
+// short dependent stages in one CTA (at 1080p about 188 steps of 8 to 9 us).
+// So the work of a step is spread over the CTA's warps and whatever another
+// step can do is taken off the chain:
+//  - The helper warp fetches the source MB and the census record above two
+//    MBs ahead, polls the row above, and (rank 0's) writes the results out.
+//  - The references' decisions pass between the CTAs as asynchronous stores
+//    onto mbarriers; a cluster barrier costs 700 to 900 cycles each.
+//  - Warp 0 walks the census while warp 1 plans the SPLITMV columns. One
+//    staging phase fetches (edge-clamped, all loads in flight together)
+//    everything the searches read: the window around the predictor, the
+//    NEAREST/NEAR six-tap halos, the 16x16 blocks at the ZERO and neighbour
+//    vectors.
+//  - Five "main" warps compute all whole-pel SADs around the predictor as a
+//    field, walk it, and refine from shared half- and quarter-pel planes, two
+//    pixels a lane and instruction; four SPLITMV warps take one partition
+//    each (groups in parallel across lanes), then NEAREST and NEAR.
+// The f64 RD decision runs on one thread with the reference's operation order;
+// the library is built with -fmad=false so no multiply-add is fused.
+// Measured, before these stages were split and packed and now: 1080p with three
+// references 2.23 -> 1.67 ms, 176x144 with one 224 -> 166 us.
 #include <cooperative_groups.h>
 #include <algorithm>
 #include <cstddef>
@@ -90,8 +100,6 @@ struct __align__(16) RefSmem {
   uint8_t blocks[MAX_BLOCKS][256];      // read as 32-bit words (sad_block16)
 };
 static_assert(sizeof(RefSmem) % 16 == 0 && offsetof(RefSmem, blocks) % 16 == 0, "RefSmem alignment");
-static_assert(sizeof(WarpScratch) - offsetof(WarpScratch, temp) >= 3 * 22 * 16,
-              "the quarter-pel planes fit in the window's six-tap scratch");
 
 struct MainOut {
   uint32_t sad_zero, sad_nearest, sad_near;
@@ -125,33 +133,31 @@ struct SplitOut {
 // SPLITMV scratch of one warp. Candidate column layout (fixed, no
 // de-duplication): 0 = ZERO, 1..4 = LEFT vectors of the MB's left column
 // anchors 0/4/8/12, 5..8 = ABOVE vectors of the top-row anchors 0..3,
-// 9..24 = the NEW4X4 result of group 0..15. Aligned to 16 bytes with a
-// size that is a multiple of 16: every warp's copy moves table columns as
-// 16-byte vectors.
+// 9..24 = the NEW4X4 result of group 0..15.
 struct __align__(16) SplitScratch {
-  uint32_t table[CMAX * 16];  // group g's SAD at column m: table[m * 16 + g], needed columns only
-  double new_cost[16 * 5];    // lambda * (NEW4X4 mode bits of context x + group g's vector bits)
-  double terms[32];           // group g's reference bits [g] and NEW vector bits [16 + g], for the total
-  vp8a_mv cmv[CMAX];
+  double table[CMAX * 16];   // group g's SAD at column m: table[m * 16 + g], needed columns only
+  uint64_t zero_new[16 * 5]; // the cheaper of ZERO and NEW for group g in context x: J's bits
+  double terms[32];          // the total's terms in order
+  vp8a_mv cmv[16];           // the groups' NEW results (columns 9 + g)
 };
 static_assert(sizeof(SplitScratch) % 16 == 0, "SplitScratch copies stay 16-byte aligned");
 struct Plan {
   int wx0, wy0;        // window origin (plane pixels)
   int hn_x, hn_y;      // NEAREST halo origin
   int hr_x, hr_y;      // NEAR halo origin
+  // A zero NEAREST or NEAR vector is never a candidate of the decision, and
+  // its SAD (for the trace) is the ZERO vector's.
+  int want_nearest, want_near;
   int nblocks;
   int box[MAX_BLOCKS], boy[MAX_BLOCKS];  // block integer offsets
   int colblk[9];       // staged block of SPLITMV column m < 9 (ZERO, LEFT x4, ABOVE x4)
+  vp8a_mv colmv[9];    // and its vector
 };
 
 __device__ __forceinline__ int int_off(int16_t v) { return eighth(v) >> 3; }
 
-// External LEFT4X4 / ABOVE4X4 vectors (left_block_mv / above_block_mv for
-// anchors on the MB's left column / top row, src/near_mv.rs:722-760).
-__device__ __forceinline__ vp8a_mv ext_left(const MbInfoDev& l, int anchor) {
-  if (l.ref_frame == VP8A_REF_INTRA) return vp8a_mv{0, 0};
-  return l.is_split ? l.split_mvs[anchor + 3] : l.mv;
-}
+// External ABOVE4X4 vectors (above_block_mv for anchors on the MB's top row,
+// src/near_mv.rs:722-760).
 __device__ __forceinline__ vp8a_mv ext_above(const MbInfoDev& a, int anchor) {
   if (a.ref_frame == VP8A_REF_INTRA) return vp8a_mv{0, 0};
   return a.is_split ? a.split_mvs[anchor + 12] : a.mv;
@@ -160,16 +166,18 @@ __device__ __forceinline__ vp8a_mv ext_above(const MbInfoDev& a, int anchor) {
 // Stage this CTA's reference: every region row is copied as 32-bit words
 // (two aligned loads and a funnel shift per word); a word whose plane bytes
 // are not all inside the row — at the frame edges — is fetched byte by byte
-// with edge clamping. Each thread keeps up to 8 words in flight.
-__device__ void stage_ref(const MePlane& P, RefSmem& R, const Plan& pl, int mbx, int mby, bool words, int tid,
-                          int nthreads) {
+// with edge clamping. Each thread keeps up to 4 words in flight.
+__device__ __forceinline__ void stage_ref(const MePlane& P, RefSmem& R, const Plan& pl, int mbx, int mby, bool words,
+                                          int tid, int nthreads) {
   constexpr int N_WIN = 40 * 10, N_HALO = 21 * 6;
-  const int total = N_WIN + 2 * N_HALO + pl.nblocks * 64;
-  for (int base = tid; base < total; base += nthreads * 8) {
-    uint32_t v[8];
-    uint32_t* d[8];
+  const int b1 = N_WIN + (pl.want_nearest ? N_HALO : 0), b2 = b1 + (pl.want_near ? N_HALO : 0),
+            total = b2 + pl.nblocks * 64;
+#pragma unroll 1
+  for (int base = tid; base < total; base += nthreads * 4) {
+    uint32_t v[4];
+    uint32_t* d[4];
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
+    for (int j = 0; j < 4; j++) {
       const int e = base + j * nthreads;
       d[j] = nullptr;
       v[j] = 0;
@@ -182,15 +190,16 @@ __device__ void stage_ref(const MePlane& P, RefSmem& R, const Plan& pl, int mbx,
           x0 = pl.wx0;
           y0 = pl.wy0;
           dst = R.ws.win + row * WS;
-        } else if (e < N_WIN + 2 * N_HALO) {
-          const int q = e - N_WIN, h = q >= N_HALO, qq = q - h * N_HALO;
-          row = qq / 6;
-          word = qq - row * 6;
-          x0 = h ? pl.hr_x : pl.hn_x;
-          y0 = h ? pl.hr_y : pl.hn_y;
-          dst = (h ? R.halo_near : R.halo_nearest) + row * HS;
+        } else if (e < b2) {
+          const bool near = e >= b1;
+          const int q = e - (near ? b1 : N_WIN);
+          row = q / 6;
+          word = q - row * 6;
+          x0 = near ? pl.hr_x : pl.hn_x;
+          y0 = near ? pl.hr_y : pl.hn_y;
+          dst = (near ? R.halo_near : R.halo_nearest) + row * HS;
         } else {
-          const int q = e - N_WIN - 2 * N_HALO, b = q >> 6;
+          const int q = e - b2, b = q >> 6;
           row = (q >> 2) & 15;
           word = q & 3;
           x0 = mbx + pl.box[b];
@@ -211,7 +220,7 @@ __device__ void stage_ref(const MePlane& P, RefSmem& R, const Plan& pl, int mbx,
       }
     }
 #pragma unroll
-    for (int j = 0; j < 8; j++)
+    for (int j = 0; j < 4; j++)
       if (d[j]) *d[j] = v[j];
   }
 }
@@ -221,25 +230,30 @@ __device__ void stage_ref(const MePlane& P, RefSmem& R, const Plan& pl, int mbx,
 // Whole-pel SADs of every position within +-FR pixels of the search start
 // (the snapped, clamped best predictor), per 4x4 block: a group SAD of any
 // SPLITMV partition at such a position is the sum of its blocks, and the
-// 16x16 SAD the sum of all 16. Both diamonds (the MB's, at most 8 steps of
-// one pixel, and every SPLITMV group's, at most 4) stay inside the field,
-// so they become table walks; vectors outside it (ZERO, the neighbours'
-// vectors) are served by the staged blocks.
-constexpr int FR = 8, FN = 2 * FR + 1, FP = FN * FN;
+// 16x16 SAD the sum of all 16. Every SPLITMV group's diamond (four rounds of
+// one pixel) stays inside the field and becomes a table walk; the MB's own
+// (eight rounds) continues on the window when it reaches the field's edge.
+// Vectors outside the field (ZERO, the neighbours' vectors) are served by the
+// staged blocks. A field of +-8 for the rare long walks took 2.0 k cycles of
+// every MB, most of it absolute differences at half rate.
+constexpr int FR = 4, FN = 2 * FR + 1, FP = FN * FN;
 static_assert(WIN_LEAD - FR >= 0 && WIN_LEAD + FR + 16 <= WS, "the window covers the field");
 
 struct __align__(16) FieldSmem {
   uint16_t blk[FP][16];  // 4x4 block SADs at each position (raster block order)
   uint32_t full[FP];     // 16x16 SADs
   uint16_t grp[FP][8];   // TopBottom 0,1 | LeftRight 0,1 | Quarters 0..3
+  // A second field of 16x16 SADs, around where the MB's walk left the first.
+  uint16_t rows[16][FP];  // one source row each
+  uint32_t full2[FP];
 };
 
 __device__ __forceinline__ int fpos(int dx, int dy) {
   return (dx >= -FR && dx <= FR && dy >= -FR && dy <= FR) ? (dy + FR) * FN + dx + FR : -1;
 }
 
-// Block SADs: one thread per (block, row of positions); the 17 positions
-// of a row share each window row's six words.
+// Block SADs: one thread per (block, row of positions); the positions of a row
+// share each window row's words.
 __device__ __forceinline__ void field_blocks(const uint8_t* win, const uint8_t* src, FieldSmem& F, int tid) {
   if (tid >= 16 * FN) return;
   const int b = tid & 15, dyi = tid >> 4;
@@ -251,9 +265,10 @@ __device__ __forceinline__ void field_blocks(const uint8_t* win, const uint8_t* 
   for (int row = 0; row < 4; row++) {
     const uint32_t sw = *(const uint32_t*)(src + (by4 + row) * 16 + bx4);
     const uint32_t* w = (const uint32_t*)(win + (WIN_LEAD - FR + dyi + by4 + row) * WS + bx4);
-    uint32_t wd[6];
+    constexpr int NWD = (WIN_LEAD - FR + FN - 1 + 3) / 4 + 1;
+    uint32_t wd[NWD];
 #pragma unroll
-    for (int k = 0; k < 6; k++) wd[k] = w[k];
+    for (int k = 0; k < NWD; k++) wd[k] = w[k];
 #pragma unroll
     for (int dxi = 0; dxi < FN; dxi++) {
       constexpr int base = WIN_LEAD - FR;
@@ -287,17 +302,32 @@ __device__ __forceinline__ void field_sums(FieldSmem& F, int tid, int nthreads) 
   }
 }
 
-// 4x4 block SADs of the staged 16x16 blocks (ZERO and neighbour vectors).
-__device__ __forceinline__ void staged_block_sads(const RefSmem& R, const uint8_t* src, int nblocks,
-                                                  uint16_t (*xs)[16], int tid, int nthreads) {
-  for (int t = tid; t < nblocks * 16; t += nthreads) {
-    const int j = t >> 4, b = t & 15, bx4 = (b & 3) * 4, by4 = (b >> 2) * 4;
+// 4x4 block SADs of the staged 16x16 blocks (ZERO and neighbour vectors) and
+// their partition-group sums (the order of FieldSmem::grp): 16 lanes a block.
+struct __align__(16) BlockSads {
+  uint16_t blk[MAX_BLOCKS][16];
+  uint16_t grp[MAX_BLOCKS][8];
+};
+__device__ __forceinline__ void staged_block_sads(const RefSmem& R, const uint8_t* src, int nblocks, BlockSads& X,
+                                                  int tid, int nthreads) {
+  const int b = tid & 15, bx4 = (b & 3) * 4, by4 = (b >> 2) * 4;
+#pragma unroll 1
+  for (int j = tid >> 4; (j & ~1) < nblocks; j += nthreads >> 4) {  // warp-uniform
     uint32_t acc = 0;
+    if (j < nblocks)
 #pragma unroll
-    for (int row = 0; row < 4; row++)
-      acc += __vsadu4(*(const uint32_t*)(R.blocks[j] + (by4 + row) * 16 + bx4),
-                      *(const uint32_t*)(src + (by4 + row) * 16 + bx4));
-    xs[j][b] = (uint16_t)acc;
+      for (int row = 0; row < 4; row++)
+        acc += __vsadu4(*(const uint32_t*)(R.blocks[j] + (by4 + row) * 16 + bx4),
+                        *(const uint32_t*)(src + (by4 + row) * 16 + bx4));
+    uint32_t q = acc + __shfl_xor_sync(FULL, acc, 1);
+    q += __shfl_xor_sync(FULL, q, 4);  // the block's quarter
+    const uint32_t rows = q + __shfl_xor_sync(FULL, q, 2), cols = q + __shfl_xor_sync(FULL, q, 8);
+    if (j < nblocks) {
+      X.blk[j][b] = (uint16_t)acc;
+      if (b == 0 || b == 8) X.grp[j][b >> 3] = (uint16_t)rows;                         // TopBottom
+      if (b == 0 || b == 2) X.grp[j][2 + (b >> 1)] = (uint16_t)cols;                   // LeftRight
+      if ((b & 5) == 0) X.grp[j][4 + ((b >> 3) << 1) + ((b >> 1) & 1)] = (uint16_t)q;  // Quarters
+    }
   }
 }
 
@@ -329,13 +359,73 @@ __device__ __forceinline__ void walk_round(const uint32_t (&r)[9], int& dx, int&
   }
 }
 
+// The second field, by the main group's thread t of n: one (row of positions,
+// source row) a thread, then the rows' sums. (wx, wy): the window position of
+// the block at its centre, at least FR from the window's edges.
+__device__ __forceinline__ void field2_rows(const uint8_t* win, const uint8_t* src, FieldSmem& F, int wx, int wy,
+                                            int t) {
+  if (t >= 16 * FN) return;
+  const int row = t / FN, dyi = t - row * FN;
+  const uint4 sv = *(const uint4*)(src + row * 16);
+  const uint8_t* p = win + (wy - FR + dyi + row) * WS;
+  const int o = wx - FR;
+  uint32_t u[7];
+#pragma unroll
+  for (int k = 0; k < 7; k++) u[k] = ((const uint32_t*)(p + (o & ~3)))[k];
+  const unsigned sh = (unsigned)(o & 3) * 8u;
+#pragma unroll
+  for (int k = 0; k < 6; k++) u[k] = __funnelshift_r(u[k], u[k + 1], sh);
+  uint16_t* out = F.rows[row] + dyi * FN;
+#pragma unroll
+  for (int dx = 0; dx < FN; dx++) {
+    const int w = dx >> 2;
+    const unsigned b = (dx & 3) * 8u;
+    out[dx] = (uint16_t)(__vsadu4(__funnelshift_r(u[w], u[w + 1], b), sv.x) +
+                         __vsadu4(__funnelshift_r(u[w + 1], u[w + 2], b), sv.y) +
+                         __vsadu4(__funnelshift_r(u[w + 2], u[w + 3], b), sv.z) +
+                         __vsadu4(b ? __funnelshift_r(u[w + 3], u[w + 4 > 5 ? 5 : w + 4], b) : u[w + 3], sv.w));
+  }
+}
+__device__ __forceinline__ void field2_sums(FieldSmem& F, int t, int n) {
+#pragma unroll 1
+  for (; t < FP; t += n) {
+    uint32_t s = 0;
+#pragma unroll
+    for (int r = 0; r < 16; r++) s += F.rows[r][t];
+    F.full2[t] = s;
+  }
+}
+
+// Up to `rounds` rounds of the walk over a field of 16x16 SADs from (x, y), with
+// SAD bs, while the neighbourhood lies in the field; rounds becomes 0 when the
+// walk has ended.
+__device__ __forceinline__ void walk_field(const uint32_t* full, int& x, int& y, uint32_t& bs, int& rounds) {
+  for (; rounds > 0 && x > -FR && x < FR && y > -FR && y < FR; rounds--) {
+    const uint32_t* c0 = full + fpos(x, y);
+    const uint32_t r[9] = {c0[-FN - 1], c0[-FN], c0[-FN + 1], c0[-1], bs, c0[1], c0[FN - 1], c0[FN], c0[FN + 1]};
+    int dx, dy;
+    uint32_t b;
+    walk_round(r, dx, dy, b);
+    if (dx == 0 && dy == 0) {
+      rounds = 0;
+      return;
+    }
+    x += dx;
+    y += dy;
+    bs = b;
+  }
+}
+
 // small_diamond_search_luma (src/motion_search.rs:381-442) walked over the
 // field: N, S, W, E from the running best, strict '<', collapse skips, at
-// most max_iters rounds. Warp-uniform; a position outside the field (not
-// reachable from an in-range start) is computed from the plane.
+// most max_iters rounds. Warp-uniform. A walk that reaches the field's edge
+// returns with `rounds` rounds left, to be continued over the second field;
+// next to the +-1023 clamp every candidate is tried in turn, positions outside
+// the field computed from the plane.
 __device__ vp8a_search_result diamond_field(const FieldSmem& F, const MePlane& P, const uint8_t* win, int wx0,
                                             int wy0, int mbx, int mby, int cxp, int cyp, vp8a_mv center,
-                                            int max_iters, const uint8_t* src, int lane) {
+                                            int max_iters, const uint8_t* src, int lane, int& rounds) {
+  rounds = 0;
   auto sad = [&](vp8a_mv m) -> uint32_t {
     const int x = mbx + m.col / 4, y = mby + m.row / 4;
     const int p = fpos(x - cxp, y - cyp);
@@ -346,28 +436,12 @@ __device__ vp8a_search_result diamond_field(const FieldSmem& F, const MePlane& P
   best.col = snap_whole(clamp_component(center.col));
   const int x0 = mbx + best.col / 4 - cxp, y0 = mby + best.row / 4 - cyp;
   const int lim = 1020 - 4 * max_iters;
-  if (best.row >= -lim && best.row <= lim && best.col >= -lim && best.col <= lim && max_iters <= FR &&
-      x0 == 0 && y0 == 0) {
-    // No candidate of the walk is clamped and every round's neighbourhood
-    // lies in the field: read it whole, decide the round with selects.
+  if (best.row >= -lim && best.row <= lim && best.col >= -lim && best.col <= lim && x0 == 0 && y0 == 0) {
     int x = 0, y = 0;
     uint32_t bs = F.full[fpos(0, 0)];
-    for (int it = 0; it < max_iters; it++) {
-      const uint32_t* c0 = F.full + fpos(x, y);
-      const uint32_t r[9] = {c0[-FN - 1], c0[-FN], c0[-FN + 1], c0[-1], bs, c0[1], c0[FN - 1], c0[FN], c0[FN + 1]};
-      int dx, dy;
-      uint32_t b;
-      walk_round(r, dx, dy, b);
-      if (dx == 0 && dy == 0) break;
-      x += dx;
-      y += dy;
-      bs = b;
-    }
-    vp8a_search_result res;
-    res.mv.row = (int16_t)(best.row + 4 * y);
-    res.mv.col = (int16_t)(best.col + 4 * x);
-    res.sad = bs;
-    return res;
+    rounds = max_iters;
+    walk_field(F.full, x, y, bs, rounds);
+    return vp8a_search_result{vp8a_mv{(int16_t)(best.row + 4 * y), (int16_t)(best.col + 4 * x)}, bs};
   }
   uint32_t best_sad = sad(best);
   for (int it = 0; it < max_iters; it++) {
@@ -416,15 +490,6 @@ __constant__ uint16_t c_group_blocks[4][16] = {
     {0x0001, 0x0002, 0x0004, 0x0008, 0x0010, 0x0020, 0x0040, 0x0080, 0x0100, 0x0200, 0x0400, 0x0800, 0x1000,
      0x2000, 0x4000, 0x8000}};
 
-__device__ __forceinline__ uint32_t group_sum(const uint16_t* v16, int pid, int g) {
-  const uint32_t m = c_group_blocks[pid][g];
-  uint32_t s = 0;
-#pragma unroll
-  for (int b = 0; b < 16; b++)
-    if ((m >> b) & 1u) s += v16[b];
-  return s;
-}
-
 // A group's whole-pel SAD at pixel (x, y) computed from the plane with
 // edge clamping, by one lane (only for positions neither the field nor a
 // staged block covers).
@@ -447,7 +512,7 @@ __device__ uint32_t direct_group_sad(const MePlane& P, const uint8_t* src, int x
 
 struct FieldView {
   const FieldSmem* F;
-  const uint16_t (*xs)[16];
+  const BlockSads* xs;
   const Plan* pl;
   int mbx, mby, cxp, cyp;
 };
@@ -462,8 +527,15 @@ __device__ __forceinline__ uint32_t group_sad(const FieldView& v, const MePlane&
     return v.F->grp[p][(pid == 0 ? 0 : (pid == 1 ? 2 : 4)) + g];
   }
   for (int j = 0; j < v.pl->nblocks; j++)
-    if (v.mbx + v.pl->box[j] == x && v.mby + v.pl->boy[j] == y) return group_sum(v.xs[j], pid, g);
+    if (v.mbx + v.pl->box[j] == x && v.mby + v.pl->boy[j] == y)
+      return pid == 3 ? v.xs->blk[j][g] : v.xs->grp[j][(pid == 0 ? 0 : (pid == 1 ? 2 : 4)) + g];
   return direct_group_sad(P, src, x, y, pid, g);
+}
+
+// An integer below 2^32 as a double: the bits of 2^52 + v, less 2^52 (exact; the
+// conversion unit is slower than an addition).
+__device__ __forceinline__ double small_double(uint32_t v) {
+  return __hiloint2double(0x43300000, (int)v) - 4503599627370496.0;
 }
 
 __device__ __forceinline__ double submv_ref_bits(const double* t, const uint8_t* p, int mode) {
@@ -497,13 +569,11 @@ __device__ __forceinline__ double mv_partition_bits(const double* t, int pid) {
 // reference evaluates, so the chain's sums are unchanged.
 __device__ void split_partition(const AnArgs& a, const double* pbits, const double* sbits, const double* lterm,
                                 const double* mvb, const FieldView& fv, const MePlane& P, const uint8_t* src, vp8a_mv bp,
-                                const MbInfoDev& above, const MbInfoDev& left, int pid, SplitScratch& W,
-                                SplitOut* out, int lane) {
+                                int pid, SplitScratch& W, SplitOut* out, int lane) {
   const int G = pid == 3 ? 16 : (pid == 2 ? 4 : 2);
   const int goff = pid == 0 ? 0 : (pid == 1 ? 2 : 4);
   // Group `lane`'s NEW4X4 result (lanes < G).
-  bool my_new_ok = false;
-  uint32_t my_new_sad = 0;
+  uint32_t my_new_sad = 0, new_wins = 0;
   double my_new_bits = 0.0;
   if (lane < G) {
     // group_small_diamond_search (src/encoder.rs:7812-7879): snap then
@@ -584,25 +654,31 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
       }
       if (!improved) break;
     }
-    W.cmv[9 + g] = best;
+    W.cmv[g] = best;
     const int dr = (int)best.row - bp.row, dc = (int)best.col - bp.col;
     const bool ok = dr >= -1023 && dr <= 1023 && dc >= -1023 && dc <= 1023;
     const double nb = ok ? mvb[dr + 1023] + mvb[MV_BITS_SPAN + dc + 1023] : 0.0;
-    my_new_ok = ok;
     my_new_sad = bs;
     my_new_bits = nb;
+    // The cheaper of ZERO and NEW in each context (ZERO first among equals):
+    // neither depends on the chain below.
+    const int zb = fv.pl->colblk[0];
+    const double tz = (double)(pid == 3 ? fv.xs->blk[zb][g] : fv.xs->grp[zb][goff + g]), tn = (double)bs;
 #pragma unroll
-    for (int x = 0; x < 5; x++) W.new_cost[g * 5 + x] = a.lambda * (sbits[x * 4 + VP8A_SUBMV_NEW] + nb);
+    for (int x = 0; x < 5; x++) {
+      const uint64_t jz = (uint64_t)__double_as_longlong(tz + lterm[x * 4 + VP8A_SUBMV_ZERO]);
+      const uint64_t jn =
+          ok ? (uint64_t)__double_as_longlong(tn + a.lambda * (sbits[x * 4 + VP8A_SUBMV_NEW] + nb)) : ~0ull;
+      if (jn < jz) new_wins |= 1u << x;
+      W.zero_new[g * 5 + x] = jn < jz ? jn : jz;
+    }
   }
-  // Columns 0-8: ZERO, the left neighbour's vectors at anchors 0/4/8/12,
-  // the above neighbour's at anchors 0-3 (one lane each).
-  if (lane < 9)
-    W.cmv[lane] = lane == 0 ? vp8a_mv{0, 0} : (lane < 5 ? ext_left(left, 4 * (lane - 1)) : ext_above(above, lane - 5));
   __syncwarp();
   // Lane m < 9 + G holds column m's vector, packed (equal vectors, equal
-  // words; the zero vector is 0).
+  // words; the zero vector is 0). Columns 0-8 are the plan's: ZERO, the left
+  // neighbour's vectors at anchors 0/4/8/12, the above neighbour's at 0-3.
   const int ncol = 9 + G;
-  const vp8a_mv mvm = lane < ncol ? W.cmv[lane] : vp8a_mv{0, 0};
+  const vp8a_mv mvm = lane < 9 ? fv.pl->colmv[lane] : (lane < ncol ? W.cmv[lane - 9] : vp8a_mv{0, 0});
   const uint32_t cvec = (uint32_t)(uint16_t)mvm.row | ((uint32_t)(uint16_t)mvm.col << 16);
   // The candidate table: lane m fills column m for every group. Columns
   // 0-8 (ZERO and the neighbours' vectors) are staged blocks; columns 9+
@@ -612,24 +688,21 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
   if (lane < ncol && ((need >> lane) & 1u)) {
     const int x = fv.mbx + int_off(mvm.col), y = fv.mby + int_off(mvm.row);
     const int cp = lane < 9 ? fv.pl->colblk[lane] : fpos(x - fv.cxp, y - fv.cyp);
-    uint32_t* col = W.table + lane * 16;
-    if (pid == 3 && (lane < 9 || cp >= 0)) {
+    double* col = W.table + lane * 16;
+    if (lane < 9 || cp >= 0) {
       // The 16 block SADs of a staged block or a field position are one
-      // 32-byte row.
-      const uint4* row = lane < 9 ? (const uint4*)fv.xs[cp] : (const uint4*)fv.F->blk[cp];
-      const uint4 lo = row[0], hi = row[1];
-      const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      // 32-byte row, the group sums one of 16 bytes.
+      const uint16_t* row = pid == 3 ? (lane < 9 ? fv.xs->blk[cp] : fv.F->blk[cp])
+                                     : (lane < 9 ? fv.xs->grp[cp] : fv.F->grp[cp]) + goff;
 #pragma unroll
-      for (int q = 0; q < 4; q++)
-        ((uint4*)col)[q] = make_uint4(w[2 * q] & 0xffffu, w[2 * q] >> 16, w[2 * q + 1] & 0xffffu, w[2 * q + 1] >> 16);
+      for (int g = 0; g < 16; g += 2)
+        if (g < G) {
+          const uint32_t w = *(const uint32_t*)(row + g);
+          *(double2*)(col + g) = make_double2(small_double(w & 0xffffu), small_double(w >> 16));
+        }
     } else {
-      for (int g = 0; g < G; g++) {
-        uint32_t v;
-        if (lane < 9) v = pid == 3 ? fv.xs[cp][g] : group_sum(fv.xs[cp], pid, g);
-        else if (cp >= 0) v = pid == 3 ? fv.F->blk[cp][g] : fv.F->grp[cp][goff + g];
-        else v = direct_group_sad(P, src, x, y, pid, g);
-        col[g] = v;
-      }
+#pragma unroll 1
+      for (int g = 0; g < G; g++) col[g] = (double)direct_group_sad(P, src, x, y, pid, g);
     }
   }
   __syncwarp();
@@ -653,19 +726,18 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
   const uint32_t new_vec = __shfl_sync(FULL, cvec, (9 + lane) & 31);
   // The group's choice: its column and that column's vector.
   int chosen = 0, mode = VP8A_SUBMV_ZERO, my_ctx = 0;
-  uint32_t chosen_vec = 0, my_sad = 0;
+  uint32_t chosen_vec = 0;
   bool my_bad = false;
+  const int lsrc = gc == 0 ? lane : lane - 1, asrc = gr == 0 ? lane : lane - gw;
+#pragma unroll 1
   for (int st = 0; st < gh + gw - 1; st++) {
-    const int lsrc = gc == 0 ? lane : lane - 1, asrc = gr == 0 ? lane : lane - gw;
     const int lch = __shfl_sync(FULL, chosen, lsrc), ach = __shfl_sync(FULL, chosen, asrc);
     const uint32_t lchv = __shfl_sync(FULL, chosen_vec, lsrc), achv = __shfl_sync(FULL, chosen_vec, asrc);
     if (lane < G && gr + gc == st) {
       const int lidx = gc == 0 ? ext_l : lch, aidx = gr == 0 ? ext_a : ach;
       const uint32_t lv = gc == 0 ? ext_lv : lchv, av = gr == 0 ? ext_av : achv;
       const bool lez = lv == 0u, aez = av == 0u, lea = lv == av;
-      const int ctxi = (lea && lez) ? 4 : (lea ? 3 : (aez ? 2 : (lez ? 1 : 0)));
-      const double* lt = lterm + ctxi * 4;
-      const uint32_t tl = W.table[lidx * 16 + lane], ta = W.table[aidx * 16 + lane], tz = W.table[lane];
+      const int ctxi = lea ? (lez ? 4 : 3) : (aez ? 2 : (lez ? 1 : 0));
       // LEFT, ABOVE, ZERO, then NEW (sad + lambda * (mode bits + vector
       // bits), the vector bits 0 for the first three); the reference keeps
       // the first strict minimum in that order. Every J here is a finite sum
@@ -673,52 +745,44 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
       // patterns as unsigned integers, and the first minimum of the four is
       // the first minimum of the first minima of (LEFT, ABOVE) and (ZERO,
       // NEW).
-      const uint64_t j0 = (uint64_t)__double_as_longlong((double)tl + lt[0]);
-      const uint64_t j1 = (uint64_t)__double_as_longlong((double)ta + lt[1]);
-      const uint64_t j2 = (uint64_t)__double_as_longlong((double)tz + lt[2]);
-      const uint64_t jn = my_new_ok ? (uint64_t)__double_as_longlong((double)my_new_sad + W.new_cost[lane * 5 + ctxi])
-                                    : 0xffffffffffffffffull;
-      const bool above_first = j1 < j0, new_second = jn < j2;
-      const uint64_t v01 = above_first ? j1 : j0, v2n = new_second ? jn : j2;
+      const double2 lt = *(const double2*)(lterm + ctxi * 4);
+      const uint64_t j0 = (uint64_t)__double_as_longlong(W.table[lidx * 16 + lane] + lt.x);
+      const uint64_t j1 = (uint64_t)__double_as_longlong(W.table[aidx * 16 + lane] + lt.y);
+      const uint64_t v2n = W.zero_new[lane * 5 + ctxi];
+      const bool above_first = j1 < j0, is_new = (new_wins >> ctxi) & 1u;
+      const uint64_t v01 = above_first ? j1 : j0;
       const bool second = v2n < v01;
-      const uint64_t best_j = second ? v2n : v01;
-      mode = second ? (new_second ? VP8A_SUBMV_NEW : VP8A_SUBMV_ZERO)
+      mode = second ? (is_new ? VP8A_SUBMV_NEW : VP8A_SUBMV_ZERO)
                     : (above_first ? VP8A_SUBMV_ABOVE : VP8A_SUBMV_LEFT);
-      chosen = second ? (new_second ? 9 + lane : 0) : (above_first ? aidx : lidx);
-      chosen_vec = second ? (new_second ? new_vec : 0u) : (above_first ? av : lv);
-      my_sad = second ? (new_second ? my_new_sad : tz) : (above_first ? ta : tl);
+      chosen = second ? (is_new ? 9 + lane : 0) : (above_first ? aidx : lidx);
+      chosen_vec = second ? (is_new ? new_vec : 0u) : (above_first ? av : lv);
       my_ctx = ctxi;
-      my_bad = best_j >= 0x7ff0000000000000ull;
+      my_bad = (second ? v2n : v01) >= 0x7ff0000000000000ull;
     }
   }
   if (lane < G) out->modes[lane] = (uint8_t)mode;
   // Totals in the reference's group order (the f64 sum is order-sensitive):
-  // the groups' terms go through shared memory and lane 0 sums them in
-  // order.
-  const bool mine = lane < G;
-  const bool isn = mine && mode == VP8A_SUBMV_NEW;
-  if (mine) {
-    W.terms[lane] = sbits[my_ctx * 4 + mode];
-    W.terms[16 + lane] = my_new_bits;
-  }
-  const uint32_t total_sad = __reduce_add_sync(FULL, mine ? my_sad : 0u);
+  // the groups' terms go through shared memory, closed up, and lane 0 sums
+  // them in order.
+  const bool mine = lane < G, isn = mine && mode == VP8A_SUBMV_NEW;
+  const uint32_t my_sad = !mine ? 0u : (isn ? my_new_sad : (uint32_t)W.table[chosen * 16 + lane]);
+  const uint32_t total_sad = __reduce_add_sync(FULL, my_sad);
   const unsigned any_bad = __ballot_sync(FULL, mine && my_bad), news = __ballot_sync(FULL, isn);
+  if (mine) {
+    const int at = lane + __popc(news & ((1u << lane) - 1u));
+    W.terms[at] = sbits[my_ctx * 4 + mode];
+    if (isn) W.terms[at + 1] = my_new_bits;
+  }
+  if (lane >= G && lane < 16) out->modes[lane] = VP8A_SUBMV_ZERO;
   __syncwarp();
   if (lane == 0) {
     // The reference stops at the first group without a finite choice.
     out->valid = any_bad == 0u;
-    if (any_bad == 0u) {
-      double total_bits = 0.0;
-#pragma unroll
-      for (int gg = 0; gg < 16; gg++) {
-        if (gg < G) {
-          total_bits += W.terms[gg];
-          if ((news >> gg) & 1u) total_bits += W.terms[16 + gg];
-        }
-      }
-      out->j = (double)total_sad + a.lambda * (pbits[pid] + total_bits);
-      for (int i = G; i < 16; i++) out->modes[i] = VP8A_SUBMV_ZERO;
-    }
+    double total_bits = 0.0;
+    const int n = G + __popc(news);
+#pragma unroll 2
+    for (int i = 0; i < n; i++) total_bits += W.terms[i];
+    out->j = (double)total_sad + a.lambda * (pbits[pid] + total_bits);
   }
   // Block b's vector: the column its group chose.
   const int gb = lane < 16 ? (((lane >> 2) >> (2 - lgh)) << lgw) + ((lane & 3) >> (2 - lgw)) : 0;
@@ -729,6 +793,12 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// A poll: an acquiring load would drop the SM's L1 lines at every try.
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
@@ -844,161 +914,12 @@ constexpr int AN_THREADS = NW * 32;
 constexpr int MAIN_WARPS = 5;         // warps 0 and 5-8: the MB search chain
 constexpr int MAIN_THREADS = MAIN_WARPS * 32;
 
-// Offsets (row, col) of the eight refinement candidates in the reference's
-// order: (-1,-1) (-1,0) (-1,1) (0,-1) (0,1) (1,-1) (1,0) (1,1).
-__device__ __forceinline__ int cand_dr(int k) { return (k < 3) ? -1 : (k < 5 ? 0 : 1); }
-__device__ __forceinline__ int cand_dc(int k) { return (k == 0 || k == 3 || k == 5) ? -1 : ((k == 1 || k == 6) ? 0 : 1); }
 
-// The H, V and D half-pel planes around a whole-pel centre whose block
-// origin in the window is (bx, by) (the planes of half_plane_sads, filled
-// by the main group's MAIN_THREADS threads): H and V first, then D from H.
-// Each thread's outputs are independent; the loops are unrolled so that
-// all of a thread's window reads are in flight together.
-__device__ __forceinline__ void half_planes_hv(WarpScratch& S, int bx, int by, int tid) {
-  constexpr int NH = 22 * 17, NO = NH + 17 * 16;
-#pragma unroll
-  for (int it = 0; it < (NO + MAIN_THREADS - 1) / MAIN_THREADS; it++) {
-    const int o = tid + it * MAIN_THREADS;
-    if (o < NH) {
-      const int r = o / 17, i = o - r * 17;
-      const uint8_t* p = S.win + (by - 3 + r) * WS + bx + i - 3;
-      S.hp[o] = (uint8_t)interp6_half(p[0], p[1], p[2], p[3], p[4], p[5]);
-    } else if (o < NO) {
-      const int q = o - NH, r = q >> 4, c = q & 15;
-      const uint8_t* p = S.win + (by + r - 3) * WS + bx + c;
-      S.vp[q] = (uint8_t)interp6_half(p[0], p[WS], p[2 * WS], p[3 * WS], p[4 * WS], p[5 * WS]);
-    }
-  }
-}
-
-// The D plane, from H (after H is complete).
-__device__ __forceinline__ void half_planes_d(WarpScratch& S, int tid) {
-#pragma unroll
-  for (int it = 0; it < (17 * 17 + MAIN_THREADS - 1) / MAIN_THREADS; it++) {
-    const int o = tid + it * MAIN_THREADS;
-    if (o < 17 * 17) {
-      const int r = o / 17, i = o - r * 17;
-      const uint8_t* p = S.hp + r * 17 + i;
-      S.dp[o] = (uint8_t)interp6_half(p[0], p[17], p[34], p[51], p[68], p[85]);
-    }
-  }
-}
-
-// SAD of half-pel candidate k against the planes (one warp).
-__device__ __forceinline__ uint32_t half_cand_sad(const WarpScratch& S, int k, const uint8_t* src, int lane) {
-  const int dy = cand_dr(k), dx = cand_dc(k);
-  const int cx = dx > 0, cy = dy > 0;
-  const uint8_t* pl;
-  int st;
-  if (dy == 0) {
-    pl = S.hp + 3 * 17 + cx;
-    st = 17;
-  } else if (dx == 0) {
-    pl = S.vp + cy * 16;
-    st = 16;
-  } else {
-    pl = S.dp + cy * 17 + cx;
-    st = 17;
-  }
-  const int c = lane & 15, r0 = (lane >> 4) * 8;
-  uint32_t s = 0;
-#pragma unroll
-  for (int r = r0; r < r0 + 8; r++) {
-    const int d = (int)pl[r * st + c] - (int)src[r * 16 + c];
-    s += (uint32_t)(d < 0 ? -d : d);
-  }
-  return __reduce_add_sync(FULL, s);
-}
-
-// quarter_pixel_refine_luma's eight candidates around `qc` share three
-// horizontal six-tap planes, one per candidate column (the columns are
-// qc.col - 1, qc.col, qc.col + 1 quarter-pels; a column whose eighth-pel
-// fraction is 0 keeps the unfiltered pixels, the reference's identity
-// elision). Each candidate's prediction is then its vertical pass over its
-// column's plane: the same taps, the same 8-bit intermediate and the same
-// edge-clamped source as its own two-pass synthesis.
-struct QuarterGeom {
-  int ix[3], fx[3], iy[3], fy[3], iy0;
-};
-
-// Fills the geometry; false when the window does not cover every
-// candidate's halo.
-__device__ __forceinline__ bool quarter_geom(vp8a_mv qc, int mbx, int mby, int wx0, int wy0, QuarterGeom& q) {
-  int xmin = 1 << 30, xmax = -(1 << 30), ymin = 1 << 30, ymax = -(1 << 30);
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const int ec = eighth(clamp_component(qc.col + k - 1)), er = eighth(clamp_component(qc.row + k - 1));
-    q.ix[k] = mbx + (ec >> 3) - wx0;
-    q.fx[k] = ec & 7;
-    q.iy[k] = mby + (er >> 3) - wy0;
-    q.fy[k] = er & 7;
-    xmin = min(xmin, q.ix[k]);
-    xmax = max(xmax, q.ix[k]);
-    ymin = min(ymin, q.iy[k]);
-    ymax = max(ymax, q.iy[k]);
-  }
-  q.iy0 = ymin - 2;  // first plane row (window coordinates)
-  // Planes span window rows iy0 .. iy0 + 21 and columns ix - 2 .. ix + 18.
-  return xmin >= 2 && xmax + 19 <= WS && ymin >= 2 && ymin + 20 <= WS && ymax - ymin <= 1;
-}
-
-// Horizontal planes: qh[k * 352 + rr * 16 + c], rr = 0..21 from window row
-// iy0 (filled by the main group; unrolled, as the half-pel planes).
-__device__ __forceinline__ void quarter_planes_h(const uint8_t* win, uint8_t* qh, const QuarterGeom& q, int t) {
-#pragma unroll
-  for (int it = 0; it < (3 * 22 * 16 + MAIN_THREADS - 1) / MAIN_THREADS; it++) {
-    const int o = t + it * MAIN_THREADS;
-    if (o < 3 * 22 * 16) {
-      const int k = o / 352, rem = o - k * 352, rr = rem >> 4, c = rem & 15;
-      const uint8_t* p = win + (q.iy0 + rr) * WS + q.ix[k] + c;
-      int v;
-      if (q.fx[k]) {
-        const int* f = c_sixtap[q.fx[k]];
-        v = interp6(f, p[-2], p[-1], p[0], p[1], p[2], p[3]);
-      } else {
-        v = p[0];
-      }
-      qh[o] = (uint8_t)v;
-    }
-  }
-}
-
-// Vertical pass and SAD of candidate t >> 4 at column t & 15, reduced over
-// the half-warp; the SAD is valid on lane (t & 15) == 0 of each half-warp.
-__device__ __forceinline__ uint32_t quarter_vsad(const uint8_t* qh, const QuarterGeom& q, const uint8_t* src, int t) {
-  const int k = t >> 4, c = t & 15;
-  const int kc = cand_dc(k) + 1, kr = cand_dr(k) + 1;
-  const uint8_t* pl = qh + kc * 352 + (q.iy[kr] - 2 - q.iy0) * 16 + c;  // plane row of prediction row -2
-  const int fy = q.fy[kr];
-  uint32_t s = 0;
-  if (fy) {
-    const int* fp = c_sixtap[fy];
-    const int f0 = fp[0], f1 = fp[1], f2 = fp[2], f3 = fp[3], f4 = fp[4], f5 = fp[5];
-    int w0 = pl[0], w1 = pl[16], w2 = pl[32], w3 = pl[48], w4 = pl[64];
-#pragma unroll
-    for (int r = 0; r < 16; r++) {
-      const int w5 = pl[(r + 5) * 16];
-      const int a = w0 * f0 + w1 * f1 + w2 * f2 + w3 * f3 + w4 * f4 + w5 * f5;
-      const int v = clampi((a + 64) >> 7, 0, 255);
-      const int d = v - (int)src[r * 16 + c];
-      s += (uint32_t)(d < 0 ? -d : d);
-      w0 = w1;
-      w1 = w2;
-      w2 = w3;
-      w3 = w4;
-      w4 = w5;
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < 16; r++) {
-      const int d = (int)pl[(r + 2) * 16] - (int)src[r * 16 + c];
-      s += (uint32_t)(d < 0 ? -d : d);
-    }
-  }
-  const unsigned hm = (t & 16) ? 0xffff0000u : 0x0000ffffu;
-#pragma unroll
-  for (int o = 8; o >= 1; o >>= 1) s += __shfl_xor_sync(hm, s, o);
-  return s;
+// The six taps of eighth-pel fraction f (even), from the CTA's copy of the
+// table (a lane's fraction differs from its neighbours').
+__device__ __forceinline__ Taps taps_of(const int4* tab, int f) {
+  const int4 a = tab[f], b = tab[f + 1];
+  return Taps{{a.x, a.y, a.z, a.w, b.x, b.y}};
 }
 
 struct __align__(16) WarpTemp {
@@ -1009,9 +930,186 @@ struct __align__(16) WarpTemp {
 // -------------------------------------------------------------- kernel
 
 
-// Barrier 1: the main group only.
+// Barrier 1: the main group only. Barrier 2: every search warp (all but the
+// helper warp).
 __device__ __forceinline__ void main_sync() { asm volatile("bar.sync 1, %0;" ::"n"(MAIN_THREADS) : "memory"); }
-static_assert(AN_THREADS >= 16 * FN, "one thread per field task");
+__device__ __forceinline__ void search_sync() { asm volatile("bar.sync 2, %0;" ::"n"(AN_THREADS) : "memory"); }
+static_assert(MAIN_THREADS >= 16 * FN, "one thread per field task");
+
+// What a CTA's helper warp and its cluster hand it, MB by MB (n counts the
+// MBs the cluster has taken): the source MB and the census record of the MB
+// above, fetched two MBs ahead, and every reference's decision. The decisions
+// arrive as asynchronous stores that complete a transaction on the mbarrier,
+// so no cluster barrier (a release of 700 to 900 cycles each) and no trip
+// through global memory lies between one MB's decision and the next MB's
+// census; rank 0's helper writes the results out and publishes the row's
+// progress meanwhile.
+constexpr int DEC_RING = 4;  // MB n's decisions are read until MB n + 2 starts
+struct Feed {
+  alignas(16) RefDec decs[DEC_RING][MAX_REFS];
+  alignas(16) uint8_t src[2][256];
+  alignas(16) MbInfoDev above[3];  // MB n's in entry n % 3; its above-left is MB n - 1's
+  alignas(16) MbInfoDev left, none;
+  uint64_t dec_bar[DEC_RING], in_bar[2];
+  int stop;  // the helper met a wait that ran out
+};
+static_assert(offsetof(Feed, src) % 16 == 0 && offsetof(Feed, above) % 16 == 0, "Feed alignment");
+
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool bar_done(uint64_t* bar, unsigned parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(done)
+      : "r"(smem_at(bar)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+__device__ __forceinline__ void bar_expect(uint64_t* bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_at(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_at(bar)) : "memory");
+}
+
+// A cluster's walk over its work items' MBs: the current item, its row, the
+// column. `job` is the item's arguments.
+struct MbCursor {
+  int it, r, c;
+  const AnArgs* job;
+};
+template <bool BATCH>
+__device__ __forceinline__ void cursor_item(MbCursor& q, const AnArgs& a0, const AnArgs* jobs, const uint32_t* items,
+                                            int n_it) {
+  q.c = 0;
+  q.job = nullptr;
+  if (q.it >= n_it) return;
+  if (BATCH) {
+    const uint32_t w = items[q.it];
+    q.job = jobs + (w >> 16);
+    q.r = (int)(w & 0xffffu);
+  } else {
+    q.job = &a0;
+    q.r = q.it;
+  }
+}
+template <bool BATCH>
+__device__ __forceinline__ void cursor_next(MbCursor& q, const AnArgs& a0, const AnArgs* jobs, const uint32_t* items,
+                                            int n_it, int n_clusters) {
+  if (++q.c < q.job->mb_cols) return;
+  q.it += n_clusters;
+  cursor_item<BATCH>(q, a0, jobs, items, n_it);
+}
+
+// decide_mb_exhaustive's reference comparison: first strict minimum of J +
+// ref_frame_tree_bits in reference order; -1 when none is finite.
+__device__ __forceinline__ int pick_reference(const RefDec* decs, int n_refs) {
+  double best = __longlong_as_double(0x7ff0000000000000LL);
+  int k = -1;
+  for (int q = 0; q < n_refs; q++)
+    if (decs[q].total < best) {
+      best = decs[q].total;
+      k = q;
+    }
+  return k;
+}
+
+// Word `w` of the census record that decision `d` leaves.
+__device__ __forceinline__ uint32_t record_word(const RefDec& d, uint32_t id, int w) {
+  const uint32_t* b = (const uint32_t*)&d;
+  const uint32_t spl = d.mode == VP8A_MODE_SPLIT;
+  if (w == 0) return id | spl << 8 | spl << 16;
+  return w == 1 ? b[4] : b[w + 5];
+}
+
+// The helper warp of CTA k.
+template <bool BATCH>
+__device__ void run_helper(Feed& F, const AnArgs& a0, const AnArgs* jobs, const uint32_t* items, int n_it, int first,
+                           int n_clusters, int k, int lane) {
+  MbCursor pre{first, 0, 0, nullptr}, pub{first, 0, 0, nullptr};
+  cursor_item<BATCH>(pre, a0, jobs, items, n_it);
+  pub = pre;
+  unsigned n_pre = 0, n_pub = 0;
+  unsigned long long polls = 0;
+  unsigned idle = 0;
+  while (pub.job) {
+    bool moved = false;
+    // MB n_pub decided everywhere?
+    if (__all_sync(FULL, bar_done(&F.dec_bar[n_pub % DEC_RING], n_pub / DEC_RING & 1u))) {
+      const RefDec* decs = F.decs[n_pub % DEC_RING];
+      const AnArgs& a = *pub.job;
+      if (k == 0) {
+        const int best = pick_reference(decs, a.n_refs);
+        const RefDec& d = decs[best < 0 ? 0 : best];
+        const uint32_t* b = (const uint32_t*)&d;
+        const uint32_t id = best >= 0 ? (uint32_t)a.ref_ids[best] : 0u;
+        uint32_t* dw = (uint32_t*)(a.dec + (size_t)pub.r * a.mb_cols + pub.c);
+        uint32_t* iw = (uint32_t*)(a.infos + (size_t)pub.r * a.mb_cols + pub.c);
+        if (lane < 18) iw[lane] = best >= 0 ? record_word(d, id, lane) : 0u;
+        __syncwarp();
+        // The release orders the warp's record before the count.
+        if (lane == 0) st_release(&a.progress[pub.r], (unsigned)(pub.c + 1));
+        if (lane < 26) {  // vp8a_mb_decision
+          uint32_t w;
+          if (lane == 0) w = id | ((uint32_t)d.mode & 0xffu) << 8 | ((uint32_t)d.pid & 0xffu) << 16;
+          else if (lane == 1) w = b[4];         // mv
+          else if (lane < 6) w = b[lane - 2];   // j, total
+          else w = b[lane + 1];                 // split_mvs, submv_modes
+          dw[lane] = best >= 0 ? w : 0u;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) bar_expect(&F.dec_bar[n_pub % DEC_RING], (unsigned)(sizeof(RefDec) * a.n_refs));
+      n_pub++;
+      cursor_next<BATCH>(pub, a0, jobs, items, n_it, n_clusters);
+      moved = true;
+    }
+    // MB n_pre's inputs: the buffers of MB n_pre - 2 are free once it is
+    // decided; the row above must have published (r - 1, c). MB (r, c) reads
+    // the records of its above, left and above-left neighbours only
+    // (find_near_mvs, SPLITMV LEFT/ABOVE sub-MVs). The reference's row
+    // contract waits for (r - 1, c + 1) (src/encoder/inter.rs:350-513)
+    // because its intra candidates predict from the above-right MB's
+    // reconstruction; with intra picking off nothing here reads that MB.
+    if (pre.job && n_pre < n_pub + 2) {
+      const AnArgs& a = *pre.job;
+      const bool ready =
+          pre.r == 0 || (__all_sync(FULL, ld_relaxed(&a.progress[pre.r - 1]) >= (unsigned)(pre.c + 1)) &&
+                         __all_sync(FULL, ld_acquire(&a.progress[pre.r - 1]) >= (unsigned)(pre.c + 1)));
+      if (ready) {
+        polls = 0;
+        // The edge-replicated source MB (extract_mb, src/encoder.rs:5549):
+        // eight pixels a lane.
+        uint8_t* s = F.src[n_pre & 1];
+        const int row = lane >> 1, x0 = pre.c * 16 + (lane & 1) * 8;
+        const uint8_t* g = a.fy + (size_t)min(pre.r * 16 + row, a.fh - 1) * a.fys;
+        uint32_t v[2] = {0, 0};
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i >> 2] |= (uint32_t)g[min(x0 + i, a.fw - 1)] << (8 * (i & 3));
+        uint32_t rec = lane == 0 ? (uint32_t)VP8A_REF_INTRA : 0u;
+        if (pre.r > 0 && lane < 18)
+          rec = __ldcg((const uint32_t*)(a.infos + (size_t)(pre.r - 1) * a.mb_cols + pre.c) + lane);
+        *(uint2*)(s + row * 16 + (lane & 1) * 8) = make_uint2(v[0], v[1]);
+        if (lane < 18) ((uint32_t*)&F.above[n_pre % 3])[lane] = rec;
+        __syncwarp();
+        if (lane == 0) bar_arrive(&F.in_bar[n_pre & 1]);
+        n_pre++;
+        cursor_next<BATCH>(pre, a0, jobs, items, n_it, n_clusters);
+        moved = true;
+      } else if (++polls > a.spin_limit) {
+        if (lane == 0) atomicCAS(a.status, 0u, (unsigned)vp8a::DEV_TIMEOUT);
+      }
+    }
+    if (!moved) {
+      if ((++idle & 15u) == 0 && __any_sync(FULL, *(volatile unsigned*)pub.job->status != 0u)) {
+        if (lane == 0) *(volatile int*)&F.stop = 1;
+        return;
+      }
+      __nanosleep(40);
+    }
+  }
+}
 
 // Work items: one MB row each. A single frame (BATCH false) takes rows
 // 0..a0.mb_rows-1 of a0; a batch takes items[i] = job << 16 | row over the
@@ -1024,8 +1122,8 @@ static_assert(AN_THREADS >= 16 * FN, "one thread per field task");
 // wavefront is mb_cols + mb_rows MB steps); sharing an SM costs each MB
 // less than that saves (1080p analysis 3.06 -> 2.40 ms).
 template <bool BATCH>
-__global__ void __launch_bounds__(AN_THREADS, 2)
-    analysis_kernel(AnArgs a0, const AnArgs* __restrict__ jobs, const uint32_t* __restrict__ items, int n_items) {
+__global__ void __launch_bounds__(AN_THREADS + 32, 2)
+    analysis_kernel(const __grid_constant__ AnArgs a0, const AnArgs* __restrict__ jobs, const uint32_t* __restrict__ items, int n_items) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   __shared__ AnArgs a;  // the current item's job
@@ -1038,20 +1136,19 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
   extern __shared__ __align__(16) uint8_t dyn_smem[];
   SplitScratch* ss = (SplitScratch*)dyn_smem;
   double* mvb = (double*)(dyn_smem + 4 * sizeof(SplitScratch));
-  __shared__ __align__(16) uint16_t xs[MAX_BLOCKS][16];
-  __shared__ __align__(16) uint8_t src[256];
+  __shared__ BlockSads xs;
   __shared__ double bit_cost[256];
   __shared__ double sbits[5 * 4];  // submv_ref_bits per context and mode
-  __shared__ double lterm[5 * 4];  // lambda * (sbits + 0.0): the LEFT/ABOVE/ZERO cost terms
+  __shared__ __align__(16) double lterm[5 * 4];  // lambda * (sbits + 0.0): the LEFT/ABOVE/ZERO cost terms
   __shared__ MainOut mo;
   __shared__ uint32_t cand_sad[8];
   __shared__ SplitOut splits[4];
   __shared__ RefDec mydec;
-  __shared__ RefDec decs[MAX_REFS];  // rank 0: every reference's decision
-  __shared__ __align__(16) MbInfoDev nb[3];  // above, left, aboveleft
+  __shared__ Feed feed;
   __shared__ Census cen;
   __shared__ Plan plan;
-  __shared__ int s_abort, s_qok;
+  __shared__ int s_stop, s_rounds;
+  __shared__ int4 tap_tab[8];  // the six taps of the even fraction f at tap_tab[f], [f + 1]
   __shared__ vp8a_mv s_prop_mv;
   __shared__ uint32_t s_prop_sad;
   __shared__ int s_prop_ok;
@@ -1059,18 +1156,34 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
   // filled during the search by warp 7; per-CTA constants below.
   __shared__ double dz, dnearest, dnear, dnew_bits, dsplit;
   __shared__ double lrbits, pbits[4];
-  __shared__ QuarterGeom s_qg;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int k = (int)cl.block_rank();  // the reference this CTA searches
   const int csize = (int)cl.num_blocks();
   const int cid = blockIdx.x / csize, n_clusters = gridDim.x / csize;
   const MePlane& P = a.refs[k];
-  uint32_t* dec_slot = (uint32_t*)cl.map_shared_rank(&decs[k], 0);
-  const int* abort0 = cl.map_shared_rank(&s_abort, 0);
-  if (tid == 0) s_mvb_src = nullptr;
+  if (tid == 0) {
+    s_mvb_src = nullptr;
+    feed.stop = 0;
+    for (int i = 0; i < DEC_RING; i++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(&feed.dec_bar[i])) : "memory");
+    for (int i = 0; i < 2; i++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(&feed.in_bar[i])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = 0; i < DEC_RING; i++) bar_expect(&feed.dec_bar[i], (unsigned)sizeof(RefDec) * csize);
+  }
+  if (tid < 4 * 6) ((int*)&tap_tab[2 * (tid / 6)])[tid % 6] = c_sixtap[2 * (tid / 6)][tid % 6];
+  if (tid < 18) ((uint32_t*)&feed.none)[tid] = tid == 0 ? (uint32_t)VP8A_REF_INTRA : 0u;
+  cl.sync();
   const int n_it = BATCH ? n_items : a0.mb_rows;
   int cur = -1;
+  unsigned n = 0;  // MBs this cluster has taken
 
+  if (warp == NW) {
+    run_helper<BATCH>(feed, a0, jobs, items, n_it, cid, n_clusters, k, lane);
+    __syncwarp();
+    cl.sync();  // no CTA leaves while another may write to it
+    return;
+  }
   for (int it = cid; it < n_it; it += n_clusters) {
     int r = it, job = 0;
     if (BATCH) {
@@ -1081,13 +1194,13 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
     if (job != cur) {
       // Load the job and its per-job constants. The barrier first: the
       // previous MB's last writes still read the old job's pointers.
-      __syncthreads();
+      search_sync();
       if (tid == 0) a = BATCH ? jobs[job] : a0;
-      __syncthreads();
+      search_sync();
       for (int i = tid; i < 256; i += AN_THREADS) bit_cost[i] = a.bit_cost[i];
       if (s_mvb_src != a.mvbits)
         for (int i = tid; i < 2 * MV_BITS_SPAN; i += AN_THREADS) mvb[i] = a.mvbits[i];
-      __syncthreads();
+      search_sync();
       if (tid < 20) {
         const double b = submv_ref_bits(bit_cost, c_submv_probs[tid >> 2], tid & 3);
         sbits[tid] = b;
@@ -1105,106 +1218,112 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
       } else if (tid == 32) {
         s_mvb_src = a.mvbits;
       }
-      __syncthreads();
+      search_sync();
       cur = job;
     }
-    for (int c = 0; c < a.mb_cols; c++) {
-      // Rank 0 waits for the row above; the cluster follows its verdict.
-      // MB (r, c) reads the records of its above, left and above-left
-      // neighbours only (find_near_mvs, SPLITMV LEFT/ABOVE sub-MVs), so it
-      // needs MB (r - 1, c) done. The reference's row contract waits for
-      // (r - 1, c + 1) (src/encoder/inter.rs:350-513) because its intra
-      // candidates predict from the above-right MB's reconstruction; with
-      // intra picking off nothing here reads that MB, and the decisions do
-      // not depend on the schedule.
-      if (k == 0 && tid == 0) {
-        int abort = 0;
-        if (r > 0) {
-          const unsigned need = (unsigned)(c + 1);
-          unsigned long long it = 0;
-          while (ld_acquire(&a.progress[r - 1]) < need) {
-            if (*(volatile unsigned*)a.status != 0u || ++it > a.spin_limit) {
-              atomicCAS(a.status, 0u, (unsigned)vp8a::DEV_TIMEOUT);
-              abort = 1;
+    for (int c = 0; c < a.mb_cols; c++, n++) {
+      const uint8_t* src = feed.src[n & 1];
+      const MbInfoDev& above = feed.above[n % 3];
+      const MbInfoDev& above_left = c > 0 ? feed.above[(n + 2) % 3] : feed.none;
+      const int mbx = c * 16, mby = r * 16;
+      if (warp < 2) {
+        // The previous MB's decisions (its record is this one's left
+        // neighbour) and this MB's inputs. Warp 0 takes the census, warp 1
+        // the vectors of the SPLITMV columns.
+        int stop = 0, best = -1;
+        const RefDec* prev = feed.decs[(n - 1) % DEC_RING];
+        if (c > 0) {
+          const unsigned m = n - 1;
+          while (!bar_done(&feed.dec_bar[m % DEC_RING], m / DEC_RING & 1u))
+            if (*(volatile int*)&feed.stop) {
+              stop = 1;
               break;
             }
-            __nanosleep(64);
-          }
-        } else if (*(volatile unsigned*)a.status != 0u) {
-          abort = 1;
+          best = pick_reference(prev, csize);
         }
-        s_abort = abort;
+        const RefDec& ld = prev[best < 0 ? 0 : best];  // the left MB's, when best >= 0
+        if (warp == 0 && lane < 18)
+          ((uint32_t*)&feed.left)[lane] = best >= 0 ? record_word(ld, (uint32_t)a.ref_ids[best], lane)
+                                                    : (lane == 0 ? (uint32_t)VP8A_REF_INTRA : 0u);
+        while (!bar_done(&feed.in_bar[n & 1], n / 2 & 1u))
+          if (*(volatile int*)&feed.stop) {
+            stop = 1;
+            break;
+          }
+        __syncwarp();
+        if (warp == 0) {
+          stop = __any_sync(FULL, stop);
+          const Census cs = census(above, feed.left, above_left, c, r, a.mb_cols, a.mb_rows);
+          if (lane == 0) {
+            s_stop = stop;
+            cen = cs;
+            const vp8a_mv bp = cs.best_predictor;
+            plan.wx0 = mbx + snap_whole(clamp_component(bp.col)) / 4 - WIN_LEAD;
+            plan.wy0 = mby + snap_whole(clamp_component(bp.row)) / 4 - WIN_LEAD;
+            plan.hn_x = mbx + int_off(cs.nearest.col) - 2;
+            plan.hn_y = mby + int_off(cs.nearest.row) - 2;
+            plan.hr_x = mbx + int_off(cs.near_.col) - 2;
+            plan.hr_y = mby + int_off(cs.near_.row) - 2;
+            plan.want_nearest = !mv_zero(cs.nearest);
+            plan.want_near = !mv_zero(cs.near_);
+          }
+        } else {
+          // Lanes 0-8 hold the column vectors (ZERO, the left neighbour's at
+          // anchors 0/4/8/12, the above neighbour's at 0-3: left_block_mv /
+          // above_block_mv, src/near_mv.rs:722-760); vectors with equal
+          // integer offsets share one staged block, numbered in column order
+          // of first appearance.
+          const bool l_split = best >= 0 && ld.mode == VP8A_MODE_SPLIT;
+          vp8a_mv m = {0, 0};
+          if (lane >= 1 && lane < 5) m = best < 0 ? m : (l_split ? ld.split_mvs[4 * lane - 1] : ld.mv);
+          else if (lane >= 5 && lane < 9) m = ext_above(above, lane - 5);
+          const int ox = int_off(m.col), oy = int_off(m.row);
+          const unsigned key = ((unsigned)(uint16_t)oy << 16) | (uint16_t)ox;
+          const unsigned same = __match_any_sync(FULL, lane < 9 ? key : 0xffffffffu) & 0x1ffu;
+          const int leader = __ffs(same) - 1;
+          const unsigned leaders = __ballot_sync(FULL, lane < 9 && leader == lane);
+          if (lane < 9) {
+            const int idx = __popc(leaders & ((1u << leader) - 1u));
+            plan.colblk[lane] = idx;
+            plan.colmv[lane] = m;
+            if (leader == lane) {
+              plan.box[idx] = ox;
+              plan.boy[idx] = oy;
+            }
+          }
+          if (lane == 0) plan.nblocks = __popc(leaders);
+        }
       }
-      cl.sync();
-      if (*abort0) {
-        cl.sync();  // rank 0's shared memory stays live until every CTA has read it
+      search_sync();
+      if (s_stop) {
+        cl.sync();
         return;
       }
-      // Neighbour records (read past L1: rank 0 and other clusters write
-      // them) and the edge-replicated source MB (extract_mb,
-      // src/encoder.rs:5549).
-      if (tid < 3 * 18) {
-        const int n = tid / 18, w = tid - n * 18;
-        const int nr = n == 1 ? r : r - 1, nc = n == 0 ? c : c - 1;
-        const uint32_t* g = (const uint32_t*)(a.infos + (size_t)nr * a.mb_cols + nc);
-        // Outside the frame: an intra record (ref_frame in byte 0, the rest 0).
-        ((uint32_t*)&nb[n])[w] = (nr >= 0 && nc >= 0) ? __ldcg(g + w) : (w == 0 ? (uint32_t)VP8A_REF_INTRA : 0u);
-      }
-      for (int i = tid; i < 256; i += AN_THREADS) {
-        const int y = min(r * 16 + (i >> 4), a.fh - 1), x = min(c * 16 + (i & 15), a.fw - 1);
-        src[i] = a.fy[(size_t)y * a.fys + x];
-      }
-      __syncthreads();
-      const int mbx = c * 16, mby = r * 16;
-      if (warp == 0) {
-        // The census (every lane, registers only) and the staging plan: lanes
-        // 0-8 hold the SPLITMV column vectors (ZERO, the left neighbour's
-        // at anchors 0/4/8/12, the above neighbour's at 0-3); vectors with
-        // equal integer offsets share one staged block, numbered in column
-        // order of first appearance.
-        const Census cs = census(nb[0], nb[1], nb[2], c, r, a.mb_cols, a.mb_rows);
-        const vp8a_mv m = lane == 0 ? vp8a_mv{0, 0}
-                                    : (lane < 5 ? ext_left(nb[1], 4 * ((lane - 1) & 3)) : ext_above(nb[0], (lane - 5) & 3));
-        const int ox = int_off(m.col), oy = int_off(m.row);
-        const unsigned key = ((unsigned)(uint16_t)oy << 16) | (uint16_t)ox;
-        const unsigned cols9 = 0x1ffu;
-        const unsigned same = __match_any_sync(FULL, lane < 9 ? key : 0xffffffffu) & cols9;
-        const int leader = __ffs(same) - 1;
-        const unsigned leaders = __ballot_sync(FULL, lane < 9 && leader == lane);
-        if (lane < 9) {
-          const int idx = __popc(leaders & ((1u << leader) - 1u));
-          plan.colblk[lane] = idx;
-          if (leader == lane) {
-            plan.box[idx] = ox;
-            plan.boy[idx] = oy;
-          }
-        }
-        if (lane == 0) {
-          cen = cs;
-          const vp8a_mv bp = cs.best_predictor;
-          plan.wx0 = mbx + snap_whole(clamp_component(bp.col)) / 4 - WIN_LEAD;
-          plan.wy0 = mby + snap_whole(clamp_component(bp.row)) / 4 - WIN_LEAD;
-          plan.hn_x = mbx + int_off(cs.nearest.col) - 2;
-          plan.hn_y = mby + int_off(cs.nearest.row) - 2;
-          plan.hr_x = mbx + int_off(cs.near_.col) - 2;
-          plan.hr_y = mby + int_off(cs.near_.row) - 2;
-          plan.nblocks = __popc(leaders);
-        }
-      }
-      __syncthreads();
       stage_ref(P, R, plan, mbx, mby, a.words, tid, AN_THREADS);
-      __syncthreads();
-      field_blocks(R.ws.win, src, F, tid);
-      __syncthreads();
+      search_sync();
+      // Warps 0-4 the field's block SADs, warps 5-8 the staged blocks'.
+      if (warp < MAIN_WARPS) field_blocks(R.ws.win, src, F, tid);
+      else staged_block_sads(R, src, plan.nblocks, xs, tid - MAIN_THREADS, AN_THREADS - MAIN_THREADS);
+      search_sync();
       field_sums(F, tid, AN_THREADS);
-      staged_block_sads(R, src, plan.nblocks, xs, tid, AN_THREADS);
-      __syncthreads();
+      search_sync();
       const vp8a_mv bp = cen.best_predictor;
       const int cxp = plan.wx0 + WIN_LEAD, cyp = plan.wy0 + WIN_LEAD;  // field centre (plane pixels)
-      const FieldView fv{&F, xs, &plan, mbx, mby, cxp, cyp};
+      const FieldView fv{&F, &xs, &plan, mbx, mby, cxp, cyp};
       if (warp >= 1 && warp <= 4) {
-        split_partition(a, pbits, sbits, lterm, mvb, fv, P, src, bp, nb[0], nb[1], warp - 1, ss[warp - 1],
+        split_partition(a, pbits, sbits, lterm, mvb, fv, P, src, bp, warp - 1, ss[warp - 1],
                         &splits[warp - 1], lane);
+        // The short partitions' warps take NEAREST and NEAR.
+        if (warp <= 2) {
+          const bool near = warp == 2, want = near ? plan.want_near : plan.want_nearest;
+          const vp8a_mv v = near ? cen.near_ : cen.nearest;
+          uint32_t sv = (uint32_t)xs.grp[0][0] + xs.grp[0][1];  // the ZERO vector's
+          if (want) {
+            const uint8_t* h = near ? R.halo_near : R.halo_nearest;
+            sv = subpel_sad(h, HS, eighth(v.col) & 7, eighth(v.row) & 7, src, wt[warp].temp, lane);
+          }
+          if (lane == 0) (near ? mo.sad_near : mo.sad_nearest) = sv;
+        }
       } else {
         // The main group (warps 0 and 5-8) runs the MB search chain while
         // warps 1-4 score the SPLITMV partitions.
@@ -1212,22 +1331,16 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
         if (warp == 0) {
           // ZEROMV SAD and the whole-pel diamond (src/encoder.rs:8560-8576).
           uint32_t z = 0;
-          if (lane < 16) z = xs[0][lane];
+          if (lane < 16) z = xs.blk[0][lane];
           z = __reduce_add_sync(FULL, z);
+          int rounds;
           const vp8a_search_result w =
-              diamond_field(F, P, R.ws.win, plan.wx0, plan.wy0, mbx, mby, cxp, cyp, bp, 8, src, lane);
+              diamond_field(F, P, R.ws.win, plan.wx0, plan.wy0, mbx, mby, cxp, cyp, bp, 8, src, lane, rounds);
           if (lane == 0) {
             mo.sad_zero = z;
             mo.whole = w;
+            s_rounds = rounds;
           }
-        } else if (warp == 5) {
-          const int er = eighth(cen.nearest.row), ec = eighth(cen.nearest.col);
-          const uint32_t sv = subpel_sad(R.halo_nearest, HS, ec & 7, er & 7, src, wt[5].temp, lane);
-          if (lane == 0) mo.sad_nearest = sv;
-        } else if (warp == 6) {
-          const int er = eighth(cen.near_.row), ec = eighth(cen.near_.col);
-          const uint32_t sv = subpel_sad(R.halo_near, HS, ec & 7, er & 7, src, wt[6].temp, lane);
-          if (lane == 0) mo.sad_near = sv;
         } else if (warp == 8) {
           // The proposed vector's exact SAD (a second NEWMV candidate).
           vp8a_mv pv = {0, 0};
@@ -1253,11 +1366,41 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
           dsplit = a.lambda * (bb(t, p[0], 1) + bb(t, p[1], 1) + bb(t, p[2], 1) + bb(t, p[3], 1));
         }
         main_sync();
+        vp8a_search_result whole = mo.whole;
+        if (s_rounds > 0) {
+          // The walk reached the field's edge: the rest of it over a second
+          // field around that position (the first took at least FR rounds, so
+          // the second covers the others), by every warp alike.
+          field2_rows(R.ws.win, src, F, mbx + whole.mv.col / 4 - plan.wx0, mby + whole.mv.row / 4 - plan.wy0, mt);
+          main_sync();
+          field2_sums(F, mt, MAIN_THREADS);
+          main_sync();
+          int x = 0, y = 0, rounds = s_rounds;
+          walk_field(F.full2, x, y, whole.sad, rounds);
+          whole.mv.row = (int16_t)(whole.mv.row + 4 * y);
+          whole.mv.col = (int16_t)(whole.mv.col + 4 * x);
+        }
+        // The first strictly better candidate in order around `from` = the
+        // smallest (SAD, index) if its SAD beats the centre's; every warp of
+        // the group finds it.
+        auto best_of = [&](vp8a_search_result from, int step) {
+          const uint32_t m = __reduce_min_sync(FULL, lane < 8 ? (cand_sad[lane] << 3) | (uint32_t)lane : ~0u);
+          if ((m >> 3) < from.sad) {
+            const int q = (int)(m & 7u);
+            from.sad = m >> 3;
+            from.mv.row = clamp_component(from.mv.row + step * cand_dr(q));
+            from.mv.col = clamp_component(from.mv.col + step * cand_dc(q));
+          }
+          return from;
+        };
+        // Candidates 2 slot and 2 slot + 1.
+        auto store_pair = [&](uint32_t both) {
+          if (lane < 2) cand_sad[2 * slot + lane] = lane ? both >> 16 : both & 0xffffu;
+        };
         // half_pixel_refine_luma around the whole-pel result: planes shared
-        // by the group, candidates spread over its warps, first strict
-        // minimum in order. For a whole-pel centre inside [-1020, 1020] no
-        // candidate is clamped.
-        const vp8a_mv hc = mo.whole.mv;
+        // by the group, two candidates a warp. For a whole-pel centre inside
+        // [-1020, 1020] no candidate is clamped.
+        const vp8a_mv hc = whole.mv;
         const int hbx = mbx + hc.col / 4 - plan.wx0, hby = mby + hc.row / 4 - plan.wy0;
         const bool whole_c = hc.row >= -1020 && hc.row <= 1020 && hc.col >= -1020 && hc.col <= 1020 &&
                              !(hc.row & 3) && !(hc.col & 3);
@@ -1265,6 +1408,8 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
         const int hix = mbx + hc.col / 4, hiy = mby + hc.row / 4;
         const bool gplanes = spb != nullptr && whole_c && sp_inside(P, hix - 1, hiy - 1) && sp_inside(P, hix, hiy);
         const bool planes = whole_c && hbx >= 3 && hby >= 3 && hbx + 19 <= WS && hby + 19 <= WS;
+        uint8_t* const pl = R.ws.temp;  // the sub-pel planes
+        vp8a_search_result half;
         if (gplanes || planes) {
           if (gplanes) {
             // Candidate q's prediction is a block of the precomputed plane
@@ -1276,44 +1421,26 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
               if ((mt & 15) == 0) cand_sad[q] = sv;
             }
           } else {
-            half_planes_hv(R.ws, hbx, hby, mt);
+            if (slot < 4) half_plane_h(R.ws.win, pl, hbx, hby, mt, 128);
+            else half_plane_v(R.ws.win, pl, hbx, hby, lane);
             main_sync();
-            half_planes_d(R.ws, mt);
+            half_plane_d(pl, mt, MAIN_THREADS);
             main_sync();
-            for (int q = slot; q < 8; q += MAIN_WARPS) {
-              const uint32_t sv = half_cand_sad(R.ws, q, src, lane);
-              if (lane == 0) cand_sad[q] = sv;
-            }
+            if (slot < 4) store_pair(half_cand_sads(pl, src, slot, lane));
           }
           main_sync();
+          half = best_of(whole, 2);
+        } else {
           if (warp == 0) {
-            // The first strictly better candidate in order = the smallest
-            // (SAD, index) if its SAD beats the centre's.
-            const uint32_t m = __reduce_min_sync(FULL, lane < 8 ? (cand_sad[lane] << 3) | (uint32_t)lane : ~0u);
-            if (lane == 0) {
-              vp8a_mv best = hc;
-              uint32_t best_sad = mo.whole.sad;
-              const int q = (int)(m & 7u);
-              if ((m >> 3) < best_sad) {
-                best_sad = m >> 3;
-                best.row = (int16_t)(hc.row + 2 * cand_dr(q));
-                best.col = (int16_t)(hc.col + 2 * cand_dc(q));
-              }
-              mo.half = vp8a_search_result{best, best_sad};
-              s_qok = quarter_geom(best, mbx, mby, plan.wx0, plan.wy0, s_qg);
-            }
+            half = refine(P, R.ws, plan.wx0, plan.wy0, mbx, mby, hc, 2, src, lane, whole.sad);
+            if (lane == 0) mo.half = half;
           }
-        } else if (warp == 0) {
-          const vp8a_search_result h = refine(P, R.ws, plan.wx0, plan.wy0, mbx, mby, hc, 2, src, lane, mo.whole.sad);
-          if (lane == 0) {
-            mo.half = h;
-            s_qok = quarter_geom(h.mv, mbx, mby, plan.wx0, plan.wy0, s_qg);
-          }
+          main_sync();
+          half = mo.half;
         }
-        main_sync();
         // quarter_pixel_refine_luma around the half-pel result; the centre's
         // SAD is the half-pel result's.
-        const vp8a_mv qc = mo.half.mv;
+        const vp8a_mv qc = half.mv;
         // The eight candidates' blocks span the integer offsets of the
         // columns qc.col - 1 .. qc.col + 1 and rows qc.row - 1 .. qc.row + 1.
         const bool gq = spb != nullptr &&
@@ -1322,6 +1449,7 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
                         sp_inside(P, mbx + (eighth(clamp_component(qc.col + 1)) >> 3),
                                   mby + (eighth(clamp_component(qc.row + 1)) >> 3));
         if (gq) {
+          main_sync();  // the half-pel candidates' SADs have been read
           if (mt < 128) {
             const int q = mt >> 4;
             const int er = eighth(clamp_component(qc.row + cand_dr(q))), ec = eighth(clamp_component(qc.col + cand_dc(q)));
@@ -1329,15 +1457,17 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
                                              mbx + (ec >> 3), mby + (er >> 3), src, mt & 15);
             if ((mt & 15) == 0) cand_sad[q] = sv;
           }
-        } else if (s_qok) {
-          uint8_t* qh = R.ws.temp;  // the six-tap scratch and half planes are free now
-          quarter_planes_h(R.ws.win, qh, s_qg, mt);
+        } else if (quarter_inside(qc, mbx, mby, plan.wx0, plan.wy0)) {
+          int iy0, f;
+          quarter_pos(qc.row - 1, mby, plan.wy0, iy0, f);
+          iy0 -= 2;  // first plane row (window coordinates)
+          // The half-pel planes are free: their candidates are scored.
+          auto taps = [&](int fr) { return taps_of(tap_tab, fr); };
+          quarter_planes_h(R.ws.win, pl, taps, qc, mbx, plan.wx0, iy0, mt, MAIN_THREADS);
           main_sync();
-          if (mt < 128) {
-            const uint32_t sv = quarter_vsad(qh, s_qg, src, mt);
-            if ((mt & 15) == 0) cand_sad[mt >> 4] = sv;
-          }
+          if (slot < 4) store_pair(quarter_cand_sads(pl, src, taps, qc, mby, plan.wy0, iy0, slot, lane));
         } else {
+          main_sync();
           for (int q = slot; q < 8; q += MAIN_WARPS) {
             const int16_t rr = clamp_component(qc.row + cand_dr(q)), cc = clamp_component(qc.col + cand_dc(q));
             const uint32_t sv =
@@ -1347,21 +1477,15 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
         }
         main_sync();
         if (warp == 0) {
-          const uint32_t m = __reduce_min_sync(FULL, lane < 8 ? (cand_sad[lane] << 3) | (uint32_t)lane : ~0u);
+          const vp8a_search_result quarter = best_of(half, 1);
           if (lane == 0) {
-            vp8a_mv best = qc;
-            uint32_t best_sad = mo.half.sad;
-            const int q = (int)(m & 7u);
-            if ((m >> 3) < best_sad) {
-              best_sad = m >> 3;
-              best.row = clamp_component(qc.row + cand_dr(q));
-              best.col = clamp_component(qc.col + cand_dc(q));
-            }
-            mo.quarter = vp8a_search_result{best, best_sad};
+            mo.whole = whole;
+            mo.half = half;
+            mo.quarter = quarter;
           }
         }
       }
-      __syncthreads();
+      search_sync();
       if (tid == 0) {
         // pick_mb_for_ref's mode decision (src/encoder.rs:8598-8652).
         // Every product lambda * bits below is the reference's own; the ones
@@ -1454,58 +1578,37 @@ __global__ void __launch_bounds__(AN_THREADS, 2)
         mydec.mode = mode;
         mydec.pid = pid;
       }
-      __syncthreads();
-      // Into rank 0, word by word; the sub-MVs and sub-MV modes come from
-      // the chosen partition (ZERO vectors and ZERO4X4 modes otherwise).
-      if (tid < (int)(sizeof(RefDec) / 4)) {
+      search_sync();
+      // To every CTA of the cluster, eight bytes a thread; the sub-MVs and
+      // sub-MV modes come from the chosen partition (ZERO vectors and ZERO4X4
+      // modes otherwise).
+      constexpr int DW = sizeof(RefDec) / 8;
+      if (tid < DW * csize) {
+        const int rank = tid / DW, w = tid - rank * DW;
         const bool spl = mydec.mode == VP8A_MODE_SPLIT;
-        uint32_t w;
-        if (tid < 7) w = ((const uint32_t*)&mydec)[tid];
-        else if (tid < 23) w = spl ? ((const uint32_t*)splits[mydec.pid].split_mvs)[tid - 7] : 0u;
-        else if (tid < 27) w = spl ? ((const uint32_t*)splits[mydec.pid].modes)[tid - 23] : 0x01010101u * VP8A_SUBMV_ZERO;
-        else w = 0u;
-        dec_slot[tid] = w;
-      }
-      cl.sync();
-      if (k == 0 && warp == 0) {
-        // decide_mb_exhaustive's reference comparison: first strict minimum
-        // of J + ref_frame_tree_bits in reference order (every lane), then
-        // the decision and census records written word by word.
-        double best_total = __longlong_as_double(0x7ff0000000000000LL);
-        int best_k = -1;
-        for (int q = 0; q < a.n_refs; q++)
-          if (decs[q].total < best_total) {
-            best_total = decs[q].total;
-            best_k = q;
-          }
-        const uint32_t* b = (const uint32_t*)&decs[best_k < 0 ? 0 : best_k];
-        const bool ok = best_k >= 0;
-        const uint32_t mode = ok ? (uint32_t)decs[best_k].mode : 0u, pid = ok ? (uint32_t)decs[best_k].pid : 0u;
-        const uint32_t id = ok ? (uint32_t)a.ref_ids[best_k] : 0u, spl = mode == VP8A_MODE_SPLIT;
-        uint32_t* dw = (uint32_t*)(a.dec + (size_t)r * a.mb_cols + c);
-        uint32_t* iw = (uint32_t*)(a.infos + (size_t)r * a.mb_cols + c);
-        if (lane < 26) {  // vp8a_mb_decision
-          uint32_t w;
-          if (lane == 0) w = id | (mode & 0xffu) << 8 | (pid & 0xffu) << 16;
-          else if (lane == 1) w = b[4];         // mv
-          else if (lane < 6) w = b[lane - 2];   // j, total
-          else w = b[lane + 1];                 // split_mvs, submv_modes
-          dw[lane] = ok ? w : 0u;
+        const uint32_t* sm = (const uint32_t*)splits[spl ? mydec.pid : 0].split_mvs;
+        const uint32_t* smo = (const uint32_t*)splits[spl ? mydec.pid : 0].modes;
+        uint32_t v[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const int x = 2 * w + i;
+          v[i] = x < 7 ? ((const uint32_t*)&mydec)[x]
+                       : (x < 23 ? (spl ? sm[x - 7] : 0u)
+                                 : (x < 27 ? (spl ? smo[x - 23] : 0x01010101u * VP8A_SUBMV_ZERO) : 0u));
         }
-        if (lane < 18) {  // the census record
-          uint32_t w;
-          if (lane == 0) w = id | spl << 8 | spl << 16;
-          else if (lane == 1) w = b[4];
-          else w = b[lane + 5];
-          iw[lane] = ok ? w : 0u;
-        }
-        __syncwarp();
-        // The release orders the warp's record writes before the count.
-        if (lane == 0) st_release(&a.progress[r], (unsigned)(c + 1));
+        uint32_t at, bar;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;"
+            : "=r"(at)
+            : "r"(smem_at(&feed.decs[n % DEC_RING][k]) + 8 * w), "r"(rank));
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_at(&feed.dec_bar[n % DEC_RING])), "r"(rank));
+        asm volatile(
+            "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(at),
+            "r"(v[0]), "r"(v[1]), "r"(bar)
+            : "memory");
       }
-      // The next MB's first cluster barrier orders these results.
     }
   }
+  cl.sync();  // no CTA leaves while another may write to it
 }
 
 }  // namespace
@@ -1668,7 +1771,7 @@ vp8a_status launch_analysis(vp8a_ctx* ctx, int n_refs, const AnArgs& a0, const A
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(AN_THREADS);
+  cfg.blockDim = dim3(AN_THREADS + 32);
   cfg.dynamicSmemBytes = (size_t)pad;
   cfg.stream = ctx->stream;
   cfg.attrs = attr;

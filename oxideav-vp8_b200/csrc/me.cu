@@ -41,8 +41,12 @@ __global__ void __launch_bounds__(ME_WARPS * 32) me_batch_kernel(MeBatch a) {
   WarpScratch& S = scratch[warp];
   uint8_t* src = srcs[warp];
   const uint8_t* gsrc = a.src_mbs + (size_t)item * 256;
+  if (((uintptr_t)a.src_mbs & 7) == 0) {
+    *(uint2*)(src + lane * 8) = *(const uint2*)(gsrc + lane * 8);
+  } else {
 #pragma unroll
-  for (int k = 0; k < 8; k++) src[lane + 32 * k] = gsrc[lane + 32 * k];
+    for (int k = 0; k < 8; k++) src[lane + 32 * k] = gsrc[lane + 32 * k];
+  }
   const int mbx = (int)a.mb_xy[2 * item] * 16, mby = (int)a.mb_xy[2 * item + 1] * 16;
   const vp8a_mv c = a.mvs[item];
   __syncwarp();
@@ -74,14 +78,14 @@ __global__ void __launch_bounds__(ME_WARPS * 32) me_batch_kernel(MeBatch a) {
       r = refine(a.P, S, wx0, wy0, mbx, mby, c, 2, src, lane);
     if (lane == 0) a.out0[item] = r;
   } else if (MODE == MODE_QUARTER) {
-    vp8a_search_result r = refine(a.P, S, wx0, wy0, mbx, mby, c, 1, src, lane);
+    vp8a_search_result r = quarter_refine(a.P, S, wx0, wy0, mbx, mby, c, src, lane);
     if (lane == 0) a.out0[item] = r;
   } else {
     vp8a_search_result w = diamond(a.P, S, wx0, wy0, mbx, mby, c, a.max_iters, src, lane);
     vp8a_search_result h;
     if (!half_refine_planes(S, wx0, wy0, mbx, mby, w.mv, src, lane, &h))
       h = refine(a.P, S, wx0, wy0, mbx, mby, w.mv, 2, src, lane);
-    vp8a_search_result q = refine(a.P, S, wx0, wy0, mbx, mby, h.mv, 1, src, lane, h.sad);
+    vp8a_search_result q = quarter_refine(a.P, S, wx0, wy0, mbx, mby, h.mv, src, lane, h.sad);
     if (lane == 0) {
       if (a.out0) a.out0[item] = w;
       if (a.out1) a.out1[item] = h;

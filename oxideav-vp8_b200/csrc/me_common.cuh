@@ -33,10 +33,7 @@ struct __align__(16) WarpScratch {
   uint8_t win[WIN_BYTES];        // 1616
   uint8_t temp[21 * 16 + 16];    // 352
   uint8_t halo[21 * 24 + 24];    // 528
-  // Half-pel planes around a whole-pel centre: H 22x17, V 17x16, D 17x17.
-  uint8_t hp[22 * 17 + 10];      // 384
-  uint8_t vp[17 * 16 + 16];      // 288
-  uint8_t dp[17 * 17 + 15];      // 304
+  uint8_t more[192];             // with temp and halo: the shared sub-pel planes
 };
 static_assert(sizeof(WarpScratch) % 16 == 0, "WarpScratch must keep 16-byte multiples");
 
@@ -55,9 +52,79 @@ __device__ __forceinline__ void load8u(const uint8_t* p, uint32_t& o0, uint32_t&
   o1 = __funnelshift_r(w1, w2, sh);
 }
 
+// ------------------------------------------------------- packed six-tap
+//
+// The §18.3 filters run four pixels a thread, two to a register (16-bit
+// fields), with the pixels read four to a word: a fifth of the loads and a
+// third of the arithmetic of one pixel a thread.
+__device__ __forceinline__ uint32_t pk16(int v) { return (uint32_t)(uint16_t)(int16_t)v * 0x00010001u; }
+// Bytes 1 and 3 as fields.
+__device__ __forceinline__ uint32_t odd_bytes(uint32_t x) { return __byte_perm(x, 0u, 0x4341); }
+// (t >> 7) - 64 clamped to 0..255, per field: t is the filter's sum plus 64 + 64 *
+// 128, which keeps every field in 0..65535 (the taps' negative sums exceed -19 *
+// 255, the positive ones stay below 160 * 255).
+constexpr int TAP_BIAS = 64 + 64 * 128;
+__device__ __forceinline__ uint32_t tap_result(uint32_t t) {
+  return __viaddmin_s16x2_relu((t >> 7) & 0x01ff01ffu, pk16(-64), pk16(255));
+}
+// The half-pel taps 3, -16, 77, 77, -16, 3.
+__device__ __forceinline__ uint32_t half6(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f) {
+  return tap_result((c + d) * 77u + pk16(TAP_BIAS) + (a + f) * 3u - (b + e) * 16u);
+}
+struct Taps {
+  int f[6];
+};
+__device__ __forceinline__ uint32_t six(const Taps& k, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e,
+                                        uint32_t f) {
+  return tap_result(pk16(TAP_BIAS) + a * (uint32_t)k.f[0] + b * (uint32_t)k.f[1] + c * (uint32_t)k.f[2] +
+                    d * (uint32_t)k.f[3] + e * (uint32_t)k.f[4] + f * (uint32_t)k.f[5]);
+}
+__device__ __forceinline__ Taps taps_const(int f) {
+  const int* t = c_sixtap[f];
+  return Taps{{t[0], t[1], t[2], t[3], t[4], t[5]}};
+}
+// Twelve bytes of a shared-memory row from byte offset `o` on, as words.
+__device__ __forceinline__ void row_words(const uint8_t* row, int o, uint32_t& u0, uint32_t& u1, uint32_t& u2) {
+  const uint32_t* w = (const uint32_t*)(row + (o & ~3));
+  const unsigned sh = (unsigned)(o & 3) * 8u;
+  const uint32_t w1 = w[1], w2 = w[2];
+  u0 = __funnelshift_r(w[0], w1, sh);
+  u1 = __funnelshift_r(w1, w2, sh);
+  u2 = __funnelshift_r(w2, w[3], sh);
+}
+__device__ __forceinline__ uint32_t row_word(const uint8_t* row, int o) {
+  const uint32_t* w = (const uint32_t*)(row + (o & ~3));
+  return __funnelshift_r(w[0], w[1], (unsigned)(o & 3) * 8u);
+}
+// Four outputs of a horizontal filter over the bytes of u0, u1, u2: output i
+// takes bytes i .. i + 5.
+template <class F>
+__device__ __forceinline__ uint32_t filter_row(uint32_t u0, uint32_t u1, uint32_t u2, F&& tap6) {
+  constexpr uint32_t M = 0x00ff00ffu;
+  const uint32_t s2 = __byte_perm(u0, u1, 0x5432), s6 = __byte_perm(u1, u2, 0x5432);
+  const uint32_t p1 = odd_bytes(u0), p2 = s2 & M, p3 = odd_bytes(s2), p4 = u1 & M, p5 = odd_bytes(u1);
+  return tap6(p1, p2, p3, p4, p5, s6 & M) * 256u + tap6(u0 & M, p1, p2, p3, p4, p5);
+}
+
+// Whether the plane can be read as aligned words.
+__device__ __forceinline__ bool word_plane(const MePlane& P) {
+  return (((uintptr_t)P.plane | (uintptr_t)P.stride) & 3) == 0;
+}
+
 // Fill a WS x WS window whose top-left is plane pixel (x0, y0), clamping
-// every coordinate into the plane.
+// every coordinate into the plane: word by word where a row's words lie
+// inside it, byte by byte at the edges.
 __device__ __forceinline__ void load_window(const MePlane& P, uint8_t* win, int x0, int y0, int lane) {
+  if (word_plane(P) && x0 >= 0 && (x0 & ~3) + WS + 4 <= P.width) {
+    const int sh = x0 & 3, xa = x0 - sh;
+    for (int t = lane; t < WS * (WS / 4); t += 32) {
+      const int r = t / (WS / 4), w = t - r * (WS / 4);
+      const uint32_t* p = (const uint32_t*)(P.plane + (size_t)clampi(y0 + r, 0, P.height - 1) * P.stride + xa) + w;
+      *(uint32_t*)(win + r * WS + 4 * w) = __funnelshift_r(__ldg(p), __ldg(p + 1), 8u * (unsigned)sh);
+    }
+    __syncwarp();
+    return;
+  }
   for (int r = 0; r < WS; r++) {
     int y = clampi(y0 + r, 0, P.height - 1);
     const uint8_t* row = P.plane + (size_t)y * P.stride;
@@ -83,6 +150,15 @@ __device__ __forceinline__ uint32_t sad_global16(const MePlane& P, int x0, int y
   int y = clampi(y0 + row, 0, P.height - 1);
   const uint8_t* pr = P.plane + (size_t)y * P.stride;
   uint32_t s = 0;
+  if (word_plane(P) && x0 >= 0 && (x0 & ~3) + 20 <= P.width) {
+    const int x = x0 + c0;
+    const uint32_t* w = (const uint32_t*)(pr + (x & ~3));
+    const unsigned sh = (unsigned)(x & 3) * 8u;
+    const uint32_t w1 = __ldg(w + 1);
+    const uint2 sv = *(const uint2*)(src + row * 16 + c0);
+    s = __vsadu4(__funnelshift_r(__ldg(w), w1, sh), sv.x) + __vsadu4(__funnelshift_r(w1, __ldg(w + 2), sh), sv.y);
+    return __reduce_add_sync(FULL, s);
+  }
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     int d = (int)pr[clampi(x0 + c0 + k, 0, P.width - 1)] - (int)src[row * 16 + c0 + k];
@@ -100,37 +176,39 @@ __device__ __forceinline__ uint32_t sad_whole_at(const MePlane& P, const uint8_t
 }
 
 // §18.3 two-pass six-tap prediction SAD (sixtap_mb_luma,
-// src/motion_comp.rs:902-1057) from a 21x21 halo at `h` (stride hs; block
-// origin at (2, 2)). The horizontal pass keeps its 8-bit clamp; a pass
-// whose fraction is 0 is the identity and is skipped (the reference's own
-// identity elision, src/motion_comp.rs:960-1007).
+// src/motion_comp.rs:902-1057) from a 21x21 halo at `h` (stride hs, a multiple
+// of 4; block origin at (2, 2); reads up to 27 bytes of a row from h on). The
+// horizontal pass keeps its 8-bit clamp; a pass whose fraction is 0 is the
+// identity (the reference's own identity elision, src/motion_comp.rs:960-1007),
+// which the taps 0, 0, 128, 0, 0, 0 reproduce.
 __device__ __forceinline__ uint32_t subpel_sad(const uint8_t* h, int hs, int mx, int my, const uint8_t* src,
                                                uint8_t* temp, int lane) {
-  const int c = lane & 15;
-  if (mx) {
-    const int* fh = c_sixtap[mx];
-    for (int r = lane >> 4; r < 21; r += 2) {
-      const uint8_t* p = h + r * hs + c;
-      temp[r * 16 + c] = (uint8_t)interp6(fh, p[0], p[1], p[2], p[3], p[4], p[5]);
-    }
-    __syncwarp();
+  const int o = (int)((uintptr_t)h & 3);
+  const Taps fh = taps_const(mx), fv = taps_const(my);
+#pragma unroll 1
+  for (int t = lane; t < 21 * 4; t += 32) {
+    const int r = t >> 2, j = t & 3;
+    uint32_t u0, u1, u2;
+    row_words(h - o + r * hs, o + 4 * j, u0, u1, u2);
+    *(uint32_t*)(temp + t * 4) = filter_row(u0, u1, u2, [&](uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e,
+                                                            uint32_t f) { return six(fh, a, b, c, d, e, f); });
   }
-  const int* fv = c_sixtap[my];
-  const int r0 = (lane >> 4) * 8;
+  __syncwarp();
+  // Word column j, rows 2 strip and 2 strip + 1.
+  const int j = lane & 3, r0 = (lane >> 2) * 2;
+  uint32_t e[7], d[7];
+#pragma unroll
+  for (int k = 0; k < 7; k++) {
+    const uint32_t w = *(const uint32_t*)(temp + (r0 + k) * 16 + j * 4);
+    e[k] = w & 0x00ff00ffu;
+    d[k] = odd_bytes(w);
+  }
   uint32_t s = 0;
-#pragma unroll 2
-  for (int r = r0; r < r0 + 8; r++) {
-    int v;
-    if (mx) {
-      const uint8_t* t = temp + r * 16 + c;
-      v = my ? interp6(fv, t[0], t[16], t[32], t[48], t[64], t[80]) : t[32];
-    } else {
-      const uint8_t* p = h + r * hs + c + 2;
-      v = my ? interp6(fv, p[0], p[hs], p[2 * hs], p[3 * hs], p[4 * hs], p[5 * hs]) : p[2 * hs];
-    }
-    int d = v - (int)src[r * 16 + c];
-    s += (uint32_t)(d < 0 ? -d : d);
-  }
+#pragma unroll
+  for (int r = 0; r < 2; r++)
+    s += __vsadu4(six(fv, d[r], d[r + 1], d[r + 2], d[r + 3], d[r + 4], d[r + 5]) * 256u +
+                      six(fv, e[r], e[r + 1], e[r + 2], e[r + 3], e[r + 4], e[r + 5]),
+                  *(const uint32_t*)(src + (r0 + r) * 16 + j * 4));
   __syncwarp();
   return __reduce_add_sync(FULL, s);
 }
@@ -275,69 +353,229 @@ __device__ __forceinline__ vp8a_search_result refine(const MePlane& P, WarpScrat
   return res;
 }
 
-// The eight half-pel candidates around a whole-pel centre share three
-// planes — horizontal (H), vertical (V) and horizontal-then-vertical (D)
-// half-pel samples — so each six-tap output is computed once per MB instead
-// of once per candidate; every candidate's prediction is a 16x16 sub-block
-// of one plane, byte-identical to its own two-pass synthesis (same taps,
-// same 8-bit intermediate, same edge-clamped source). half_plane_sads fills
-// sads[k] for the offsets (row, col) = (-1,-1) (-1,0) (-1,1) (0,-1) (0,1)
-// (1,-1) (1,0) (1,1) half-pels, in that order (the order of
-// half_pixel_refine_luma, src/motion_search.rs:589-598, and of
-// sub_pixel_refine, src/encoder/inter_search.rs:520-535), and returns false
-// when the window does not cover the planes.
+// Offsets (row, col) of the eight refinement candidates in the reference's
+// order: (-1,-1) (-1,0) (-1,1) (0,-1) (0,1) (1,-1) (1,0) (1,1).
+__device__ __forceinline__ int cand_dr(int k) { return (k < 3) ? -1 : (k < 5 ? 0 : 1); }
+__device__ __forceinline__ int cand_dc(int k) { return (k == 0 || k == 3 || k == 5) ? -1 : ((k == 1 || k == 6) ? 0 : 1); }
+
+// The eight half-pel candidates around a whole-pel centre whose block origin
+// in the window is (bx, by) share three planes of half-pel samples: H (22 rows
+// x 17, row r = window row by - 3 + r, sample i at bx + i - 1/2), V (17 x 16,
+// at by + r - 1/2) and D (17 x 17, vertical over H), so each six-tap output is
+// computed once per MB instead of once per candidate; every candidate's
+// prediction is a 16 x 16 block of one plane, byte-identical to its own
+// two-pass synthesis (same taps, same 8-bit intermediate, same edge-clamped
+// source). Rows of 20, 16 and 20 bytes. The functions below give thread t of n
+// its share.
+constexpr int HP_H = 0, HP_V = HP_H + 22 * 20, HP_D = HP_V + 17 * 16, HP_BYTES = HP_D + 17 * 20;
+constexpr int QP_BYTES = 3 * 22 * 16;  // the quarter-pel planes
+constexpr int PLANE_BYTES = sizeof(WarpScratch) - offsetof(WarpScratch, temp);
+static_assert(HP_BYTES + 16 <= PLANE_BYTES && QP_BYTES <= PLANE_BYTES, "the planes fit behind the window");
+static_assert(offsetof(WarpScratch, temp) % 16 == 0, "the planes are read as words");
+
+// H: one (row, word) a thread and round.
+__device__ __forceinline__ void half_plane_h(const uint8_t* win, uint8_t* hp, int bx, int by, int t, int n) {
+#pragma unroll 1
+  for (; t < 22 * 5; t += n) {
+    const int r = t / 5, j = t - 5 * r;
+    uint32_t u0, u1, u2;
+    row_words(win + (by - 3 + r) * WS, bx - 3 + 4 * j, u0, u1, u2);
+    *(uint32_t*)(hp + HP_H + t * 4) = filter_row(u0, u1, u2, half6);
+  }
+}
+// V, on one warp: one word column and two or three rows a lane.
+__device__ __forceinline__ void half_plane_v(const uint8_t* win, uint8_t* hp, int bx, int by, int lane) {
+  {
+    const int j = lane & 3, strip = lane >> 2, r0 = 2 * strip + (strip > 0), r1 = 2 * strip + 3;
+    const uint8_t* p = win + (by + r0 - 3) * WS;
+    uint32_t e[6], o[6];
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+      const uint32_t w = row_word(p + k * WS, bx + 4 * j);
+      e[k] = w & 0x00ff00ffu;
+      o[k] = odd_bytes(w);
+    }
+    for (int r = r0; r < r1; r++, p += WS) {
+      const uint32_t w = row_word(p + 5 * WS, bx + 4 * j);
+      e[5] = w & 0x00ff00ffu;
+      o[5] = odd_bytes(w);
+      *(uint32_t*)(hp + HP_V + r * 16 + j * 4) =
+          half6(o[0], o[1], o[2], o[3], o[4], o[5]) * 256u + half6(e[0], e[1], e[2], e[3], e[4], e[5]);
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        e[k] = e[k + 1];
+        o[k] = o[k + 1];
+      }
+    }
+  }
+}
+
+// The D plane, from H (after H is complete): one (row, word) a thread and
+// round.
+__device__ __forceinline__ void half_plane_d(uint8_t* hp, int t, int n) {
+#pragma unroll 1
+  for (; t < 17 * 5; t += n) {
+    const uint8_t* p = hp + HP_H + t * 4;
+    uint32_t e[6], o[6];
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      const uint32_t w = *(const uint32_t*)(p + k * 20);
+      e[k] = w & 0x00ff00ffu;
+      o[k] = odd_bytes(w);
+    }
+    *(uint32_t*)(hp + HP_D + t * 4) =
+        half6(o[0], o[1], o[2], o[3], o[4], o[5]) * 256u + half6(e[0], e[1], e[2], e[3], e[4], e[5]);
+  }
+}
+
+// Sums of the warp's half-warps (each below 65536) in one reduction: lanes 0-15
+// in the low half of the result.
+__device__ __forceinline__ uint32_t pair_sum(uint32_t s, int lane) {
+  return __reduce_add_sync(FULL, lane < 16 ? s : s << 16);
+}
+
+// SADs of the half-pel candidates 2 slot and 2 slot + 1 (one warp): row lane
+// & 15 of candidate k.
+__device__ __forceinline__ uint32_t half_cand_sads(const uint8_t* hp, const uint8_t* src, int slot, int lane) {
+  const int k = 2 * slot + (lane >> 4), row = lane & 15, dy = cand_dr(k), dx = cand_dc(k), cx = dx > 0, cy = dy > 0;
+  const int at = dy == 0 ? HP_H + (3 + row) * 20 : (dx == 0 ? HP_V + (cy + row) * 16 : HP_D + (cy + row) * 20);
+  const uint32_t* w = (const uint32_t*)(hp + at);
+  const uint4 sv = *(const uint4*)(src + row * 16);
+  const unsigned sh = cx * 8u;
+  const uint32_t w1 = w[1], w2 = w[2], w3 = w[3];
+  const uint32_t s = __vsadu4(__funnelshift_r(w[0], w1, sh), sv.x) + __vsadu4(__funnelshift_r(w1, w2, sh), sv.y) +
+                     __vsadu4(__funnelshift_r(w2, w3, sh), sv.z) + __vsadu4(__funnelshift_r(w3, w[4], sh), sv.w);
+  return pair_sum(s, lane);
+}
+
+// quarter_pixel_refine_luma's eight candidates around `qc` share three
+// horizontal six-tap planes, one per candidate column (qc.col - 1, qc.col,
+// qc.col + 1 quarter-pels; fraction 0 is the unfiltered pixel, which the taps 0,
+// 0, 128, 0, 0, 0 reproduce). Each candidate's prediction is then its vertical
+// pass over its column's plane: the same taps, the same 8-bit intermediate and
+// the same edge-clamped source as its own two-pass synthesis.
+// Integer position (in the window) and eighth-pel fraction of component v.
+__device__ __forceinline__ void quarter_pos(int v, int mb, int w0, int& i, int& f) {
+  const int e = eighth(clamp_component(v));
+  i = mb + (e >> 3) - w0;
+  f = e & 7;
+}
+// Whether the window covers every candidate's halo.
+__device__ __forceinline__ bool quarter_inside(vp8a_mv qc, int mbx, int mby, int wx0, int wy0) {
+  int x0, x1, y0, y1, f;
+  quarter_pos(qc.col - 1, mbx, wx0, x0, f);
+  quarter_pos(qc.col + 1, mbx, wx0, x1, f);
+  quarter_pos(qc.row - 1, mby, wy0, y0, f);
+  quarter_pos(qc.row + 1, mby, wy0, y1, f);
+  return x0 >= 2 && x1 + 19 <= WS && y0 >= 2 && y0 + 20 <= WS && y1 - y0 <= 1;
+}
+// Horizontal planes: plane k's row rr (window row iy0 + rr) at qh + (k * 22 +
+// rr) * 16; one (plane, row, word) a thread and round.
+template <class TapsOf>
+__device__ __forceinline__ void quarter_planes_h(const uint8_t* win, uint8_t* qh, TapsOf&& taps_of, vp8a_mv qc, int mbx,
+                                                 int wx0, int iy0, int t, int n) {
+#pragma unroll 1
+  for (; t < 3 * 22 * 4; t += n) {
+    const int k = t / 88, rr = (t - 88 * k) >> 2, j = t & 3;
+    int ix, fx;
+    quarter_pos(qc.col + k - 1, mbx, wx0, ix, fx);
+    const Taps f = taps_of(fx);
+    uint32_t u0, u1, u2;
+    row_words(win + (iy0 + rr) * WS, ix - 2 + 4 * j, u0, u1, u2);
+    *(uint32_t*)(qh + t * 4) = filter_row(u0, u1, u2, [&](uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e,
+                                                          uint32_t g) { return six(f, a, b, c, d, e, g); });
+  }
+}
+
+// Vertical passes and SADs of candidates 2 slot and 2 slot + 1 (one warp): lane
+// (candidate, strip of four rows, word).
+template <class TapsOf>
+__device__ __forceinline__ uint32_t quarter_cand_sads(const uint8_t* qh, const uint8_t* src, TapsOf&& taps_of,
+                                                      vp8a_mv qc, int mby, int wy0, int iy0, int slot, int lane) {
+  const int k = 2 * slot + (lane >> 4), strip = (lane >> 2) & 3, j = lane & 3;
+  int iy, fy;
+  quarter_pos(qc.row + cand_dr(k), mby, wy0, iy, fy);
+  const Taps f = taps_of(fy);
+  const uint8_t* p = qh + ((cand_dc(k) + 1) * 22 + iy - 2 - iy0 + strip * 4) * 16 + j * 4;
+  uint32_t e[6], o[6], s = 0;
+#pragma unroll
+  for (int i = 0; i < 5; i++) {
+    const uint32_t w = *(const uint32_t*)(p + i * 16);
+    e[i] = w & 0x00ff00ffu;
+    o[i] = odd_bytes(w);
+  }
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    const uint32_t w = *(const uint32_t*)(p + (r + 5) * 16);
+    e[5] = w & 0x00ff00ffu;
+    o[5] = odd_bytes(w);
+    s += __vsadu4(six(f, o[0], o[1], o[2], o[3], o[4], o[5]) * 256u + six(f, e[0], e[1], e[2], e[3], e[4], e[5]),
+                  *(const uint32_t*)(src + (strip * 4 + r) * 16 + j * 4));
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+      e[i] = e[i + 1];
+      o[i] = o[i + 1];
+    }
+  }
+  return pair_sum(s, lane);
+}
+
+// half_pixel_refine_luma's candidates (src/motion_search.rs:589-598; also of
+// sub_pixel_refine, src/encoder/inter_search.rs:520-535) on one warp: sads[k] for
+// the offsets (row, col) = (-1,-1) (-1,0) (-1,1) (0,-1) (0,1) (1,-1) (1,0) (1,1)
+// half-pels; false when the window does not cover the planes.
 __device__ __forceinline__ bool half_plane_sads(WarpScratch& S, int wx0, int wy0, int mbx, int mby, vp8a_mv center,
                                                 const uint8_t* src, int lane, uint32_t* sads) {
   if ((center.row & 3) || (center.col & 3)) return false;
   const int bx = mbx + center.col / 4 - wx0, by = mby + center.row / 4 - wy0;  // block origin in window
   if (bx < 3 || by < 3 || bx + 19 > WS || by + 19 > WS) return false;
-  // H: 22 rows (window rows by-3 .. by+18), 17 outputs at x = bx + i - 0.5.
-  for (int o = lane; o < 22 * 17; o += 32) {
-    const int r = o / 17, i = o - r * 17;
-    const uint8_t* p = S.win + (by - 3 + r) * WS + bx + i - 3;
-    S.hp[o] = (uint8_t)interp6_half(p[0], p[1], p[2], p[3], p[4], p[5]);
-  }
-  // V: 17 rows at y = by + r - 0.5, 16 columns.
-  for (int o = lane; o < 17 * 16; o += 32) {
-    const int r = o >> 4, c = o & 15;
-    const uint8_t* p = S.win + (by + r - 3) * WS + bx + c;
-    S.vp[o] = (uint8_t)interp6_half(p[0], p[WS], p[2 * WS], p[3 * WS], p[4 * WS], p[5 * WS]);
-  }
+  uint8_t* hp = S.temp;
+  half_plane_h(S.win, hp, bx, by, lane, 32);
+  half_plane_v(S.win, hp, bx, by, lane);
   __syncwarp();
-  // D: vertical half-pel over H (rows r..r+5 of H), 17 x 17.
-  for (int o = lane; o < 17 * 17; o += 32) {
-    const int r = o / 17, i = o - r * 17;
-    const uint8_t* p = S.hp + r * 17 + i;
-    S.dp[o] = (uint8_t)interp6_half(p[0], p[17], p[34], p[51], p[68], p[85]);
-  }
+  half_plane_d(hp, lane, 32);
   __syncwarp();
-  const int c = lane & 15, r0 = (lane >> 4) * 8;
-#pragma unroll 1
-  for (int k = 0; k < 8; k++) {
-    const int dy = (k < 3) ? -1 : (k < 5 ? 0 : 1);
-    const int dx = (k == 0 || k == 3 || k == 5) ? -1 : ((k == 1 || k == 6) ? 0 : 1);
-    const int cx = dx > 0, cy = dy > 0;
-    const uint8_t* pl;
-    int st;
-    if (dy == 0) {
-      pl = S.hp + 3 * 17 + cx;
-      st = 17;
-    } else if (dx == 0) {
-      pl = S.vp + cy * 16;
-      st = 16;
-    } else {
-      pl = S.dp + cy * 17 + cx;
-      st = 17;
-    }
-    uint32_t s = 0;
 #pragma unroll
-    for (int r = r0; r < r0 + 8; r++) {
-      const int d = (int)pl[r * st + c] - (int)src[r * 16 + c];
-      s += (uint32_t)(d < 0 ? -d : d);
-    }
-    sads[k] = __reduce_add_sync(FULL, s);
+  for (int k = 0; k < 4; k++) {
+    const uint32_t both = half_cand_sads(hp, src, k, lane);
+    sads[2 * k] = both & 0xffffu;
+    sads[2 * k + 1] = both >> 16;
   }
+  __syncwarp();
   return true;
+}
+
+// quarter_pixel_refine_luma (src/motion_search.rs:666-728) on one warp over the
+// shared planes where the window covers them, else candidate by candidate.
+// `center_sad` as in refine.
+__device__ __forceinline__ vp8a_search_result quarter_refine(const MePlane& P, WarpScratch& S, int wx0, int wy0,
+                                                             int mbx, int mby, vp8a_mv center, const uint8_t* src,
+                                                             int lane, uint32_t center_sad = ~0u) {
+  if (!quarter_inside(center, mbx, mby, wx0, wy0))
+    return refine(P, S, wx0, wy0, mbx, mby, center, 1, src, lane, center_sad);
+  vp8a_search_result best{center, center_sad};
+  if (center_sad == ~0u) best.sad = sad_at_mv(P, S, wx0, wy0, mbx, mby, center.row, center.col, src, lane);
+  int iy0, f;
+  quarter_pos(center.row - 1, mby, wy0, iy0, f);
+  iy0 -= 2;
+  auto taps = [](int fr) { return taps_const(fr); };
+  quarter_planes_h(S.win, S.temp, taps, center, mbx, wx0, iy0, lane, 32);
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const uint32_t both = quarter_cand_sads(S.temp, src, taps, center, mby, wy0, iy0, k, lane);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const uint32_t s = i ? both >> 16 : both & 0xffffu;
+      if (s < best.sad) {
+        best.sad = s;
+        best.mv.row = clamp_component(center.row + cand_dr(2 * k + i));
+        best.mv.col = clamp_component(center.col + cand_dc(2 * k + i));
+      }
+    }
+  }
+  __syncwarp();
+  return best;
 }
 
 // half_pixel_refine_luma (src/motion_search.rs:564-627) over the shared
