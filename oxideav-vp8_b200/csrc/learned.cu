@@ -6,21 +6,22 @@
 // cells seed an exact local search (the plain search's SAD kernels), so
 // the net only proposes; every returned vector and SAD is exact.
 //
-// Kernels (all hand-written; the GEMM-shaped ones on the tensor cores, the
-// training layers with mma.sync m16n8k16 BF16 -> FP32, inference and the
-// 32 -> 32 forward layers with tcgen05 and TMEM accumulators):
+// Kernels (all hand-written; the GEMM-shaped ones on the tensor cores:
+// inference and the 32 -> 32 layers and their input gradients with tcgen05 and
+// TMEM accumulators, the other training layers with mma.sync BF16 -> FP32):
 //   lp_windows_kernel       coarse cost volumes -> NHWC [n, 32, 32, 2] BF16
 //   lp_net_kernel           the whole net and the top-k cells per map in one
 //                           launch (inference), activations on chip
 //   lp_seeded_search_kernel every whole-pel vector near the seed cells,
 //                           first smallest SAD
-//   lp_conv_fwd_smem_kernel implicit-GEMM conv (+ bias, ReLU), one CTA per
-//                           image staged with its halo in shared memory
-//   lp_conv_bwd_data_kernel dX = conv^T(dY, W), masked by the ReLU of X
-//   lp_conv_fwd_tc_kernel   the 32 -> 32 forward layers on tcgen05 tensor
-//                           cores (TMEM accumulators)
-//   lp_conv_bwd_w_smem_kernel dW = sum over pixels of dY x shifted X (16
-//                           staged chunks per CTA, one atomic per weight), db
+//   lp_conv_tc_kernel       the 32 -> 32 layers, forward and dX, on tcgen05
+//   lp_conv_first_kernel, lp_conv_last_kernel   the 2 -> 32 and 32 -> 1 layers
+//   lp_conv_bwd_last_kernel dX of the 32 -> 1 layer
+//   lp_conv_bwd_w_kernel, lp_conv_bwd_w_edge_kernel   dW = sum over pixels of
+//                           dY x shifted X, and db
+//   lp_conv_fwd_smem_kernel, lp_conv_bwd_data_kernel, lp_conv_bwd_w_smem_kernel
+//                           the same for tensors off the 16-byte boundary and
+//                           for other output types, element by element
 //   lp_softmax_ce_kernel    softmax over the 1024 cells, cross-entropy,
 //                           d(logits) = (p - onehot) / n
 //   lp_adam_kernel          Adam on FP32 master weights, BF16 copies
@@ -46,7 +47,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __device__ __forceinline__ uint32_t pack_raw(uint16_t lo, uint16_t hi) { return (uint32_t)lo | ((uint32_t)hi << 16); }
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -443,41 +444,17 @@ __global__ void lp_lf_head_kernel(const float* sums, float count, int C, const f
   if (t == label && loss) *loss += -(zi - m - __logf(s));
 }
 
-// ------------------------------------------- tcgen05 forward, 32 -> 32
-// The 32 -> 32 layers on the 5th-generation tensor cores: one CTA per
-// image, the 3x3 convolution as an implicit GEMM D[pixel][n] = sum over
-// (tap, ci) of A[pixel + tap offset][ci] * W[n][tap][ci]. The image sits in
-// shared memory with a zero halo on a 34-pixel row pitch, channel-group
-// major (group g of 8 channels: 16 bytes per halo pixel). Four TMA tile
-// loads bring it in: the activations as a 4-D tensor (channel, x, y,
-// image), a box of 8 channels x 34 x 34 pixels x 1 image per channel
-// group, started at (8 g, -1, -1, image), so the box lands in exactly that
-// layout and the halo ring is the loads' out-of-bounds zero fill. So that 8
-// consecutive "virtual" output pixels v = y * 34 + x form one 8 x 16-byte
-// core matrix of the K-major, unswizzled canonical layout and a tap
-// (dy, dx) is only a base-address shift of (dy + 1) * 34 + dx + 1 pixels.
-// The virtual grid computes 2 discarded columns per row (x = 32, 33) and
-// is covered by 9 M = 128 tiles; each tile takes 18 MMAs of K = 16 (9 taps
-// x 2 channel halves) into a 32-column FP32 accumulator in tensor memory.
-// The weights sit as [k-group of 8][n][8] (k = tap * 32 + ci). One thread
-// issues the MMAs of up to four tiles, one commit signals an mbarrier, and
-// the 8 warps read the accumulators back (warp w: lanes 32 (w % 4) .. +31,
-// columns 16 (w / 4) .. +15 of each tile), add the bias, apply the ReLU and
-// store BF16.
+// ------------------------------- tcgen05 convolutions: layout and waits
 namespace lptc {
 constexpr int NV = 1224;                    // halo pixels per channel group (>= 1151 + 70 + 1)
 constexpr int REGION = NV * 16;             // bytes per channel group
 constexpr int IMG_BYTES = 4 * REGION;
 constexpr int W_BYTES = 36 * 32 * 16;       // 36 k-groups x 32 n x 16 bytes
-constexpr int SMEM = IMG_BYTES + W_BYTES + 32;
-constexpr uint32_t BOX_BYTES = 8 * 34 * 34 * 2;  // one channel group's TMA box
 static_assert(REGION % 128 == 0, "TMA destinations are 128-byte aligned");
 constexpr int TILES = 9;                    // ceil(32 * 34 / 128)
-constexpr uint32_t TMEM_COLS = 128;         // four 32-column accumulators
 // Instruction descriptor (kind::f16): D FP32, A and B BF16, both K-major,
 // N = 32, M = 128.
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((32u >> 3) << 17) | ((128u >> 4) << 24);
-constexpr int WAIT_LIMIT = 1 << 22;
 
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
   // Unswizzled K-major shared-memory matrix descriptor: start address,
@@ -501,142 +478,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, int limi
         : "memory");
   }
   return done != 0;
-}
-
-__global__ void __launch_bounds__(256, 2) lp_conv_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmx,
-                                                                 const uint16_t* W, const float* bias, int relu,
-                                                                 uint16_t* Y, uint32_t* status) {
-  using namespace lptc;
-  extern __shared__ __align__(128) uint8_t smt[];
-  uint8_t* img_s = smt;
-  uint8_t* w_s = smt + IMG_BYTES;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(smt + IMG_BYTES + W_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smt + IMG_BYTES + W_BYTES + 16);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const size_t im = blockIdx.x;
-  const uint32_t img_a = (uint32_t)__cvta_generic_to_shared(img_s);
-  const uint32_t w_a = (uint32_t)__cvta_generic_to_shared(w_s);
-  const uint32_t bar_a = (uint32_t)__cvta_generic_to_shared(mbar);
-  const uint32_t bar_t = bar_a + 8;  // the image loads' mbarrier
-
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     (uint32_t)__cvta_generic_to_shared(tmem_slot)),
-                 "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_a), "r"(1));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_t), "r"(1));
-    asm volatile("fence.mbarrier_init.release.cluster;");
-    // The image: four TMA tile loads (one per channel group, the halo ring
-    // from their out-of-bounds fill) completing on bar_t.
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_t), "r"(4 * BOX_BYTES)
-                 : "memory");
-    const uint64_t tm = reinterpret_cast<uint64_t>(&tmx);
-    for (int g = 0; g < 4; g++)
-      asm volatile(
-          "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-          "[%6];" ::"r"(img_a + (uint32_t)(g * REGION)),
-          "l"(tm), "r"(8 * g), "r"(-1), "r"(-1), "r"((int)im), "r"(bar_t)
-          : "memory");
-  }
-  // The weights by 16-byte asynchronous copies, and zeros into each
-  // channel group's tail past the 34 x 34 box, which no load touches.
-  for (int q = tid; q < 32 * 36; q += 256) {
-    const int n = q / 36, kg = q % 36;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(w_a + (uint32_t)((kg * 32 + n) * 16)),
-                 "l"(W + n * 288 + kg * 8)
-                 : "memory");
-  }
-  constexpr int TAIL = NV - 34 * 34;
-  for (int q = tid; q < 4 * TAIL; q += 256)
-    reinterpret_cast<uint4*>(img_s + (q / TAIL) * REGION)[34 * 34 + q % TAIL] = make_uint4(0, 0, 0, 0);
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();  // the mbarrier inits are visible from here on
-  // Bounded wait for the image; a load that never lands is reported, and
-  // the CTA waits once more (bounded) for it before leaving.
-  bool failed = __syncthreads_or(!mbar_wait(bar_t, 0, WAIT_LIMIT));
-  if (failed) {
-    if (tid == 0) atomicExch(status, 1u);  // DEV_TIMEOUT
-    mbar_wait(bar_t, 0, WAIT_LIMIT);
-  }
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
-
-  uint32_t phase = 0;
-  for (int t0 = 0; t0 < TILES && !failed; t0 += 4) {
-    const int nt = TILES - t0 < 4 ? TILES - t0 : 4;
-    if (tid == 0) {
-      for (int u = 0; u < nt; u++) {
-        const int v0 = (t0 + u) * 128;
-        const uint32_t d = tmem + (uint32_t)(u * 32);
-        for (int ks = 0; ks < 18; ks++) {
-          const int tap = ks >> 1, hh = ks & 1;
-          const int off = (tap / 3) * 34 + tap % 3;
-          const uint64_t ad = smem_desc(img_a + (uint32_t)(2 * hh * REGION + (v0 + off) * 16), REGION, 128);
-          const uint64_t bd = smem_desc(w_a + (uint32_t)((tap * 4 + 2 * hh) * 32 * 16), 512, 128);
-          const uint32_t acc = ks > 0 ? 1u : 0u;
-          asm volatile(
-              "{\n\t.reg .pred p;\n\t"
-              "setp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-              "l"(ad), "l"(bd), "r"(IDESC), "r"(acc));
-        }
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_a)
-                   : "memory");
-    }
-    // Bounded wait for the commit; a timeout is reported, not waited out.
-    const bool done = mbar_wait(bar_a, phase, WAIT_LIMIT);
-    phase ^= 1u;
-    failed = __syncthreads_or(!done);
-    if (failed) {
-      if (tid == 0) atomicExch(status, 1u);  // DEV_TIMEOUT
-      break;
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int lq = warp & 3, half = warp >> 2;
-    for (int u = 0; u < nt; u++) {
-      uint32_t r[16];
-      const uint32_t ta = tmem + ((uint32_t)(32 * lq) << 16) + (uint32_t)(u * 32 + half * 16);
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-          "%14, %15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(ta));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      const int v = (t0 + u) * 128 + 32 * lq + lane, y = v / 34, x = v % 34;
-      if (y < 32 && x < 32) {
-        uint32_t o[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const int n = half * 16 + 2 * j;
-          float a = __uint_as_float(r[2 * j]) + __ldg(bias + n);
-          float b = __uint_as_float(r[2 * j + 1]) + __ldg(bias + n + 1);
-          if (relu) {
-            a = fmaxf(a, 0.f);
-            b = fmaxf(b, 0.f);
-          }
-          o[j] = pack_bf16(a, b);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(Y + (im * LP_P + y * 32 + x) * 32 + half * 16);
-        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-      }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  }
-  __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
-  }
 }
 
 // ------------------------------------------ fused net inference (tcgen05)
@@ -1109,6 +950,871 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
   }
 }
 
+// ------------------------------------- training on persistent pipelines
+//
+// The training pass's convolutions for 16-byte aligned tensors (others take
+// lp_conv_fwd_smem_kernel, lp_conv_bwd_data_kernel and lp_conv_bwd_w_smem_kernel).
+// All of them are bound by the activations' way through memory (64 KB an
+// image and 32-channel tensor, read or written once a kernel) as long as
+// neither the loads nor the tensor cores wait: so each kernel is one CTA an SM
+// that walks its images with a producer warp issuing the TMA loads of the next
+// while the others compute. Every wait is bounded; one that runs out sets the
+// context's status word and the abort word, and the CTA leaves once its own
+// copies and MMAs are in (bounded again).
+//
+// Measured at 2048 images, us a launch, with the element-wise kernels and a
+// one-image-a-CTA tcgen05 forward, then with these: 2 -> 32 forward 87 -> 55, 32 ->
+// 32 forward 129 -> 73, dX 943 -> 86, dW 1397 -> 126, 32 -> 1 forward 115 -> 25, dX
+// 153 -> 48, dW 954 -> 28, dW of 2 -> 32 549 -> 48; the training step 6.85 -> 0.85 ms.
+namespace lptrain {
+using lpnet::arrive;
+using lpnet::mma;
+using lpnet::tmem_ld16;
+using lpnet::wait;
+using lptc::smem_desc;
+constexpr uint32_t FULL = 0xffffffffu;
+constexpr int LIMIT = lpnet::LIMIT;
+constexpr int HALF_BYTES = 16 * 32 * 64;  // 16 rows of 32 pixels, 32 channels
+
+__device__ __forceinline__ void bar_init(uint32_t bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+// K-major shared-memory matrix descriptor of 64-byte rows in the 64-byte swizzle:
+// 8-row atoms 512 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc64(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
+}
+__device__ __forceinline__ void expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma4(uint32_t dst, const CUtensorMap* tm, int c, int x, int y, int im, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+      "[%6];" ::"r"(dst),
+      "l"(tm), "r"(c), "r"(x), "r"(y), "r"(im), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma3(uint32_t dst, const CUtensorMap* tm, int x, int y, int im, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+      "[%5];" ::"r"(dst),
+      "l"(tm), "r"(x), "r"(y), "r"(im), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldsm2t(uint32_t addr, uint32_t (&r)[2]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ float bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+// Two channels of `v` where the same channels of x are above zero (the ReLU's
+// gradient; NaN is not above).
+__device__ __forceinline__ uint32_t relu_mask(uint32_t v, uint32_t x) {
+  return (bf_lo(x) > 0.f ? v & 0xffffu : 0u) | (bf_hi(x) > 0.f ? v & 0xffff0000u : 0u);
+}
+// Byte offset of channel group cg (8 channels, 16 bytes) of pixel p in a tile of
+// 64-byte pixels that TMA's 64-byte swizzle wrote (512-byte aligned): 8
+// consecutive pixels' groups lie on distinct banks.
+__device__ __forceinline__ uint32_t swz(int p, int cg) { return (uint32_t)(p * 64 + (((cg ^ (p >> 1)) & 3) << 4)); }
+
+}  // namespace lptrain
+
+// The 32 -> 32 convolution, forward or (BWD) the gradient of its input. An
+// implicit GEMM D[pixel][n] = sum over (tap, k) of A[pixel + tap][k] *
+// W'[n][tap][k] on the 5th-generation tensor cores: forward A = X, W' = W;
+// backward A = dY, W'[ci][tap][co] = W[co][8 - tap][ci], and the result is
+// masked by the ReLU of X. An image lies in shared memory with a zero halo on
+// a 34-pixel row pitch, 64 bytes a pixel in TMA's 64-byte swizzle, as one tile
+// load brings it in: the activations as a 4-D tensor (channel, x, y, image), a
+// box of 32 channels x 34 x 34 pixels from (0, -1, -1, image), the halo ring from
+// the out-of-bounds zero fill. 8 consecutive "virtual" output pixels v = y * 34 +
+// x are the 8 rows of a K-major swizzle atom (512 bytes, the pattern a function
+// of the address bits), so a tap (dy, dx) is only a base-address shift of (dy + 1)
+// * 34 + dx + 1 pixels. (Channel-group major tiles need no swizzle, but their four
+// boxes come as 4624 rows of 16 bytes an image: 99 us a
+// launch instead of 72.) The
+// virtual grid computes 2 discarded columns per row (x = 32, 33) and is covered
+// by 9 M = 128 tiles; each takes 18 MMAs of K = 16 (9 taps x 2 channel halves)
+// into a 32-column FP32 accumulator in tensor memory. The weights sit as
+// [k-group of 8][n][8] (k = tap * 32 + channel).
+//
+// Warps 0-7 read accumulators back (warp w: lanes 32 (w % 4) .. +31, columns
+// 16 (w / 4) .. +15 of a tile), 8-10 issue the MMAs of three tiles an image
+// each (one issuing thread sustains one MMA per ~63 cycles, several one per
+// ~40, the rate at which A streams from shared memory), 11 loads. Two image
+// buffers; five accumulator slots of three tiles, so the next image's MMAs run
+// while this one is read back.
+namespace lptc3 {
+constexpr int SLOTS = 5, GROUP = 3;                      // accumulator slots of GROUP tiles
+constexpr int OFF_W = 2 * lptc::IMG_BYTES;
+constexpr int OFF_BAR = OFF_W + lptc::W_BYTES;
+constexpr int BAR_FULL = 0, BAR_FREE = 2, BAR_ACC = 4, BAR_READ = BAR_ACC + SLOTS, BAR_FIN = BAR_READ + SLOTS;
+constexpr int NBAR = BAR_FIN + 3;
+constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
+constexpr int SMEM = OFF_TMEM + 8 + 1024;                // + the abort word, + alignment
+constexpr int EPI = 256, THREADS = EPI + 4 * 32;
+constexpr uint32_t TMEM_COLS = 512;
+static_assert(SLOTS * GROUP * 32 <= (int)TMEM_COLS && 3 * GROUP == lptc::TILES, "slots");
+}  // namespace lptc3
+
+template <bool BWD>
+__global__ void __launch_bounds__(lptc3::THREADS, 1)
+    lp_conv_tc_kernel(const __grid_constant__ CUtensorMap tmx, int n, const uint16_t* W, const float* bias, int relu,
+                      const uint16_t* Xa, uint16_t* Y, uint32_t* status) {
+  using namespace lptrain;
+  using namespace lptc3;
+  using lptc::IDESC;
+  using lptc::NV;
+  extern __shared__ uint8_t sm_raw[];
+  uint8_t* smt = sm_raw + ((1024u - ((uint32_t)__cvta_generic_to_shared(sm_raw) & 1023u)) & 1023u);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smt);
+  const uint32_t w_a = base + OFF_W;
+  auto bar = [&](int i) { return base + (uint32_t)(OFF_BAR + 8 * i); };
+  volatile uint32_t* abort_w = reinterpret_cast<volatile uint32_t*>(smt + OFF_TMEM + 4);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(base + OFF_TMEM),
+                 "r"(TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    for (int i = 0; i < NBAR; i++)
+      bar_init(bar(i), i == BAR_FREE || i == BAR_FREE + 1 ? 3 : (i >= BAR_READ && i < BAR_FIN ? 8 : 1));
+    *abort_w = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  uint16_t* w_s = reinterpret_cast<uint16_t*>(smt + OFF_W);
+  if (BWD) {
+    for (int q = tid; q < 9 * 32 * 32; q += THREADS) {
+      const int nn = q & 31, co = (q >> 5) & 31, tap = q >> 10;
+      w_s[((tap * 4 + (co >> 3)) * 32 + nn) * 8 + (co & 7)] = W[(co * 9 + 8 - tap) * 32 + nn];
+    }
+  } else {
+    for (int q = tid; q < 32 * 36; q += THREADS)
+      reinterpret_cast<uint4*>(w_s)[(q % 36) * 32 + q / 36] = reinterpret_cast<const uint4*>(W)[q];
+  }
+  // Zeros past the 34 x 34 box, which no load touches.
+  constexpr int TAIL = (NV - 34 * 34) * 4;
+  for (int q = tid; q < 2 * TAIL; q += THREADS)
+    reinterpret_cast<uint4*>(smt + (q / TAIL) * lptc::IMG_BYTES)[34 * 34 * 4 + q % TAIL] = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *reinterpret_cast<uint32_t*>(smt + OFF_TMEM);
+  const int first = blockIdx.x, stride = gridDim.x;
+  bool ok = true;
+
+  if (warp == 11) {
+    if (lane == 0) {
+      int j = 0;
+      for (int img = first; img < n; img += stride, j++) {
+        const int b = j & 1;
+        if (j >= 2) ok = wait(bar(BAR_FREE + b), (uint32_t)((j >> 1) - 1) & 1u, abort_w);
+        if (!ok) break;
+        expect(bar(BAR_FULL + b), 34 * 34 * 64);
+        tma4(base + (uint32_t)(b * lptc::IMG_BYTES), &tmx, 0, -1, -1, img, bar(BAR_FULL + b));
+      }
+      // The last loads are in before the CTA leaves.
+      for (int k = j > 2 ? j - 2 : 0; k < j; k++) mbar_wait(bar(BAR_FULL + (k & 1)), (uint32_t)(k >> 1) & 1u, LIMIT);
+    }
+  } else if (warp >= 8) {
+    if (lane == 0) {
+      const int s = warp - 8;
+      int j = 0;
+      for (int img = first; img < n; img += stride, j++) {
+        const int b = j & 1;
+        const uint32_t q = (uint32_t)(3 * j + s), slot = q % SLOTS, use = q / SLOTS;
+        ok = wait(bar(BAR_FULL + b), (uint32_t)(j >> 1) & 1u, abort_w) &&
+             (use == 0 || wait(bar(BAR_READ + (int)slot), (use - 1) & 1u, abort_w));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int u = 0; u < GROUP; u++) {
+          const uint32_t a0 = base + (uint32_t)(b * lptc::IMG_BYTES + (s * GROUP + u) * 128 * 64);
+          const uint32_t d = tmem + slot * (GROUP * 32) + (uint32_t)(u * 32);
+          for (int ks = 0; ks < 18; ks++) {
+            const int tap = BWD ? 8 - (ks >> 1) : ks >> 1, hh = ks & 1;
+            const int off = (tap / 3) * 34 + tap % 3;
+            mma(d, smem_desc64(a0 + (uint32_t)(off * 64 + hh * 32)),
+                smem_desc(w_a + (uint32_t)((tap * 4 + 2 * hh) * 512), 512, 128), IDESC, ks > 0 ? 1u : 0u);
+          }
+        }
+        commit(bar(BAR_ACC + (int)slot));
+        commit(bar(BAR_FREE + b));
+      }
+      commit(bar(BAR_FIN + s));
+      mbar_wait(bar(BAR_FIN + s), 0, LIMIT);
+    }
+  } else {
+    const int lq = warp & 3, half = warp >> 2;
+    float bv[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) bv[i] = BWD ? 0.f : bias[half * 16 + i];
+    // Where this lane's pixels of group s of an image lie.
+    auto place = [&](int img, int s, int u, bool& in) {
+      const int v = (s * GROUP + u) * 128 + 32 * lq + lane, y = v / 34, x = v - y * 34;
+      in = y < 32 && x < 32;
+      return ((size_t)img * LP_P + y * 32 + x) * 32 + half * 16;
+    };
+    // The ReLU's inputs, a group ahead.
+    uint4 ahead[GROUP][2] = {};
+    auto fetch = [&](int img, int s) {
+#pragma unroll
+      for (int u = 0; u < GROUP; u++) {
+        bool in;
+        const size_t at = place(img, s, u, in);
+        if (in) {
+          ahead[u][0] = reinterpret_cast<const uint4*>(Xa + at)[0];
+          ahead[u][1] = reinterpret_cast<const uint4*>(Xa + at)[1];
+        }
+      }
+    };
+    if (BWD && Xa) fetch(first, 0);
+    uint32_t q = 0;
+    for (int img = first; img < n && ok; img += stride) {
+      for (int s = 0; s < 3 && ok; s++, q++) {
+        const uint32_t slot = q % SLOTS;
+        size_t at[GROUP];
+        bool in[GROUP];
+        uint4 xm[GROUP][2];
+#pragma unroll
+        for (int u = 0; u < GROUP; u++) {
+          at[u] = place(img, s, u, in[u]);
+          xm[u][0] = ahead[u][0];
+          xm[u][1] = ahead[u][1];
+        }
+        if (BWD && Xa && (s < 2 || img + stride < n)) fetch(s < 2 ? img : img + stride, s < 2 ? s + 1 : 0);
+        ok = __all_sync(FULL, wait(bar(BAR_ACC + (int)slot), (q / SLOTS) & 1u, abort_w));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t r[GROUP][16];
+#pragma unroll
+        for (int u = 0; u < GROUP; u++)
+          tmem_ld16(tmem + ((uint32_t)(32 * lq) << 16) + slot * (GROUP * 32) + (uint32_t)(u * 32 + half * 16), r[u]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive(bar(BAR_READ + (int)slot));
+#pragma unroll
+        for (int u = 0; u < GROUP; u++) {
+          if (!in[u]) continue;
+          uint32_t o[8];
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            float a = __uint_as_float(r[u][2 * i]), b = __uint_as_float(r[u][2 * i + 1]);
+            if (!BWD) {
+              a += bv[2 * i];
+              b += bv[2 * i + 1];
+              if (relu) {
+                a = fmaxf(a, 0.f);
+                b = fmaxf(b, 0.f);
+              }
+            }
+            o[i] = pack_bf16(a, b);
+          }
+          if (BWD && Xa) {
+            o[0] = relu_mask(o[0], xm[u][0].x);
+            o[1] = relu_mask(o[1], xm[u][0].y);
+            o[2] = relu_mask(o[2], xm[u][0].z);
+            o[3] = relu_mask(o[3], xm[u][0].w);
+            o[4] = relu_mask(o[4], xm[u][1].x);
+            o[5] = relu_mask(o[5], xm[u][1].y);
+            o[6] = relu_mask(o[6], xm[u][1].z);
+            o[7] = relu_mask(o[7], xm[u][1].w);
+          }
+          uint4* dst = reinterpret_cast<uint4*>(Y + at[u]);
+          dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+          dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        }
+      }
+    }
+  }
+  if (!ok) {
+    atomicExch(status, 1u);  // DEV_TIMEOUT
+    *abort_w = 1;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  }
+}
+
+// dW and db of the 32 -> 32 convolution: dW[co][tap][ci] = sum over pixels p of
+// dY[p][co] X[p + off(tap)][ci]. M = co, N = (tap, ci), K = pixels, by
+// mma.sync with both operands read through ldmatrix.trans from the tiles that
+// TMA left in shared memory (half an image a stage: 16 rows of dY, 18 rows of X
+// with a zero halo); the contraction is over pixels, so each tap is the same
+// tile at another pixel offset. A CTA takes groups of LP_WCPB half images and
+// adds a group's sums with one atomic per weight: the FP32 chains (512 MMA steps)
+// are lp_conv_bwd_w_smem_kernel's, pixel by pixel, so the partial sums are the
+// same bits (four shorter chains a warp each measured 20 % less time and gradients
+// 2e-5 apart). That fixes K, so the twelve warps split N: warp w holds 8 input
+// channels (w / 3) and (ROWS = 3) kernel row w % 3, or (ROWS = 1: few groups, one
+// kernel row a CTA) kernel column w % 3.
+constexpr int LP_WCPB = 16;  // half images whose gradients one FP32 chain adds up
+namespace lpdw {
+constexpr int X_BYTES = 18 * 34 * 64, X_SPACE = (X_BYTES + 511) / 512 * 512;
+constexpr int STAGE = X_SPACE + lptrain::HALF_BYTES;
+constexpr int STAGES = 3, WARPS = 12, THREADS = (WARPS + 1) * 32;
+constexpr int OFF_BAR = STAGES * STAGE;
+constexpr int SMEM = OFF_BAR + 2 * STAGES * 8 + 8 + 512;  // + the abort word, + alignment
+}  // namespace lpdw
+
+template <int ROWS>
+__global__ void __launch_bounds__(lpdw::THREADS, 1)
+    lp_conv_bwd_w_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmd, int n,
+                         float* dW, float* db, uint32_t* status) {
+  using namespace lptrain;
+  using namespace lpdw;
+  constexpr int KX = ROWS == 3 ? 3 : 1;  // kernel columns of a warp
+  extern __shared__ uint8_t sm_raw[];
+  uint8_t* sm = sm_raw + ((512u - ((uint32_t)__cvta_generic_to_shared(sm_raw) & 511u)) & 511u);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+  auto full = [&](int i) { return base + (uint32_t)(OFF_BAR + 8 * i); };
+  auto empty = [&](int i) { return base + (uint32_t)(OFF_BAR + 8 * (STAGES + i)); };
+  volatile uint32_t* abort_w = reinterpret_cast<volatile uint32_t*>(sm + OFF_BAR + 16 * STAGES);
+  if (tid == 0) {
+    for (int i = 0; i < STAGES; i++) {
+      bar_init(full(i), 1);
+      bar_init(empty(i), WARPS);
+    }
+    *abort_w = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  __syncthreads();
+  const int items = 2 * n, first = blockIdx.x * LP_WCPB, stride = gridDim.x * LP_WCPB;
+  bool ok = true;
+  int j = 0;  // half images so far
+  if (warp == WARPS) {
+    if (lane == 0) {
+      for (int i0 = first; i0 < items && ok; i0 += stride)
+        for (int it = i0; it < items && it < i0 + LP_WCPB; it++, j++) {
+          const int s = j % STAGES;
+          if (j >= STAGES) ok = wait(empty(s), (uint32_t)(j / STAGES - 1) & 1u, abort_w);
+          if (!ok) break;
+          expect(full(s), X_BYTES + HALF_BYTES);
+          tma4(base + (uint32_t)(s * STAGE), &tmx, 0, -1, (it & 1) * 16 - 1, it >> 1, full(s));
+          tma4(base + (uint32_t)(s * STAGE + X_SPACE), &tmd, 0, 0, (it & 1) * 16, it >> 1, full(s));
+        }
+      // The last loads are in before the CTA leaves.
+      for (int k = j > STAGES ? j - STAGES : 0; k < j; k++)
+        mbar_wait(full(k % STAGES), (uint32_t)(k / STAGES) & 1u, LIMIT);
+    }
+  } else {
+    const int ky = ROWS == 3 ? warp % 3 : (int)blockIdx.y, kx0 = ROWS == 3 ? 0 : warp % 3, cg = warp / 3;
+    // This lane's row of the 8 x 8 matrices a load takes: of dY (pixels 0-7 and
+    // 8-15, channel groups 0 and 1; 2 and 3 for co 16-31), of X (pixels 0-15 of
+    // group cg, at two kernel columns).
+    const int pa = (lane & 7) + ((lane >> 4) & 1) * 8, ca = (lane >> 3) & 1;
+    const int pb = (lane & 15) + kx0 + (ROWS == 3 ? lane >> 4 : 0) + ky * 34;
+    float bs[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    for (int i0 = first; i0 < items && ok; i0 += stride) {
+      float acc[KX][2][4] = {};
+      for (int it = i0; it < items && it < i0 + LP_WCPB; it++, j++) {
+        const int s = j % STAGES;
+        ok = __all_sync(FULL, wait(full(s), (uint32_t)(j / STAGES) & 1u, abort_w));
+        if (!ok) break;
+        const uint32_t xs = base + (uint32_t)(s * STAGE), ds = xs + X_SPACE;
+        // Step k = 8 o + i takes pixels 16 k .. + 15: row 4 o + i / 2, columns 16 (i
+        // % 2) on. The swizzle depends on that row's place in four (a 34-pixel
+        // pitch): four base addresses, the rest is immediate. The next step's
+        // fragments load while this one's MMAs run.
+        uint32_t xb[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          xb[r] = xs + (uint32_t)(pb * 64 + (((cg ^ (r + (pb >> 1))) & 3) << 4));
+        uint32_t aa = ds + swz(pa, ca), ab = aa ^ 32u;
+        uint32_t a[2][2][4], b[2][3][2];
+        auto load = [&](int i) {
+          const int u = i & 1, r = i >> 1, q = (r * 34 + (i & 1) * 16) * 64;
+          ldsm4t(aa + i * 1024, a[u][0]);
+          ldsm4t(ab + i * 1024, a[u][1]);
+          if (ROWS == 3) {
+            uint32_t f[4];
+            ldsm4t(xb[r & 3] + q, f);
+            ldsm2t(xb[(r + 1) & 3] + q + 128, b[u][2]);
+            b[u][0][0] = f[0];
+            b[u][0][1] = f[1];
+            b[u][1][0] = f[2];
+            b[u][1][1] = f[3];
+          } else {
+            ldsm2t(xb[r & 3] + q, b[u][0]);
+          }
+        };
+        load(0);
+#pragma unroll 1
+        for (int o = 0; o < 4; o++) {
+          const bool sums = cg == o;  // db: each warp takes a twelfth of the pixels
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const int u = i & 1;
+            if (i < 7) {
+              load(i + 1);
+            } else if (o < 3) {
+              // Four rows on.
+              aa += 8 * 1024;
+              ab += 8 * 1024;
+#pragma unroll
+              for (int r = 0; r < 4; r++) xb[r] += 4 * 34 * 64;
+              load(0);
+            }
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+              for (int x = 0; x < KX; x++) mma_bf16(acc[x][m], a[u][m], b[u][x]);
+            if (sums && i % 3 == warp % 3) {
+#pragma unroll
+              for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+                  bs[m][e] +=
+                      (bf_lo(a[u][m][e]) + bf_hi(a[u][m][e])) + (bf_lo(a[u][m][e + 2]) + bf_hi(a[u][m][e + 2]));
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) arrive(empty(s));
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int x = 0; x < KX; x++)
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+          for (int f = 0; f < 4; f++)
+            atomicAdd(dW + (m * 16 + g + 8 * (f >> 1)) * 288 + (ky * 3 + kx0 + x) * 32 + cg * 8 + 2 * t + (f & 1),
+                      acc[x][m][f]);
+    }
+    if (ok && (ROWS == 3 || blockIdx.y == 0)) {
+#pragma unroll
+      for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          float v = bs[m][e];
+          v += __shfl_xor_sync(FULL, v, 1);
+          v += __shfl_xor_sync(FULL, v, 2);
+          if (t == 0) atomicAdd(db + m * 16 + 8 * e + g, v);
+        }
+    }
+  }
+  if (!ok) {
+    atomicExch(status, 1u);  // DEV_TIMEOUT
+    *abort_w = 1;
+  }
+  __syncwarp();
+  __syncthreads();
+}
+
+// dW and db where one side has C channels, 1 or 2, and the other 32. C = 2 (the
+// first layer, 2 -> 32): dW[co][tap][c] = sum of dY[p][co] X[p + off][c]. C = 1
+// (the last, 32 -> 1): dW[tap][ci] = sum of X[q][ci] dY[q - off]. Either way M =
+// the 32 channels, read through ldmatrix.trans from half an image a stage, N =
+// (tap, c) gathered from the small tensor's 18 rows (8 elements of zero halo
+// beside each, so that the TMA box starts on 16 bytes), K = pixels; a warp holds
+// one 16 x 8 tile of dW, its FP32 chain as long as the element-wise kernel's. Bound
+// by reading the 32-channel tensor once.
+namespace lpdws {
+constexpr int STAGE = lptrain::HALF_BYTES + 4096, STAGES = 3;  // two CTAs an SM
+constexpr int OFF_BAR = STAGES * STAGE;
+constexpr int SMEM = OFF_BAR + 2 * STAGES * 8 + 8 + 512;
+template <int C>
+constexpr int WARPS_OF = 2 * ((9 * C + 7) / 8);  // 16 x 8 tiles of dW
+}  // namespace lpdws
+
+template <int C>
+__global__ void __launch_bounds__(32 * lpdws::WARPS_OF<C> + 32, 2)
+    lp_conv_bwd_w_edge_kernel(const __grid_constant__ CUtensorMap tm32, const __grid_constant__ CUtensorMap tms, int n,
+                              float* dW, float* db, uint32_t* status) {
+  using namespace lptrain;
+  using namespace lpdws;
+  constexpr int RP = 32 * C + 16, SMALL = 18 * RP * 2, N = 9 * C, WARPS = WARPS_OF<C>, S = C == 2 ? 1 : -1;
+  static_assert(SMALL <= 4096, "the small tensor's rows fit");
+  extern __shared__ uint8_t sm_raw[];
+  uint8_t* sm = sm_raw + ((512u - ((uint32_t)__cvta_generic_to_shared(sm_raw) & 511u)) & 511u);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+  auto full = [&](int i) { return base + (uint32_t)(OFF_BAR + 8 * i); };
+  auto empty = [&](int i) { return base + (uint32_t)(OFF_BAR + 8 * (STAGES + i)); };
+  volatile uint32_t* abort_w = reinterpret_cast<volatile uint32_t*>(sm + OFF_BAR + 16 * STAGES);
+  if (tid == 0) {
+    for (int i = 0; i < STAGES; i++) {
+      bar_init(full(i), 1);
+      bar_init(empty(i), WARPS);
+    }
+    *abort_w = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  __syncthreads();
+  const int items = 2 * n, first = blockIdx.x * LP_WCPB, stride = gridDim.x * LP_WCPB;
+  bool ok = true;
+  int j = 0;
+  if (warp == WARPS) {
+    if (lane == 0) {
+      for (int i0 = first; i0 < items && ok; i0 += stride)
+        for (int it = i0; it < items && it < i0 + LP_WCPB; it++, j++) {
+          const int s = j % STAGES;
+          if (j >= STAGES) ok = wait(empty(s), (uint32_t)(j / STAGES - 1) & 1u, abort_w);
+          if (!ok) break;
+          expect(full(s), HALF_BYTES + SMALL);
+          tma4(base + (uint32_t)(s * STAGE), &tm32, 0, 0, (it & 1) * 16, it >> 1, full(s));
+          tma3(base + (uint32_t)(s * STAGE + HALF_BYTES), &tms, -8, (it & 1) * 16 - 1, it >> 1, full(s));
+        }
+      for (int k = j > STAGES ? j - STAGES : 0; k < j; k++)
+        mbar_wait(full(k % STAGES), (uint32_t)(k / STAGES) & 1u, LIMIT);
+    }
+  } else {
+    const int m = warp & 1, i = warp >> 1;  // 16 channels, 8 columns
+    const int pa = (lane & 7) + ((lane >> 4) & 1) * 8, ca = ((lane >> 3) & 1) + 2 * m;
+    // This lane's column's element at pixel 2 t of a row's first 16.
+    const int nn = i * 8 + g < N ? i * 8 + g : 0, tap = nn / C;
+    const int nb = (1 + S * (tap / 3 - 1)) * RP + 8 + (2 * t + S * (tap % 3 - 1)) * C + nn % C;
+    float bs[2] = {0.f, 0.f};
+    for (int i0 = first; i0 < items && ok; i0 += stride) {
+      float acc[4] = {};
+      for (int it = i0; it < items && it < i0 + LP_WCPB; it++, j++) {
+        const int s = j % STAGES;
+        ok = __all_sync(FULL, wait(full(s), (uint32_t)(j / STAGES) & 1u, abort_w));
+        if (!ok) break;
+        const uint32_t as = base + (uint32_t)(s * STAGE);
+        const uint16_t* small = reinterpret_cast<const uint16_t*>(sm + s * STAGE + HALF_BYTES);
+        // Four steps' fragments load while the four before run.
+        uint32_t a[2][4][4], b[2][4][2];
+        auto load = [&](int v) {
+#pragma unroll
+          for (int w = 0; w < 4; w++) {
+            const int k = v * 4 + w;
+            ldsm4t(as + swz(pa, ca) + (uint32_t)k * 1024u, a[v & 1][w]);
+            const uint16_t* e = small + (k >> 1) * RP + (k & 1) * 16 * C + nb;
+            b[v & 1][w][0] = pack_raw(e[0], e[C]);
+            b[v & 1][w][1] = pack_raw(e[8 * C], e[9 * C]);
+          }
+        };
+        load(0);
+#pragma unroll 2
+        for (int v = 0; v < 8; v++) {
+          const int u = v & 1;
+          if (v < 7) load(v + 1);
+#pragma unroll
+          for (int w = 0; w < 4; w++) {
+            mma_bf16(acc, a[u][w], b[u][w]);
+            const int k = v * 4 + w;
+            if (C == 2) {
+              if (i == w % 3)
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                  bs[h] += (bf_lo(a[u][w][h]) + bf_hi(a[u][w][h])) + (bf_lo(a[u][w][h + 2]) + bf_hi(a[u][w][h + 2]));
+            } else if (lane < 16 && warp == w) {
+              bs[0] += __uint_as_float((uint32_t)small[((k >> 1) + 1) * RP + 8 + (k & 1) * 16 + lane] << 16);
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) arrive(empty(s));
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int f = 0; f < 4; f++) {
+        const int ch = m * 16 + g + 8 * (f >> 1), c = i * 8 + 2 * t + (f & 1);
+        if (c < N) atomicAdd(dW + (C == 2 ? ch * N + c : c * 32 + ch), acc[f]);
+      }
+    }
+    if (ok) {
+#pragma unroll
+      for (int h = 0; h < (C == 2 ? 2 : 1); h++) {
+        float v = bs[h];
+#pragma unroll
+        for (int o = 1; o < (C == 2 ? 4 : 32); o <<= 1) v += __shfl_xor_sync(FULL, v, o);
+        if (C == 2 ? t == 0 : lane == 0) atomicAdd(db + (C == 2 ? m * 16 + 8 * h + g : 0), v);
+      }
+    }
+  }
+  if (!ok) {
+    atomicExch(status, 1u);  // DEV_TIMEOUT
+    *abort_w = 1;
+  }
+  __syncwarp();
+  __syncthreads();
+}
+
+// The first layer, 2 -> 32: a tile of 16 pixels takes one K = 8 step a tap (its
+// first pair of columns is the pixel's channel pair, the others zero): the sums
+// grow tap by tap as in lp_conv_fwd_smem_kernel, so the BF16 results are the same
+// ones; eight taps in one K = 16 step would round differently and costs only the
+// tensor time that the stores hide. The weights stay in registers, their columns
+// ordered so that a lane ends up with 8 consecutive channels of a pixel: column c
+// of block j is channel 8 (c / 2) + 2 j + c % 2. One CTA an image; bound by
+// writing the 64 KB of its output.
+__device__ __forceinline__ void mma_bf16_k8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+  asm(
+      "mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(b));
+}
+__global__ void __launch_bounds__(256) lp_conv_first_kernel(const uint16_t* X, const uint16_t* W, const float* bias,
+                                                            int relu, uint16_t* Y) {
+  constexpr int RP = 40;  // words a row: 3 unused, the halo, 32 pixels, the halo
+  __shared__ uint32_t xs[34 * RP];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const size_t img = blockIdx.x;
+  const uint32_t* Xi = reinterpret_cast<const uint32_t*>(X) + img * LP_P;
+  uint32_t v[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) v[i] = Xi[tid + 256 * i];
+  if (tid < 2 * 34) xs[(tid / 34) * 33 * RP + 3 + tid % 34] = 0;
+  else if (tid < 2 * 34 + 64) xs[(1 + ((tid - 68) >> 1)) * RP + 3 + ((tid - 68) & 1) * 33] = 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int p = tid + 256 * i;
+    xs[((p >> 5) + 1) * RP + 4 + (p & 31)] = v[i];
+  }
+  uint32_t b[4][9];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const uint16_t* w = W + (8 * (g >> 1) + 2 * j + (g & 1)) * 18;
+#pragma unroll
+    for (int tap = 0; tap < 9; tap++) b[j][tap] = t == 0 ? pack_raw(w[2 * tap], w[2 * tap + 1]) : 0u;
+  }
+  float bv[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) bv[i] = bias[8 * t + i];
+  __syncthreads();
+#pragma unroll 2
+  for (int u = 0; u < 8; u++) {
+    const int tile = warp * 8 + u, y = tile >> 1, xb = (tile & 1) * 16;
+    const uint32_t* r = xs + y * RP + xb + g + 3;
+    float d[4][4] = {};
+#pragma unroll
+    for (int tap = 0; tap < 9; tap++) {
+      const uint32_t* q = r + (tap / 3) * RP + tap % 3;
+      const uint32_t a0 = t == 0 ? q[0] : 0u, a1 = t == 0 ? q[8] : 0u;
+#pragma unroll
+      for (int j = 0; j < 4; j++) mma_bf16_k8(d[j], a0, a1, b[j][tap]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        float p = d[j][2 * h] + bv[2 * j], q = d[j][2 * h + 1] + bv[2 * j + 1];
+        if (relu) {
+          p = fmaxf(p, 0.f);
+          q = fmaxf(q, 0.f);
+        }
+        o[j] = pack_bf16(p, q);
+      }
+      *reinterpret_cast<uint4*>(Y + (img * LP_P + y * 32 + xb + g + 8 * h) * 32 + 8 * t) =
+          make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+}
+
+// The gradient of the last layer's input, 1 -> 32: K = the 9 taps of dY around a
+// pixel (one K = 16 step a tile), masked by the ReLU of X; weights in registers
+// in lp_conv_first_kernel's column order. Bound by reading X and writing dX.
+__global__ void __launch_bounds__(256) lp_conv_bwd_last_kernel(const uint16_t* dY, const uint16_t* W,
+                                                               const uint16_t* Xa, uint16_t* dX) {
+  using lptrain::relu_mask;
+  constexpr int RP = 40;
+  __shared__ uint16_t ys[34 * RP];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const size_t img = blockIdx.x;
+  uint32_t v[2];
+#pragma unroll
+  for (int i = 0; i < 2; i++) v[i] = reinterpret_cast<const uint32_t*>(dY + img * LP_P)[tid + 256 * i];
+  if (tid < 2 * 34) ys[(tid / 34) * 33 * RP + 3 + tid % 34] = 0;
+  else if (tid < 2 * 34 + 64) ys[(1 + ((tid - 68) >> 1)) * RP + 3 + ((tid - 68) & 1) * 33] = 0;
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int p = 2 * (tid + 256 * i);
+    *reinterpret_cast<uint32_t*>(&ys[((p >> 5) + 1) * RP + 4 + (p & 31)]) = v[i];
+  }
+  uint32_t b[4][2];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const uint16_t* w = W + 8 * (g >> 1) + 2 * j + (g & 1);
+    b[j][0] = pack_raw(w[2 * t * 32], w[(2 * t + 1) * 32]);
+    b[j][1] = t == 0 ? (uint32_t)w[8 * 32] : 0u;
+  }
+  // dY at p - off(tap).
+  auto off = [&](int tap) { return (2 - tap / 3) * RP + 2 - tap % 3 + 3; };
+  const int o0 = off(2 * t), o1 = off(2 * t + 1), o2 = off(8);
+  __syncthreads();
+#pragma unroll 4
+  for (int u = 0; u < 8; u++) {
+    const int tile = warp * 8 + u, y = tile >> 1, xb = (tile & 1) * 16;
+    const size_t at = (img * LP_P + y * 32 + xb + g) * 32 + 8 * t;
+    uint4 xm[2];
+    if (Xa) {
+      xm[0] = *reinterpret_cast<const uint4*>(Xa + at);
+      xm[1] = *reinterpret_cast<const uint4*>(Xa + at + 8 * 32);
+    }
+    const uint16_t* r = ys + y * RP + xb + g;
+    const uint32_t a[4] = {pack_raw(r[o0], r[o1]), pack_raw(r[8 + o0], r[8 + o1]), t == 0 ? (uint32_t)r[o2] : 0u,
+                           t == 0 ? (uint32_t)r[8 + o2] : 0u};
+    float d[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.f;
+      mma_bf16(d[j], a, b[j]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) o[j] = pack_bf16(d[j][2 * h], d[j][2 * h + 1]);
+      if (Xa) {
+        o[0] = relu_mask(o[0], xm[h].x);
+        o[1] = relu_mask(o[1], xm[h].y);
+        o[2] = relu_mask(o[2], xm[h].z);
+        o[3] = relu_mask(o[3], xm[h].w);
+      }
+      *reinterpret_cast<uint4*>(dX + at + (size_t)h * 8 * 32) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+}
+
+// The last layer, 32 -> 1: z[p][tap] = X[p] . W[tap], a contraction of K = 32
+// with the taps as N (4 MMAs a tile of 16 pixels, the weights in registers), then
+// y[p] = sum over taps of z[p + off(tap)][tap] + bias from shared memory. Half an
+// image a stage by TMA; bound by reading X.
+namespace lplast {
+constexpr int STAGES = 4, WARPS = 8, THREADS = (WARPS + 1) * 32, ZP = 34;  // z row pitch with its halo
+constexpr int OFF_Z = STAGES * lptrain::HALF_BYTES;
+constexpr int OFF_BAR = OFF_Z + 9 * 34 * ZP * 4;
+constexpr int SMEM = OFF_BAR + 2 * STAGES * 8 + 8 + 512;
+static_assert(OFF_BAR % 8 == 0, "barrier alignment");
+}  // namespace lplast
+
+__global__ void __launch_bounds__(lplast::THREADS, 1)
+    lp_conv_last_kernel(const __grid_constant__ CUtensorMap tmx, int n, const uint16_t* W, const float* bias, int relu,
+                        float* Y, uint32_t* status) {
+  using namespace lptrain;
+  using namespace lplast;
+  extern __shared__ uint8_t sm_raw[];
+  uint8_t* sm = sm_raw + ((512u - ((uint32_t)__cvta_generic_to_shared(sm_raw) & 511u)) & 511u);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+  float* z = reinterpret_cast<float*>(sm + OFF_Z);  // [9][34][34]
+  auto full = [&](int i) { return base + (uint32_t)(OFF_BAR + 8 * i); };
+  auto empty = [&](int i) { return base + (uint32_t)(OFF_BAR + 8 * (STAGES + i)); };
+  volatile uint32_t* abort_w = reinterpret_cast<volatile uint32_t*>(sm + OFF_BAR + 16 * STAGES);
+  if (tid == 0) {
+    for (int i = 0; i < STAGES; i++) {
+      bar_init(full(i), 1);
+      bar_init(empty(i), WARPS);
+    }
+    *abort_w = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  for (int q = tid; q < 9 * 34 * ZP; q += THREADS) z[q] = 0.f;
+  __syncthreads();
+  const int first = blockIdx.x, stride = gridDim.x;
+  bool ok = true;
+  if (warp == WARPS) {
+    if (lane == 0) {
+      int j = 0;
+      for (int img = first; img < n && ok; img += stride)
+        for (int h = 0; h < 2; h++, j++) {
+          const int s = j % STAGES;
+          if (j >= STAGES) ok = wait(empty(s), (uint32_t)(j / STAGES - 1) & 1u, abort_w);
+          if (!ok) break;
+          expect(full(s), HALF_BYTES);
+          tma4(base + (uint32_t)(s * HALF_BYTES), &tmx, 0, 0, h * 16, img, full(s));
+        }
+      for (int k = j > STAGES ? j - STAGES : 0; k < j; k++)
+        mbar_wait(full(k % STAGES), (uint32_t)(k / STAGES) & 1u, LIMIT);
+    }
+  } else {
+    const int pa = (lane & 7) + ((lane >> 3) & 1) * 8, ca = (lane >> 4) & 1;
+    uint32_t b[2][2][2];  // [16 channels][8 taps][fragment]
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int tap = i * 8 + g;
+        const uint16_t* w = W + (tap < 9 ? tap : 0) * 32 + k * 16 + 2 * t;
+        b[k][i][0] = tap < 9 ? pack_raw(w[0], w[1]) : 0u;
+        b[k][i][1] = tap < 9 ? pack_raw(w[8], w[9]) : 0u;
+      }
+    const float bv = bias[0];
+    int j = 0;
+    for (int img = first; img < n && ok; img += stride) {
+      for (int h = 0; h < 2; h++, j++) {
+        const int s = j % STAGES;
+        ok = __all_sync(FULL, wait(full(s), (uint32_t)(j / STAGES) & 1u, abort_w));
+        if (!ok) break;
+        const uint32_t xs = base + (uint32_t)(s * HALF_BYTES);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int y = 2 * warp + (u >> 1), xb = (u & 1) * 16;
+          uint32_t a[2][4];
+          const uint32_t aa = xs + swz(y * 32 + xb + pa, ca);
+          ldsm4(aa, a[0]);
+          ldsm4(aa ^ 32u, a[1]);
+          float d[2][4] = {};
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            mma_bf16(d[i], a[0], b[0][i]);
+            mma_bf16(d[i], a[1], b[1][i]);
+          }
+          float* zr = z + (h * 16 + y + 1) * ZP + xb + 1 + g;
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            zr[(2 * t + e) * 34 * ZP] = d[0][e];
+            zr[(2 * t + e) * 34 * ZP + 8] = d[0][2 + e];
+          }
+          if (t == 0) {
+            zr[8 * 34 * ZP] = d[1][0];
+            zr[8 * 34 * ZP + 8] = d[1][2];
+          }
+        }
+        __syncwarp();
+        if (lane == 0) arrive(empty(s));
+      }
+      ok = !lpnet::epi_or(!ok);  // the eight warps leave together
+      if (!ok) break;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int p = tid + 256 * i;
+        const float* zr = z + (p >> 5) * ZP + (p & 31);
+        float v = 0.f;
+#pragma unroll
+        for (int tap = 0; tap < 9; tap++) v += zr[(tap * 34 + tap / 3) * ZP + tap % 3];
+        v += bv;
+        Y[(size_t)img * LP_P + p] = relu ? fmaxf(v, 0.f) : v;
+      }
+      lpnet::epi_sync();
+    }
+  }
+  if (!ok) {
+    atomicExch(status, 1u);  // DEV_TIMEOUT
+    *abort_w = 1;
+  }
+  __syncwarp();
+  __syncthreads();
+}
+
 // cuTensorMapEncodeTiled, taken from the driver once.
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1128,25 +1834,114 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// The TMA map of n NHWC [32][32][32] BF16 images for the tcgen05 conv: a
-// 4-D tensor (channel, x, y, image) with boxes of 8 channels x 34 x 34 x 1.
-vp8a_status conv_image_map(const uint16_t* x, uint32_t n, CUtensorMap* tm) {
+vp8a_status encode_map(const uint16_t* x, int rank, const cuuint64_t* dim, const cuuint64_t* stride,
+                       const cuuint32_t* box, CUtensorMapSwizzle swizzle, CUtensorMap* tm) {
   const EncodeTiledFn enc = encode_tiled();
   if (!enc) {
     vp8a::set_error("the driver does not provide cuTensorMapEncodeTiled");
     return VP8A_E_CUDA;
   }
-  const cuuint64_t gdim[4] = {32, 32, 32, (cuuint64_t)n};
-  const cuuint64_t gstride[3] = {32 * 2, 32 * 32 * 2, 32 * 32 * 32 * 2};  // bytes, dims 1..3
-  const cuuint32_t box[4] = {8, 34, 34, 1}, estride[4] = {1, 1, 1, 1};
-  const CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<uint16_t*>(x), gdim, gstride, box, estride,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  const cuuint32_t estride[4] = {1, 1, 1, 1};
+  const CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<uint16_t*>(x), dim, stride, box,
+                         estride, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     vp8a::set_error("cuTensorMapEncodeTiled rejected the activation map (error " + std::to_string((int)r) + ")");
     return VP8A_E_CUDA;
   }
   return VP8A_OK;
+}
+
+// The TMA map of n NHWC [32][32][32] BF16 images: a 4-D tensor (channel, x, y,
+// image) with boxes of `ch` channels (8 unswizzled, 32 with the 64-byte
+// swizzle) x w x h x 1.
+vp8a_status image_map(const uint16_t* x, uint32_t n, uint32_t ch, uint32_t w, uint32_t h, CUtensorMap* tm) {
+  const cuuint64_t dim[4] = {32, 32, 32, n};
+  const cuuint64_t stride[3] = {32 * 2, 32 * 32 * 2, 32 * 32 * 32 * 2};  // bytes, dims 1..3
+  const cuuint32_t box[4] = {ch, w, h, 1};
+  return encode_map(x, 4, dim, stride, box, ch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE, tm);
+}
+
+// The TMA map of n NHWC [32][32][C] images as (x * C + c, y, image): boxes of 18
+// rows with 8 elements beside each.
+vp8a_status row_map(const uint16_t* x, uint32_t n, uint32_t c, CUtensorMap* tm) {
+  const cuuint64_t dim[3] = {32 * c, 32, n};
+  const cuuint64_t stride[2] = {64 * c, 2048 * c};
+  const cuuint32_t box[3] = {32 * c + 16, 18, 1};
+  return encode_map(x, 3, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE, tm);
+}
+
+template <typename K>
+vp8a_status use_smem(K* kernel, int bytes) {
+  VP8A_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  return VP8A_OK;
+}
+
+// The persistent kernels' launches (16-byte aligned tensors, n > 0).
+template <bool BWD>
+vp8a_status conv_tc(vp8a_ctx* ctx, const uint16_t* a, const uint16_t* W, const float* bias, int n, int relu,
+                    const uint16_t* Xa, uint16_t* Y) {
+  CUtensorMap tm;
+  vp8a_status s = image_map(a, (uint32_t)n, 32, 34, 34, &tm);
+  if (s == VP8A_OK) s = use_smem(lp_conv_tc_kernel<BWD>, lptc3::SMEM);
+  if (s != VP8A_OK) return s;
+  lp_conv_tc_kernel<BWD><<<std::min(n, ctx->sm_count), lptc3::THREADS, lptc3::SMEM, ctx->stream>>>(
+      tm, n, W, bias, relu, Xa, Y, ctx->d_status);
+  VP8A_CUDA(cudaGetLastError());
+  ctx->launches++;
+  return VP8A_OK;
+}
+
+vp8a_status conv_last(vp8a_ctx* ctx, const uint16_t* X, const uint16_t* W, const float* bias, int n, int relu,
+                      float* Y) {
+  CUtensorMap tm;
+  vp8a_status s = image_map(X, (uint32_t)n, 32, 32, 16, &tm);
+  if (s == VP8A_OK) s = use_smem(lp_conv_last_kernel, lplast::SMEM);
+  if (s != VP8A_OK) return s;
+  lp_conv_last_kernel<<<std::min(n, ctx->sm_count), lplast::THREADS, lplast::SMEM, ctx->stream>>>(
+      tm, n, W, bias, relu, Y, ctx->d_status);
+  VP8A_CUDA(cudaGetLastError());
+  ctx->launches++;
+  return VP8A_OK;
+}
+
+// All kernel rows in one CTA a group, each byte staged once (512 images 60 us,
+// 2048 122 us; a row a CTA 87 and 254), or a row a CTA while three a group find an
+// SM each (256 images 46 us; one a group 60).
+vp8a_status conv_bwd_w_32(vp8a_ctx* ctx, const uint16_t* dY, const uint16_t* X, int n, float* dW, float* db) {
+  CUtensorMap tmx, tmd;
+  const int groups = (2 * n + LP_WCPB - 1) / LP_WCPB;
+  const bool split = 3 * groups <= ctx->sm_count;
+  const auto kernel = split ? lp_conv_bwd_w_kernel<1> : lp_conv_bwd_w_kernel<3>;
+  vp8a_status s = image_map(X, (uint32_t)n, 32, 34, 18, &tmx);
+  if (s == VP8A_OK) s = image_map(dY, (uint32_t)n, 32, 32, 16, &tmd);
+  if (s == VP8A_OK) s = use_smem(kernel, lpdw::SMEM);
+  if (s != VP8A_OK) return s;
+  kernel<<<dim3(std::min(groups, ctx->sm_count), split ? 3 : 1), lpdw::THREADS, lpdw::SMEM, ctx->stream>>>(
+      tmx, tmd, n, dW, db, ctx->d_status);
+  VP8A_CUDA(cudaGetLastError());
+  ctx->launches++;
+  return VP8A_OK;
+}
+
+template <int C>
+vp8a_status conv_bwd_w_edge(vp8a_ctx* ctx, const uint16_t* t32, const uint16_t* small, int n, float* dW, float* db) {
+  CUtensorMap tm, tms;
+  const int groups = (2 * n + LP_WCPB - 1) / LP_WCPB;
+  vp8a_status s = image_map(t32, (uint32_t)n, 32, 32, 16, &tm);
+  if (s == VP8A_OK) s = row_map(small, (uint32_t)n, C, &tms);
+  if (s == VP8A_OK) s = use_smem(lp_conv_bwd_w_edge_kernel<C>, lpdws::SMEM);
+  if (s != VP8A_OK) return s;
+  lp_conv_bwd_w_edge_kernel<C>
+      <<<std::min(groups, 2 * ctx->sm_count), 32 * lpdws::WARPS_OF<C> + 32, lpdws::SMEM, ctx->stream>>>(tm, tms, n, dW, db,
+                                                                                                ctx->d_status);
+  VP8A_CUDA(cudaGetLastError());
+  ctx->launches++;
+  return VP8A_OK;
+}
+
+bool aligned16(const void* a, const void* b = nullptr, const void* c = nullptr) {
+  return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) == 0;
 }
 
 template <int CIN, int NT>
@@ -1179,7 +1974,6 @@ vp8a_status conv_bwd_data(vp8a_ctx* ctx, const uint16_t* dY, const uint16_t* W, 
 // in shared memory; warp w accumulates the n-tiles w, w + 4, ... of
 // dW = dY^T x im2col(X) in registers across all its chunks, and the CTA
 // adds its partial sums with one atomic per weight at the end.
-constexpr int LP_WCPB = 16;
 template <int CIN, int MT>
 __global__ void __launch_bounds__(128) lp_conv_bwd_w_smem_kernel(const uint16_t* dY, const uint16_t* X, int cout,
                                                                  long n_chunks, float* dW, float* db) {
@@ -1363,6 +2157,12 @@ vp8a_status vp8a_lp_conv_forward(vp8a_ctx* ctx, const uint16_t* x, uint32_t cin,
     return VP8A_E_INVALID_ARGUMENT;
   }
   VP8A_CUDA(cudaSetDevice(ctx->device));
+  if (cin == 2 && cout == 32 && y && !y_f32 && n > 0 && aligned16(y)) {
+    lp_conv_first_kernel<<<n, 256, 0, ctx->stream>>>(x, w, bias, (int)relu, y);
+    VP8A_CUDA(cudaGetLastError());
+    ctx->launches++;
+    return VP8A_OK;
+  }
   if (cin == 2 && cout == 32) return conv_fwd<2, 4>(ctx, x, w, bias, 32, (int)n, relu, y, y_f32);
   if (cin == 32 && cout == 32 && y && !y_f32 && n > 0) {
     // The tensor-core path: 16-byte aligned activations and weights.
@@ -1370,16 +2170,11 @@ vp8a_status vp8a_lp_conv_forward(vp8a_ctx* ctx, const uint16_t* x, uint32_t cin,
       vp8a::set_error("tensor-core conv needs 16-byte aligned buffers");
       return VP8A_E_INVALID_ARGUMENT;
     }
-    CUtensorMap tm;
-    const vp8a_status s = conv_image_map(x, n, &tm);
-    if (s != VP8A_OK) return s;
-    VP8A_CUDA(cudaFuncSetAttribute(lp_conv_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lptc::SMEM));
-    lp_conv_fwd_tc_kernel<<<n, 256, lptc::SMEM, ctx->stream>>>(tm, w, bias, (int)relu, y, ctx->d_status);
-    VP8A_CUDA(cudaGetLastError());
-    ctx->launches++;
-    return VP8A_OK;
+    return conv_tc<false>(ctx, x, w, bias, (int)n, (int)relu, nullptr, y);
   }
   if (cin == 32 && cout == 32) return conv_fwd<32, 4>(ctx, x, w, bias, 32, (int)n, relu, y, y_f32);
+  if (cin == 32 && cout == 1 && y_f32 && n > 0 && aligned16(x) && encode_tiled())
+    return conv_last(ctx, x, w, bias, (int)n, (int)relu, y_f32);
   if (cin == 32 && cout == 1) return conv_fwd<32, 1>(ctx, x, w, bias, 1, (int)n, relu, y, y_f32);
   vp8a::set_error("conv shape must be 2->32, 32->32 or 32->1");
   return VP8A_E_INVALID_ARGUMENT;
@@ -1395,18 +2190,31 @@ vp8a_status vp8a_lp_conv_backward(vp8a_ctx* ctx, const uint16_t* x, uint32_t cin
   VP8A_CUDA(cudaSetDevice(ctx->device));
   vp8a_status s;
   const uint16_t* mask = x_relu ? x : nullptr;
+  // The persistent kernels read whole 16-byte groups; any other alignment takes
+  // the element-wise ones.
+  const bool wide = n > 0 && aligned16(x, dy, dx) && encode_tiled();
   if (cin == 2 && cout == 32) {
-    if ((s = conv_bwd_w<2>(ctx, dy, x, 32, (int)n, dw, db)) != VP8A_OK) return s;
+    s = wide ? conv_bwd_w_edge<2>(ctx, dy, x, (int)n, dw, db) : conv_bwd_w<2>(ctx, dy, x, 32, (int)n, dw, db);
+    if (s != VP8A_OK) return s;
     if (dx) return conv_bwd_data<32, 1>(ctx, dy, w, 2, (int)n, mask, dx);
     return VP8A_OK;
   }
   if (cin == 32 && cout == 32) {
-    if ((s = conv_bwd_w<32>(ctx, dy, x, 32, (int)n, dw, db)) != VP8A_OK) return s;
+    s = wide ? conv_bwd_w_32(ctx, dy, x, (int)n, dw, db) : conv_bwd_w<32>(ctx, dy, x, 32, (int)n, dw, db);
+    if (s != VP8A_OK) return s;
+    if (dx && wide) return conv_tc<true>(ctx, dy, w, nullptr, (int)n, 0, mask, dx);
     if (dx) return conv_bwd_data<32, 4>(ctx, dy, w, 32, (int)n, mask, dx);
     return VP8A_OK;
   }
   if (cin == 32 && cout == 1) {
-    if ((s = conv_bwd_w<32>(ctx, dy, x, 1, (int)n, dw, db)) != VP8A_OK) return s;
+    s = wide ? conv_bwd_w_edge<1>(ctx, x, dy, (int)n, dw, db) : conv_bwd_w<32>(ctx, dy, x, 1, (int)n, dw, db);
+    if (s != VP8A_OK) return s;
+    if (dx && wide) {
+      lp_conv_bwd_last_kernel<<<n, 256, 0, ctx->stream>>>(dy, w, mask, dx);
+      VP8A_CUDA(cudaGetLastError());
+      ctx->launches++;
+      return VP8A_OK;
+    }
     if (dx) return conv_bwd_data<1, 4>(ctx, dy, w, 32, (int)n, mask, dx);
     return VP8A_OK;
   }
