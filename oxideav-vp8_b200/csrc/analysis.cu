@@ -91,7 +91,6 @@ struct AnArgs {
 // edge-clamped, so later reads need no bounds checks.
 constexpr int HS = 24;        // halo stride
 constexpr int MAX_BLOCKS = 9; // zero + 4 left + 4 above offsets
-constexpr int CMAX = 25;      // SPLITMV candidate vectors per partition
 
 struct __align__(16) RefSmem {
   WarpScratch ws;                       // window + six-tap scratch + half planes
@@ -135,9 +134,9 @@ struct SplitOut {
 // anchors 0/4/8/12, 5..8 = ABOVE vectors of the top-row anchors 0..3,
 // 9..24 = the NEW4X4 result of group 0..15.
 struct __align__(16) SplitScratch {
-  double table[CMAX * 16];   // group g's SAD at column m: table[m * 16 + g], needed columns only
+  uint16_t far[16][16];      // the groups' SADs at a NEW result beyond the field
   uint64_t zero_new[16 * 5]; // the cheaper of ZERO and NEW for group g in context x: J's bits
-  double terms[32];          // the total's terms in order
+  double terms[32];          // the total's terms in order, then zeros
   vp8a_mv cmv[16];           // the groups' NEW results (columns 9 + g)
 };
 static_assert(sizeof(SplitScratch) % 16 == 0, "SplitScratch copies stay 16-byte aligned");
@@ -532,6 +531,14 @@ __device__ __forceinline__ uint32_t group_sad(const FieldView& v, const MePlane&
   return direct_group_sad(P, src, x, y, pid, g);
 }
 
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// Group g's SAD in the row of SADs at a shared address.
+__device__ __forceinline__ uint32_t row_sad(uint32_t row, int g) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(row + 2 * g));
+  return v;
+}
+
 // An integer below 2^32 as a double: the bits of 2^52 + v, less 2^52 (exact; the
 // conversion unit is slower than an addition).
 __device__ __forceinline__ double small_double(uint32_t v) {
@@ -558,10 +565,12 @@ __device__ __forceinline__ double mv_partition_bits(const double* t, int pid) {
 }
 
 // score_split_partition (src/encoder.rs:8080-8246) on one warp: lane g
-// walks group g's NEW4X4 diamond over the field, the lanes then fill a
-// table of group SADs at every vector the sub-MV choice can consider (ZERO,
-// the external neighbours' vectors, every group's NEW result), and the
-// sequential LEFT/ABOVE/ZERO/NEW choice over groups reads that table.
+// walks group g's NEW4X4 diamond over the field, and the LEFT/ABOVE/ZERO/NEW
+// choice over groups reads the groups' SADs at each vector it can consider
+// (ZERO, the external neighbours' vectors, every group's NEW result) from the
+// row of the field or of the staged blocks that holds them. (A table of them as
+// doubles, filled before the choice, cost 1200 cycles of the 16-group
+// partition's 7500 and saved one conversion a step.)
 //
 // The per-group costs that do not depend on the chain are computed before
 // it: sbits[ctx * 4 + mode] = submv_ref_bits of each context and mode, and
@@ -655,23 +664,38 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
       if (!improved) break;
     }
     W.cmv[g] = best;
-    const int dr = (int)best.row - bp.row, dc = (int)best.col - bp.col;
-    const bool ok = dr >= -1023 && dr <= 1023 && dc >= -1023 && dc <= 1023;
-    const double nb = ok ? mvb[dr + 1023] + mvb[MV_BITS_SPAN + dc + 1023] : 0.0;
     my_new_sad = bs;
-    my_new_bits = nb;
+  }
+  __syncwarp();
+  {
     // The cheaper of ZERO and NEW in each context (ZERO first among equals):
-    // neither depends on the chain below.
-    const int zb = fv.pl->colblk[0];
-    const double tz = (double)(pid == 3 ? fv.xs->blk[zb][g] : fv.xs->grp[zb][goff + g]), tn = (double)bs;
+    // neither depends on the chain below. Lane g takes group g's contexts 0-2,
+    // lane 16 + g contexts 3 and 4.
+    const int g = lane & 15;
+    const uint32_t bs = __shfl_sync(FULL, my_new_sad, g);
+    W.terms[lane] = 0.0;
+    if (g < G) {
+      const vp8a_mv best = W.cmv[g];
+      const int dr = (int)best.row - bp.row, dc = (int)best.col - bp.col;
+      const bool ok = dr >= -1023 && dr <= 1023 && dc >= -1023 && dc <= 1023;
+      const double nb = ok ? mvb[dr + 1023] + mvb[MV_BITS_SPAN + dc + 1023] : 0.0;
+      my_new_bits = nb;
+      const int zb = fv.pl->colblk[0];
+      const double tz = small_double(pid == 3 ? fv.xs->blk[zb][g] : fv.xs->grp[zb][goff + g]), tn = small_double(bs);
+      const int x0 = lane < 16 ? 0 : 3;
 #pragma unroll
-    for (int x = 0; x < 5; x++) {
-      const uint64_t jz = (uint64_t)__double_as_longlong(tz + lterm[x * 4 + VP8A_SUBMV_ZERO]);
-      const uint64_t jn =
-          ok ? (uint64_t)__double_as_longlong(tn + a.lambda * (sbits[x * 4 + VP8A_SUBMV_NEW] + nb)) : ~0ull;
-      if (jn < jz) new_wins |= 1u << x;
-      W.zero_new[g * 5 + x] = jn < jz ? jn : jz;
+      for (int i = 0; i < 3; i++) {
+        const int x = x0 + i;
+        if (x < 5) {
+          const uint64_t jz = (uint64_t)__double_as_longlong(tz + lterm[x * 4 + VP8A_SUBMV_ZERO]);
+          const uint64_t jn =
+              ok ? (uint64_t)__double_as_longlong(tn + a.lambda * (sbits[x * 4 + VP8A_SUBMV_NEW] + nb)) : ~0ull;
+          if (jn < jz) new_wins |= 1u << x;
+          W.zero_new[g * 5 + x] = jn < jz ? jn : jz;
+        }
+      }
     }
+    new_wins |= __shfl_down_sync(FULL, new_wins, 16);
   }
   __syncwarp();
   // Lane m < 9 + G holds column m's vector, packed (equal vectors, equal
@@ -680,30 +704,23 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
   const int ncol = 9 + G;
   const vp8a_mv mvm = lane < 9 ? fv.pl->colmv[lane] : (lane < ncol ? W.cmv[lane - 9] : vp8a_mv{0, 0});
   const uint32_t cvec = (uint32_t)(uint16_t)mvm.row | ((uint32_t)(uint16_t)mvm.col << 16);
-  // The candidate table: lane m fills column m for every group. Columns
-  // 0-8 (ZERO and the neighbours' vectors) are staged blocks; columns 9+
-  // (the groups' NEW results) lie in the field, or, beyond it, are summed
-  // from the plane. Only the columns the partition's choice can reach.
-  const uint32_t need = c_need_cols[pid];
-  if (lane < ncol && ((need >> lane) & 1u)) {
+  // Lane m's row of SADs: column m's for every group (shared address). Columns
+  // 0-8 (ZERO and the neighbours' vectors) are staged blocks; columns 9+ (the
+  // groups' NEW results) lie in the field, or, beyond it, are summed from the
+  // plane. Only the columns the partition's choice can reach.
+  uint32_t my_row = 0;
+  if (lane < ncol && ((c_need_cols[pid] >> lane) & 1u)) {
     const int x = fv.mbx + int_off(mvm.col), y = fv.mby + int_off(mvm.row);
     const int cp = lane < 9 ? fv.pl->colblk[lane] : fpos(x - fv.cxp, y - fv.cyp);
-    double* col = W.table + lane * 16;
+    const uint16_t* row = W.far[lane < 9 ? 0 : lane - 9];
     if (lane < 9 || cp >= 0) {
-      // The 16 block SADs of a staged block or a field position are one
-      // 32-byte row, the group sums one of 16 bytes.
-      const uint16_t* row = pid == 3 ? (lane < 9 ? fv.xs->blk[cp] : fv.F->blk[cp])
-                                     : (lane < 9 ? fv.xs->grp[cp] : fv.F->grp[cp]) + goff;
-#pragma unroll
-      for (int g = 0; g < 16; g += 2)
-        if (g < G) {
-          const uint32_t w = *(const uint32_t*)(row + g);
-          *(double2*)(col + g) = make_double2(small_double(w & 0xffffu), small_double(w >> 16));
-        }
+      row = pid == 3 ? (lane < 9 ? fv.xs->blk[cp] : fv.F->blk[cp])
+                     : (lane < 9 ? fv.xs->grp[cp] : fv.F->grp[cp]) + goff;
     } else {
 #pragma unroll 1
-      for (int g = 0; g < G; g++) col[g] = (double)direct_group_sad(P, src, x, y, pid, g);
+      for (int g = 0; g < G; g++) W.far[lane - 9][g] = (uint16_t)direct_group_sad(P, src, x, y, pid, g);
     }
+    my_row = smem_at(row);
   }
   __syncwarp();
   // The sub-MV choice. Lane g decides group g. A group's LEFT/ABOVE come
@@ -724,17 +741,21 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
   const int ext_l = 1 + (anchor >> 2), ext_a = 5 + anchor;
   const uint32_t ext_lv = __shfl_sync(FULL, cvec, ext_l & 31), ext_av = __shfl_sync(FULL, cvec, ext_a & 31);
   const uint32_t new_vec = __shfl_sync(FULL, cvec, (9 + lane) & 31);
-  // The group's choice: its column and that column's vector.
-  int chosen = 0, mode = VP8A_SUBMV_ZERO, my_ctx = 0;
+  const uint32_t ext_lr = __shfl_sync(FULL, my_row, ext_l & 31), ext_ar = __shfl_sync(FULL, my_row, ext_a & 31);
+  const uint32_t new_row = __shfl_sync(FULL, my_row, (9 + lane) & 31), zero_row = __shfl_sync(FULL, my_row, 0);
+  // The group's choice: its column's row and vector, and the group's SAD there.
+  uint32_t chosen = zero_row, my_sad = 0;
+  int mode = VP8A_SUBMV_ZERO, my_ctx = 0;
   uint32_t chosen_vec = 0;
   bool my_bad = false;
   const int lsrc = gc == 0 ? lane : lane - 1, asrc = gr == 0 ? lane : lane - gw;
 #pragma unroll 1
   for (int st = 0; st < gh + gw - 1; st++) {
-    const int lch = __shfl_sync(FULL, chosen, lsrc), ach = __shfl_sync(FULL, chosen, asrc);
+    const uint32_t lch = __shfl_sync(FULL, chosen, lsrc), ach = __shfl_sync(FULL, chosen, asrc);
     const uint32_t lchv = __shfl_sync(FULL, chosen_vec, lsrc), achv = __shfl_sync(FULL, chosen_vec, asrc);
     if (lane < G && gr + gc == st) {
-      const int lidx = gc == 0 ? ext_l : lch, aidx = gr == 0 ? ext_a : ach;
+      const uint32_t lrow = gc == 0 ? ext_lr : lch, arow = gr == 0 ? ext_ar : ach;
+      const uint32_t ls = row_sad(lrow, lane), as = row_sad(arow, lane);
       const uint32_t lv = gc == 0 ? ext_lv : lchv, av = gr == 0 ? ext_av : achv;
       const bool lez = lv == 0u, aez = av == 0u, lea = lv == av;
       const int ctxi = lea ? (lez ? 4 : 3) : (aez ? 2 : (lez ? 1 : 0));
@@ -746,15 +767,16 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
       // the first minimum of the first minima of (LEFT, ABOVE) and (ZERO,
       // NEW).
       const double2 lt = *(const double2*)(lterm + ctxi * 4);
-      const uint64_t j0 = (uint64_t)__double_as_longlong(W.table[lidx * 16 + lane] + lt.x);
-      const uint64_t j1 = (uint64_t)__double_as_longlong(W.table[aidx * 16 + lane] + lt.y);
+      const uint64_t j0 = (uint64_t)__double_as_longlong(small_double(ls) + lt.x);
+      const uint64_t j1 = (uint64_t)__double_as_longlong(small_double(as) + lt.y);
       const uint64_t v2n = W.zero_new[lane * 5 + ctxi];
       const bool above_first = j1 < j0, is_new = (new_wins >> ctxi) & 1u;
       const uint64_t v01 = above_first ? j1 : j0;
       const bool second = v2n < v01;
       mode = second ? (is_new ? VP8A_SUBMV_NEW : VP8A_SUBMV_ZERO)
                     : (above_first ? VP8A_SUBMV_ABOVE : VP8A_SUBMV_LEFT);
-      chosen = second ? (is_new ? 9 + lane : 0) : (above_first ? aidx : lidx);
+      chosen = second ? (is_new ? new_row : zero_row) : (above_first ? arow : lrow);
+      my_sad = second ? (is_new ? my_new_sad : row_sad(zero_row, lane)) : (above_first ? as : ls);
       chosen_vec = second ? (is_new ? new_vec : 0u) : (above_first ? av : lv);
       my_ctx = ctxi;
       my_bad = (second ? v2n : v01) >= 0x7ff0000000000000ull;
@@ -765,7 +787,6 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
   // the groups' terms go through shared memory, closed up, and lane 0 sums
   // them in order.
   const bool mine = lane < G, isn = mine && mode == VP8A_SUBMV_NEW;
-  const uint32_t my_sad = !mine ? 0u : (isn ? my_new_sad : (uint32_t)W.table[chosen * 16 + lane]);
   const uint32_t total_sad = __reduce_add_sync(FULL, my_sad);
   const unsigned any_bad = __ballot_sync(FULL, mine && my_bad), news = __ballot_sync(FULL, isn);
   if (mine) {
@@ -779,9 +800,19 @@ __device__ void split_partition(const AnArgs& a, const double* pbits, const doub
     // The reference stops at the first group without a finite choice.
     out->valid = any_bad == 0u;
     double total_bits = 0.0;
+    // Adding the zeros past the last term changes nothing.
     const int n = G + __popc(news);
-#pragma unroll 2
-    for (int i = 0; i < n; i++) total_bits += W.terms[i];
+#pragma unroll 1
+    for (int i = 0; i < n; i += 8) {
+      double2 t[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) t[k] = *(const double2*)(W.terms + i + 2 * k);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        total_bits += t[k].x;
+        total_bits += t[k].y;
+      }
+    }
     out->j = (double)total_sad + a.lambda * (pbits[pid] + total_bits);
   }
   // Block b's vector: the column its group chose.
@@ -955,7 +986,6 @@ struct Feed {
 };
 static_assert(offsetof(Feed, src) % 16 == 0 && offsetof(Feed, above) % 16 == 0, "Feed alignment");
 
-__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool bar_done(uint64_t* bar, unsigned parity) {
   uint32_t done;
   asm volatile(
