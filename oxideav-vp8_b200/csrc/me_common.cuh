@@ -175,6 +175,21 @@ __device__ __forceinline__ uint32_t sad_whole_at(const MePlane& P, const uint8_t
   return sad_global16(P, x0, y0, src, lane);
 }
 
+// Whole-pel SADs of two blocks of the window, at its pixels (xa, ya) and (xb, yb):
+// block a's in the low half of the result. A half-warp takes a block, a lane a row
+// (the window's 40-byte rows fall on distinct banks).
+__device__ __forceinline__ uint32_t sad_win16_pair(const uint8_t* win, int xa, int ya, int xb, int yb,
+                                                   const uint8_t* src, int lane) {
+  const int x = lane < 16 ? xa : xb, row = lane & 15;
+  const uint32_t* w = (const uint32_t*)(win + ((lane < 16 ? ya : yb) + row) * WS + (x & ~3));
+  const uint4 sv = *(const uint4*)(src + row * 16);
+  const unsigned sh = (unsigned)(x & 3) * 8u;
+  const uint32_t w1 = w[1], w2 = w[2], w3 = w[3];
+  const uint32_t s = __vsadu4(__funnelshift_r(w[0], w1, sh), sv.x) + __vsadu4(__funnelshift_r(w1, w2, sh), sv.y) +
+                     __vsadu4(__funnelshift_r(w2, w3, sh), sv.z) + __vsadu4(__funnelshift_r(w3, w[4], sh), sv.w);
+  return __reduce_add_sync(FULL, lane < 16 ? s : s << 16);
+}
+
 // §18.3 two-pass six-tap prediction SAD (sixtap_mb_luma,
 // src/motion_comp.rs:902-1057) from a 21x21 halo at `h` (stride hs, a multiple
 // of 4; block origin at (2, 2); reads up to 27 bytes of a row from h on). The
@@ -487,12 +502,12 @@ __device__ __forceinline__ void quarter_planes_h(const uint8_t* win, uint8_t* qh
   }
 }
 
-// Vertical passes and SADs of candidates 2 slot and 2 slot + 1 (one warp): lane
-// (candidate, strip of four rows, word).
+// Vertical passes and SADs of two candidates (one warp), the first in the low half
+// of the result: lane (candidate, strip of four rows, word), k the lane's candidate.
 template <class TapsOf>
-__device__ __forceinline__ uint32_t quarter_cand_sads(const uint8_t* qh, const uint8_t* src, TapsOf&& taps_of,
-                                                      vp8a_mv qc, int mby, int wy0, int iy0, int slot, int lane) {
-  const int k = 2 * slot + (lane >> 4), strip = (lane >> 2) & 3, j = lane & 3;
+__device__ __forceinline__ uint32_t quarter_pair_sads(const uint8_t* qh, const uint8_t* src, TapsOf&& taps_of,
+                                                      vp8a_mv qc, int mby, int wy0, int iy0, int k, int lane) {
+  const int strip = (lane >> 2) & 3, j = lane & 3;
   int iy, fy;
   quarter_pos(qc.row + cand_dr(k), mby, wy0, iy, fy);
   const Taps f = taps_of(fy);
@@ -518,6 +533,13 @@ __device__ __forceinline__ uint32_t quarter_cand_sads(const uint8_t* qh, const u
     }
   }
   return pair_sum(s, lane);
+}
+
+// Candidates 2 slot and 2 slot + 1.
+template <class TapsOf>
+__device__ __forceinline__ uint32_t quarter_cand_sads(const uint8_t* qh, const uint8_t* src, TapsOf&& taps_of,
+                                                      vp8a_mv qc, int mby, int wy0, int iy0, int slot, int lane) {
+  return quarter_pair_sads(qh, src, taps_of, qc, mby, wy0, iy0, 2 * slot + (lane >> 4), lane);
 }
 
 // half_pixel_refine_luma's candidates (src/motion_search.rs:589-598; also of

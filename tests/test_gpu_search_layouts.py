@@ -70,3 +70,25 @@ def test_searches_any_layout(ctx, oracle, w, h, offset, pad):
                 getattr(oracle, name)(ref, mbs, xy, arg)), (name, trial)
         assert sr_tuples(vp8a.small_diamond_search_luma(ctx, plane, mbs, xy, mv, 8)) == sr_tuples(
             oracle.small_diamond_search_luma(ref, mbs, xy, mv, 8)), trial
+
+
+@pytest.mark.parametrize("effort", [0, 2, 3])
+@pytest.mark.parametrize("w,h,offset,pad", [(16, 16, 0, 0), (97, 80, 0, 0), (97, 80, 3, 1), (160, 48, 4, 4)])
+def test_rd_search_long_descents_any_layout(ctx, oracle, effort, w, h, offset, pad):
+    # Neighbours far from the true vector (up to 40 px) and descents of up to 32
+    # rounds: more than the staged window covers, also across the plane's edges.
+    uw, uh = (w + 1) // 2, (h + 1) // 2
+    grey = np.full((uh, uw), 128, np.uint8)
+    frame = [ramp(w, h, 0, 0, 1), grey, grey]
+    refs = [vp8a.pad_to_mb(ramp(w, h, dx, dy, 2 + i), grey, grey) for i, (dx, dy) in enumerate([(13.5, -9.25), (0, 17)])]
+    lam = vp8a.rd_lambda(12)
+    nb = oracle.neighbours_from_decisions(oracle.analyse_inter_frame(frame, refs, [1, 2], lam))
+    rng = np.random.default_rng(w + effort)
+    for mv in (nb["mv"], nb["split_mvs"]) if "split_mvs" in nb.dtype.names else (nb["mv"],):
+        for f in ("row", "col"):
+            mv[f] = rng.integers(-160, 161, mv[f].shape)
+    want = oracle.rd_inter_search(frame, refs, [1, 2], lam, 8, effort, nb)
+    got = vp8a.rd_inter_search(ctx, [placed(p, offset, pad) for p in frame],
+                               [[placed(p, offset, pad) for p in r] for r in refs], [1, 2], lam, 8, effort, nb)
+    for f in ("ref_frame", "mode", "n_searched", "leader", "mv", "sad", "cost", "bits", "found"):
+        assert np.array_equal(got[f], want[f]), f
