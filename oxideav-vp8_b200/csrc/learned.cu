@@ -484,16 +484,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, int limi
 // The whole proposal net, one image at a time per persistent CTA (one per
 // SM, the weights staged once), warp-specialised: the MMA warps (8 on)
 // issue the tcgen05.mma of the tiles in turn (lane 0 of each) into a ring
-// of 16 TMEM accumulators of 32 columns; warps 0-7 read each one back as soon
-// as its MMAs commit, add the bias, apply the ReLU, store BF16 into the
-// next layer's activation buffer and mark the (layer, tile) written. A tile
+// of 16 TMEM accumulators of 32 columns; warps 0-3 and 4-7, two groups that take
+// alternate tiles, read each one back as soon as its MMAs commit, add the bias,
+// apply the ReLU, store BF16 into the next layer's activation buffer and mark the
+// (layer, tile) written (a tile's read-back is a chain of 500 to 700 cycles, so
+// one group of eight warps waits where two overlap). A tile
 // u of the next layer reads the halo rows of tiles u - 1 .. u + 1, so its
 // MMAs start once those three are written, while the epilogue of the later
 // tiles runs. Two activation buffers alternate: B holds the input and layer
-// 2's output, A layers 1 and 3. Layouts are the 32 -> 32 kernel's: a
-// 34-pixel halo pitch, channel-group major (8 channels = 16 bytes per
-// pixel), each 3x3 tap a descriptor offset, 9 M = 128 tiles of virtual
-// pixels.
+// 2's output, A layers 1 and 3. Layouts: a 34-pixel halo pitch, channel-group
+// major (8 channels = 16 bytes per pixel), each 3x3 tap a descriptor offset, 9 M
+// = 128 tiles of virtual pixels.
 //
 // One thread issuing tcgen05.mma (M = 128, K = 16) sustains one per ~63
 // cycles whatever N up to 128, and between a tile's commit and its next
@@ -515,18 +516,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, int limi
 //    tails are zeroed again after); after the last tile the epilogue forms
 //    logit[o] = b4 + sum_t z[o + off_t][t] in one pass.
 // The next image's 4 KB input arrives by one bulk copy while this image
-// runs and is repacked into B's first group at layer 4's first tile. The
-// one epilogue group consumes the tiles in order, waiting on each commit,
-// so whenever it writes a buffer every MMA issued before that reads it has
-// completed, whichever warp issued it. The top k cells of the logits
-// (first index on ties) are written per image, and the logits themselves
-// when asked.
+// runs; a third group of four warps repacks it into B's first group once layer
+// 3's MMAs are done, and makes this image's logits and its top k cells (first
+// index on ties) while the others go on with the next image: only z has to be
+// read before layer 2 of that image is stored over it.
+//
+// No read of a buffer is overtaken: the epilogue of layer l + 1's tile u waits
+// for MMAs that were issued after layer l's tiles u - 1 .. u + 1 were stored, so
+// after every MMA that read those rows of the buffer it stores into; layer 4's z
+// and the repacked input go over B once all of layer 3's tiles are stored.
+// Measured (8160 images, k = 4): 784 us with one epilogue group that also made the
+// outputs, 670 us so; of that the tensor pipe takes one M = 128 MMA per ~63
+// cycles, 360 an image.
 //
 // Every slot's tiles come from one issuer (16 is a multiple of the issuer
-// count) and go to the one
-// epilogue group in order, and each (layer, tile) barrier completes once
-// an image, so no parity wait can run a phase ahead of its barrier. Every
-// wait is bounded; a wait that runs out sets the context's status word,
+// count), and each (layer, tile) barrier completes once an image, so no parity
+// wait can run a phase ahead of its barrier. Every wait is bounded; a wait that runs out sets the context's status word,
 // the other warps leave at their next wait, and the CTA drains its MMAs
 // and copy before freeing TMEM.
 namespace lpnet {
@@ -541,23 +546,26 @@ constexpr int OFF_W4 = OFF_W3 + 36 * 32 * 16;  // 4 k-groups x 16 n (taps 0-8, z
 constexpr int OFF_STAGE = OFF_W4 + 4 * 16 * 16;  // the next image's input, 32 x 32 x 2 BF16
 constexpr int OFF_Z = OFF_B + REGION;          // layer 4's z, [9 taps][1152 rows] FP32, in B's groups 1-3
 constexpr int OFF_LOG = OFF_STAGE + 4096;      // 1024 FP32 logits
-constexpr int OFF_RED = OFF_LOG + 1024 * 4;    // 2 x 8 u64 per-warp maxima (by round parity)
+constexpr int OFF_RED = OFF_LOG + 1024 * 4;    // 2 x 4 u64 per-warp maxima (by round parity)
 constexpr int OFF_BAR = OFF_RED + 2 * 8 * 8;
 constexpr int TILES = 9;                       // ceil(32 * 34 / 128)
 constexpr int NSLOT = 16;                      // TMEM accumulators of 32 columns
 constexpr int ISSUERS = 4;
 constexpr int BAR_FULL = 0;                    // [16] MMAs of a slot committed
-constexpr int BAR_EMPTY = BAR_FULL + NSLOT;    // [16] a slot read back (8 warp arrivals)
-constexpr int BAR_WRITTEN = BAR_EMPTY + NSLOT; // [3][9] layer l's tile u stored (8 warp arrivals)
-constexpr int BAR_INPUT = BAR_WRITTEN + 3 * TILES;  // the image's input repacked (8 warp arrivals)
+constexpr int BAR_EMPTY = BAR_FULL + NSLOT;    // [16] a slot read back (4 warp arrivals)
+constexpr int BAR_WRITTEN = BAR_EMPTY + NSLOT; // [3][9] layer l's tile u stored (4 warp arrivals)
+constexpr int BAR_INPUT = BAR_WRITTEN + 3 * TILES;  // the image's input repacked (4 warp arrivals)
 constexpr int BAR_STAGE = BAR_INPUT + 1;       // the bulk copy landed
 constexpr int BAR_FIN = BAR_STAGE + 1;         // [4] an issuer's MMAs all completed
 constexpr int NBAR = BAR_FIN + ISSUERS;
-constexpr int OFF_TMEM = OFF_BAR + NBAR * 8;
+constexpr int OFF_BIAS = (OFF_BAR + NBAR * 8 + 15) / 16 * 16;  // layers 1-3, 32 FP32 each
+constexpr int OFF_TMEM = OFF_BIAS + 3 * 32 * 4;
 constexpr int OFF_ABORT = OFF_TMEM + 4;
 constexpr int SMEM = OFF_ABORT + 12;
 constexpr int EPI = 256;                       // 8 epilogue warps
-constexpr int THREADS = EPI + 32 * ISSUERS;
+constexpr int GRP = 128;                       // in two groups
+constexpr int ISSUE_END = EPI / 32 + ISSUERS;  // the output group's first warp
+constexpr int THREADS = EPI + 32 * ISSUERS + GRP;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr int LIMIT = 1 << 22;
 constexpr uint32_t IDESC32 = lptc::IDESC;
@@ -606,6 +614,21 @@ __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, const volati
 
 __device__ __forceinline__ void arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Named barrier 3 over the epilogue and output groups' threads; the OR of `p`.
+__device__ __forceinline__ bool out_or(bool p) {
+  uint32_t r;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred q, r;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "bar.red.or.pred r, 3, %2, q;\n\t"
+      "selp.b32 %0, 1, 0, r;\n\t}\n"
+      : "=r"(r)
+      : "r"((uint32_t)p), "n"(EPI + GRP)
+      : "memory");
+  return r != 0;
 }
 
 // Named barrier 1 over the 256 epilogue threads; the OR of `p` over them.
@@ -672,7 +695,7 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
   if (tid == 0) {
     for (int i = 0; i < NBAR; i++) {
       const bool one = (i >= BAR_FULL && i < BAR_FULL + NSLOT) || i == BAR_STAGE || i >= BAR_FIN;
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar(i)), "r"(one ? 1 : 8));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar(i)), "r"(one ? 1 : GRP / 32));
     }
     *abort_w = 0;
     asm volatile("fence.mbarrier_init.release.cluster;");
@@ -696,6 +719,7 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
     w2s[q] = W2[nn * 288 + kg * 8 + e];
     w3s[q] = W3[nn * 288 + kg * 8 + e];
   }
+  if (tid < 96) reinterpret_cast<float*>(sm_ + OFF_BIAS)[tid] = (tid < 32 ? b1 : (tid < 64 ? b2 : b3))[tid & 31];
   uint16_t* w4s = reinterpret_cast<uint16_t*>(sm_ + OFF_W4);
   for (int q = tid; q < 4 * 16 * 8; q += THREADS) {
     // n = tap t (rows 9-15 zero), k = channel.
@@ -709,7 +733,7 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
   const uint32_t tmem = *tmem_slot;
   const int first = blockIdx.x, stride = gridDim.x;
 
-  if (warp >= EPI / 32) {
+  if (warp >= EPI / 32 && warp < ISSUE_END) {
     // ---- the MMA warps: issuer i takes the tiles t = i, i + ISSUERS, ... of
     // the 36 an image (layers 1-4 x 9); lane 0 issues, the whole warp waits.
     const int iss = warp - EPI / 32;
@@ -786,20 +810,21 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
     if (iss == 0) mbar_wait(bar(BAR_STAGE), (uint32_t)(copies - 1) & 1u, LIMIT);
     __syncwarp();
   } else {
-    // ---- the epilogue warps: warp w reads TMEM lanes 32 (w % 4) .. +31,
-    // columns 16 (w / 4) .. +15 of each accumulator.
-    const int lq = warp & 3, half = warp >> 2;
+    // ---- the epilogue warps, in two groups of four: warp w reads TMEM lanes 32
+    // (w % 4) .. +31, all 32 columns, of its group's accumulators. A third group
+    // repacks inputs and makes an image's outputs while they go on.
+    const int lq = warp & 3, grp = warp >= ISSUE_END ? 2 : warp >> 2, gt = tid & 127;
     float* z = reinterpret_cast<float*>(sm_ + OFF_Z);
     float* log_s = reinterpret_cast<float*>(sm_ + OFF_LOG);
     unsigned long long* red = reinterpret_cast<unsigned long long*>(sm_ + OFF_RED);
     const float bias4 = __ldg(b4);
     bool ok = true;
-    // One image's input from the stage into B's first group: pixel (y, x)
-    // holds the pairs of (x - 1, x, x + 1) (zero outside the image) and two
-    // zeros; then the hand-over to the MMA warps.
+    // One image's input from the stage into B's first group (the output group):
+    // pixel (y, x) holds the pairs of (x - 1, x, x + 1) (zero outside the image)
+    // and two zeros; then the hand-over to the MMA warps.
     auto repack = [&]() {
       const uint32_t* st = reinterpret_cast<const uint32_t*>(sm_ + OFF_STAGE);
-      for (int p = tid; p < 1024; p += EPI) {
+      for (int p = gt; p < 1024; p += GRP) {
         const int y = p >> 5, x = p & 31;
         const uint32_t l = x > 0 ? st[p - 1] : 0u, c = st[p], r = x < 31 ? st[p + 1] : 0u;
         *reinterpret_cast<uint4*>(sm_ + OFF_B + ((y + 1) * 34 + x + 1) * 16) = make_uint4(l, c, r, 0u);
@@ -808,9 +833,20 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
       __syncwarp();
       if (lane == 0) arrive(bar(BAR_INPUT));
     };
-    // The logits from z (halo rows past the last tile are zero).
-    auto outputs = [&]() {
-      for (int o = tid; o < 32 * 34; o += EPI) {
+    // A bounded wait by the whole warp; one that runs out stops the other warps'.
+    auto wait_warp = [&](int i, uint32_t parity) {
+      const bool done = __all_sync(0xffffffffu, wait(bar(i), parity, abort_w));
+      if (!done && lane == 0) *abort_w = 1;
+      return done;
+    };
+    auto group_sync = [&]() {
+      __syncwarp();
+      asm volatile("bar.sync 2, %0;" ::"n"(GRP) : "memory");
+    };
+    // An image's logits from z, by the output group; then B's groups 1-3 are free.
+    auto make_logits = [&]() {
+      // The logits (halo rows past the last tile are zero).
+      for (int o = gt; o < 32 * 34; o += GRP) {
         const int y = o / 34, x = o % 34;
         if (x < 32) {
           float acc = 0.f;
@@ -822,76 +858,8 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
           log_s[y * 32 + x] = acc + bias4;
         }
       }
-    };
-    ok = !epi_or(!wait(bar(BAR_STAGE), 0u, abort_w));
-    if (ok) repack();
-    int j = 0;
-    for (int img = first; img < n && ok; img += stride, j++) {
-      for (int layer = 0; layer < 3 && ok; layer++) {
-        const uint32_t dst = layer == 1 ? OFF_B : OFF_A;
-        const float* bias = layer == 0 ? b1 : layer == 1 ? b2 : b3;
-        float bb[16];
-#pragma unroll
-        for (int q = 0; q < 16; q++) bb[q] = __ldg(bias + half * 16 + q);
-        for (int u = 0; u < TILES; u++) {
-          const uint32_t seq = (uint32_t)j * (4u * TILES) + (uint32_t)(layer * TILES + u);
-          const uint32_t s = seq % NSLOT, use = seq / NSLOT;
-          ok = !epi_or(!wait(bar(BAR_FULL + (int)s), use & 1u, abort_w));
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          uint32_t r[16];
-          tmem_ld16(tmem + ((uint32_t)(32 * lq) << 16) + s * 32 + (uint32_t)(half * 16), r);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) arrive(bar(BAR_EMPTY + (int)s));
-          const int v = u * 128 + 32 * lq + lane, y = v / 34, x = v % 34;
-          if (y < 32 && x < 32) {
-            uint32_t o[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++)
-              o[q] = pack_bf16(fmaxf(__uint_as_float(r[2 * q]) + bb[2 * q], 0.f),
-                               fmaxf(__uint_as_float(r[2 * q + 1]) + bb[2 * q + 1], 0.f));
-            uint8_t* px = sm_ + dst + ((y + 1) * 34 + x + 1) * 16;
-            *reinterpret_cast<uint4*>(px + (2 * half) * REGION) = make_uint4(o[0], o[1], o[2], o[3]);
-            *reinterpret_cast<uint4*>(px + (2 * half + 1) * REGION) = make_uint4(o[4], o[5], o[6], o[7]);
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) arrive(bar(BAR_WRITTEN + layer * TILES + u));
-        }
-      }
-      if (!ok) break;
-      // Layer 4: z into B's groups 1-3, then the logits in one pass.
-      for (int u = 0; u < TILES; u++) {
-        const uint32_t seq = (uint32_t)j * (4u * TILES) + (uint32_t)(3 * TILES + u);
-        const uint32_t s = seq % NSLOT, use = seq / NSLOT;
-        ok = !epi_or(!wait(bar(BAR_FULL + (int)s), use & 1u, abort_w));
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (half == 0) {
-          uint32_t r[16];
-          tmem_ld16(tmem + ((uint32_t)(32 * lq) << 16) + s * 32, r);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          float* zs = z + u * 128 + 32 * lq + lane;
-#pragma unroll
-          for (int t = 0; t < 9; t++) zs[t * (TILES * 128)] = __uint_as_float(r[t]);
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) arrive(bar(BAR_EMPTY + (int)s));
-        if (u == 0 && img + stride < n) {
-          // Every layer-3 tile's MMAs are done: B's first group takes the next input.
-          ok = !epi_or(!wait(bar(BAR_STAGE), (uint32_t)(j + 1) & 1u, abort_w));
-          if (!ok) break;
-          repack();
-        }
-      }
-      if (!ok) break;
-      epi_sync();  // z complete
-      outputs();
-      epi_sync();  // z read: B's groups 1-3 get their zero halo rings and tails back
-      for (int q = tid; q < 3 * (34 * 34 - 32 * 32 + lptc::NV - 34 * 34); q += EPI) {
+      group_sync();  // z read: B's groups 1-3 get their zero halo rings and tails back
+      for (int q = gt; q < 3 * (34 * 34 - 32 * 32 + lptc::NV - 34 * 34); q += GRP) {
         const int g = 1 + q / (lptc::NV - 32 * 32), r = q % (lptc::NV - 32 * 32);
         // r-th non-interior pixel of the group: the ring (34 x 34 minus the
         // 32 x 32 interior), then the tail past 34 x 34.
@@ -902,21 +870,23 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
         else h = 34 * 34 + (r - 132);                          // tail
         *reinterpret_cast<uint4*>(sm_ + OFF_B + g * REGION + h * 16) = make_uint4(0, 0, 0, 0);
       }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    };
+    auto outputs = [&](int img) {
       if (logits)
-        for (int q = tid; q < 1024; q += EPI) logits[(size_t)img * 1024 + q] = log_s[q];
+        for (int q = gt; q < 1024; q += GRP) logits[(size_t)img * 1024 + q] = log_s[q];
       // The top k cells, best first, the first index among equal scores:
-      // each thread keeps its four scores in registers; a round publishes
+      // each thread keeps its eight scores in registers; a round publishes
       // the warp maxima (one barrier, the array alternating by round),
       // every thread reduces them alike and the owner drops the chosen cell.
-      float mine[4];
+      float mine[8];
 #pragma unroll
-      for (int i = 0; i < 4; i++) mine[i] = log_s[tid + EPI * i];
+      for (int i = 0; i < 8; i++) mine[i] = log_s[gt + GRP * i];
       for (int round = 0; round < k; round++) {
         unsigned long long best = 0;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const unsigned long long key =
-              ((unsigned long long)fkey(mine[i]) << 32) | (uint32_t)(1023 - (tid + EPI * i));
+        for (int i = 0; i < 8; i++) {
+          const unsigned long long key = ((unsigned long long)fkey(mine[i]) << 32) | (uint32_t)(1023 - (gt + GRP * i));
           best = key > best ? key : best;
         }
 #pragma unroll
@@ -924,18 +894,104 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
           const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
           best = other > best ? other : best;
         }
-        unsigned long long* rr = red + (round & 1) * 8;
-        if (lane == 0) rr[warp] = best;
-        epi_sync();
+        unsigned long long* rr = red + (round & 1) * 4;
+        if (lane == 0) rr[lq] = best;
+        group_sync();
         unsigned long long b = rr[0];
 #pragma unroll
-        for (int w = 1; w < 8; w++) b = rr[w] > b ? rr[w] : b;
+        for (int w = 1; w < 4; w++) b = rr[w] > b ? rr[w] : b;
         const int cell = 1023 - (int)(b & 0x3ffu);
-        if (tid == 0) cells[(size_t)img * k + round] = cell;
+        if (gt == 0) cells[(size_t)img * k + round] = cell;
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-          if (cell == tid + EPI * i) mine[i] = -INFINITY;
+        for (int i = 0; i < 8; i++)
+          if (cell == gt + GRP * i) mine[i] = -INFINITY;
       }
+    };
+    // Tiles u0, u0 + step, ... of layer 1, 2 or 3 (layer = 0, 1, 2) of image j.
+    auto tiles = [&](int j, int layer, int u0, int step) {
+      const uint32_t dst = layer == 1 ? OFF_B : OFF_A;
+      float bb[32];
+#pragma unroll
+      for (int q = 0; q < 32; q++) bb[q] = reinterpret_cast<const float*>(sm_ + OFF_BIAS)[layer * 32 + q];
+      for (int u = u0; u < TILES && ok; u += step) {
+        const uint32_t seq = (uint32_t)j * (4u * TILES) + (uint32_t)(layer * TILES + u);
+        const uint32_t s = seq % NSLOT, use = seq / NSLOT;
+        ok = wait_warp(BAR_FULL + (int)s, use & 1u);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t r[2][16];
+        tmem_ld16(tmem + ((uint32_t)(32 * lq) << 16) + s * 32, r[0]);
+        tmem_ld16(tmem + ((uint32_t)(32 * lq) << 16) + s * 32 + 16u, r[1]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive(bar(BAR_EMPTY + (int)s));
+        const int v = u * 128 + 32 * lq + lane, y = v / 34, x = v % 34;
+        if (y < 32 && x < 32) {
+          uint8_t* px = sm_ + dst + ((y + 1) * 34 + x + 1) * 16;
+#pragma unroll
+          for (int g = 0; g < 4; g++) {
+            uint32_t o[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              const int c = 8 * g + 2 * q;
+              o[q] = pack_bf16(fmaxf(__uint_as_float(r[c >> 4][c & 15]) + bb[c], 0.f),
+                               fmaxf(__uint_as_float(r[c >> 4][(c & 15) + 1]) + bb[c + 1], 0.f));
+            }
+            *reinterpret_cast<uint4*>(px + g * REGION) = make_uint4(o[0], o[1], o[2], o[3]);
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive(bar(BAR_WRITTEN + layer * TILES + u));
+      }
+    };
+    if (grp == 2) {
+      ok = wait_warp(BAR_STAGE, 0u);
+      if (ok) repack();
+    }
+    int j = 0, last = -1;
+    for (int img = first; img < n; img += stride, j++) {
+      if (grp < 2) tiles(j, 0, grp, 2);
+      else if (last >= 0) make_logits();
+      ok = !out_or(!ok);  // z is read: B's groups 1-3 are free
+      if (!ok) break;
+      if (grp < 2) {
+        tiles(j, 1, grp, 2);
+        tiles(j, 2, grp, 2);
+      } else if (last >= 0) {
+        outputs(last);
+      }
+      // Once every layer-3 tile's MMAs are done: the next input into B's first
+      // group, layer 4's z into the others.
+      for (int u = 0; u < TILES && ok; u++) ok = wait_warp(BAR_WRITTEN + 2 * TILES + u, (uint32_t)j & 1u);
+      if (ok && grp == 2 && img + stride < n) {
+        ok = wait_warp(BAR_STAGE, (uint32_t)(j + 1) & 1u);
+        if (ok) repack();
+      }
+      for (int u = grp; grp < 2 && u < TILES && ok; u += 2) {
+        const uint32_t seq = (uint32_t)j * (4u * TILES) + (uint32_t)(3 * TILES + u);
+        const uint32_t s = seq % NSLOT, use = seq / NSLOT;
+        ok = wait_warp(BAR_FULL + (int)s, use & 1u);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t r[16];
+        tmem_ld16(tmem + ((uint32_t)(32 * lq) << 16) + s * 32, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive(bar(BAR_EMPTY + (int)s));
+        float* zs = z + u * 128 + 32 * lq + lane;
+#pragma unroll
+        for (int t = 0; t < 9; t++) zs[t * (TILES * 128)] = __uint_as_float(r[t]);
+      }
+      ok = !out_or(!ok);  // z complete, and layer 4's MMAs: A takes the next layer 1
+      if (!ok) break;
+      last = img;
+    }
+    if (ok && grp == 2 && last >= 0) {
+      make_logits();
+      outputs(last);
     }
     if (!ok && tid == 0) {
       atomicExch(status, 1u);  // DEV_TIMEOUT
