@@ -868,6 +868,26 @@ vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* header,
                                    const int8_t* mb_segment, const uint8_t* token_prob_updates,
                                    uint8_t* out, uint64_t out_capacity, uint64_t* out_size);
 
+/* A whole P frame from host planes (encode_p_frame_multi_ref_auto_loop_filter,
+ * src/encoder.rs:9373, intra picking off): vp8a_analyse_inter_frame (with
+ * `proposals`, optional, as vp8a_analyse_inter_frame_proposals takes them),
+ * vp8a_reconstruct_inter_frame, with `auto_lf` vp8a_select_filter_params (else
+ * the header's level and sharpness), vp8a_filter_frame into `filtered` when the
+ * level is not 0, and vp8a_write_inter_frame, with the same results. Every
+ * buffer but `proposals` is host memory, no output overlaps an input;
+ * segmentation is off. Returns
+ * VP8A_E_INVALID_ARGUMENT with *out_size > out_capacity when `out` is too small
+ * (the other outputs are written). */
+vp8a_status vp8a_encode_inter_frame(vp8a_ctx* ctx, const vp8a_i420* frame, const vp8a_planes* refs,
+                                    const uint8_t* ref_ids, uint32_t n_refs,
+                                    const vp8a_mv_contexts* mv_contexts, double lambda,
+                                    const vp8a_mv* proposals, const vp8a_frame_header* header,
+                                    uint32_t auto_lf, vp8a_mb_decision* decisions, int16_t* coeffs,
+                                    uint8_t* mb_flags, vp8a_mb_lf_info* lf_info,
+                                    const vp8a_planes* recon, const vp8a_planes* filtered,
+                                    uint8_t* level_out, uint8_t* sharpness_out, uint8_t* out,
+                                    uint64_t out_capacity, uint64_t* out_size);
+
 #ifdef __cplusplus
 }
 #endif

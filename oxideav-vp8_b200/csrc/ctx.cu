@@ -273,6 +273,9 @@ vp8a_status vp8a_ctx_destroy(vp8a_ctx* ctx) {
   for (int k = 0; k < vp8a_ctx::UP_SLOTS; k++)
     if (ctx->up_ev[k]) cudaEventDestroy(ctx->up_ev[k]);
   if (ctx->up_host) cudaFreeHost(ctx->up_host);
+  if (ctx->down_host) cudaFreeHost(ctx->down_host);
+  if (ctx->aux_ev) cudaEventDestroy(ctx->aux_ev);
+  if (ctx->aux) cudaStreamDestroy(ctx->aux);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return VP8A_OK;

@@ -14,33 +14,39 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <thread>
 #include <vector>
 
 #include "../../include/vp8a.h"
 #include "coeff_tables.h"
+#include "emit.h"
 
 namespace vp8a_emit {
 namespace {
 
 // RFC 6386 §7.3 boolean encoder (BoolEncoder, src/encoder.rs:255-500):
 // `bottom` holds the low end of the interval with 24 bits of headroom;
-// a byte is complete after `pending` more shifts.
-struct BoolWriter {
-  std::vector<uint8_t> out;
+// a byte is complete after `pending` more shifts. The chain from one put to the
+// next is what bounds the writer, so the whole state is a value that the callers'
+// loops keep in registers (bytes stored through a member's pointer would have it
+// reloaded at every put); room for the bytes is the owner's to keep.
+struct BoolCoder {
   uint32_t range = 255, bottom = 0;
   int pending = 24;
+  uint8_t *p, *begin;
 
+  explicit BoolCoder(uint8_t* at) : p(at), begin(at) {}
   void carry() {
-    for (size_t i = out.size(); i-- > 0;) {
-      if (out[i] != 255) {
-        out[i]++;
+    for (uint8_t* q = p; q-- > begin;) {
+      if (*q != 255) {
+        ++*q;
         return;
       }
-      out[i] = 0;
+      *q = 0;
     }
   }
-  void put(int prob, bool bit) {
+  __attribute__((always_inline)) void put(int prob, bool bit) {
     const uint32_t split = 1 + (((range - 1) * (uint32_t)prob) >> 8);
     // Branch-free choice of the sub-interval: the bit is data, not control.
     const uint32_t m = 0u - (uint32_t)bit;
@@ -58,11 +64,51 @@ struct BoolWriter {
     bottom <<= pending - 1;
     if (bottom & 0x80000000u) carry();
     bottom <<= 1;
-    out.push_back((uint8_t)(bottom >> 24));
+    *p++ = (uint8_t)(bottom >> 24);
     bottom &= 0xFFFFFFu;
     const int rest = shift - pending;
     bottom <<= rest;
     pending = 8 - rest;
+  }
+  // flush_bool_encoder (RFC 6386 §7.3): settle a carry into the output,
+  // then write the four bytes that hold the rest of `bottom`.
+  void flush() {
+    const int c = pending;
+    uint32_t v = bottom;
+    if (v & (1u << (32 - c))) carry();
+    v <<= c & 7;
+    for (int k = c >> 3; k > 0; k--) v <<= 8;
+    for (int k = 0; k < 4; k++) {
+      *p++ = (uint8_t)(v >> 24);
+      v <<= 8;
+    }
+  }
+};
+
+// A growing output for a coder: room(w, k) before k more puts.
+struct Bytes {
+  std::unique_ptr<uint8_t[]> data;
+  size_t size;
+  explicit Bytes(size_t n) : data(new uint8_t[n]), size(n) {}
+  void room(BoolCoder& w, size_t k) {
+    const size_t used = (size_t)(w.p - w.begin);
+    if (size - used >= k) return;
+    size = 2 * size + k;
+    std::unique_ptr<uint8_t[]> to(new uint8_t[size]);
+    std::memcpy(to.get(), w.begin, used);
+    data = std::move(to);
+    w.begin = data.get();
+    w.p = w.begin + used;
+  }
+};
+
+// The coder with its own output, for the header and the modes.
+struct BoolWriter {
+  Bytes bytes{4096};
+  BoolCoder w{bytes.data.get()};
+  void put(int prob, bool bit) {
+    bytes.room(w, 8);
+    w.put(prob, bit);
   }
   void literal(uint32_t v, int bits) {
     while (bits-- > 0) put(128, (v >> bits) & 1);
@@ -71,19 +117,10 @@ struct BoolWriter {
     literal((uint32_t)std::abs(v), bits);
     put(128, v < 0);
   }
-  // flush_bool_encoder (RFC 6386 §7.3): settle a carry into the output,
-  // then write the four bytes that hold the rest of `bottom`.
   std::vector<uint8_t> finish() {
-    const int c = pending;
-    uint32_t v = bottom;
-    if (v & (1u << (32 - c))) carry();
-    v <<= c & 7;
-    for (int k = c >> 3; k > 0; k--) v <<= 8;
-    for (int k = 0; k < 4; k++) {
-      out.push_back((uint8_t)(v >> 24));
-      v <<= 8;
-    }
-    return std::move(out);
+    bytes.room(w, 8);
+    w.flush();
+    return std::vector<uint8_t>(w.begin, w.p);
   }
 };
 
@@ -132,7 +169,7 @@ using Probs = uint8_t[4][8][3][11];
 
 // encode_coeff_block_into (src/encoder.rs:1915): one block's tokens in
 // zigzag order from `first`; returns the block's nonzero count.
-int code_block(BoolWriter& w, const Probs& probs, int plane, int first, int ctx, const int16_t* raster) {
+__attribute__((always_inline)) inline int code_block(BoolCoder& w, const Probs& probs, int plane, int first, int ctx, const int16_t* raster) {
   int16_t scan[16];
   int last = -1;
   for (int i = 0; i < 16; i++) {
@@ -318,26 +355,9 @@ int mb_blocks(const int16_t* mb, bool has_y2, BlockRef* out) {
   return n;
 }
 
-// Whether the block has a nonzero coefficient it codes (raster and scan
-// order hold the same set past the DC): four 64-bit ORs.
-bool block_nonzero(const BlockRef& b) {
-  uint64_t w[4];
-  std::memcpy(w, b.c, sizeof w);
-  if (b.first) w[0] &= ~(uint64_t)0xFFFF;
-  return (w[0] | w[1] | w[2] | w[3]) != 0;
-}
-
 }  // namespace
-}  // namespace vp8a_emit
 
-using namespace vp8a_emit;
-
-extern "C" vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* h, const vp8a_mb_decision* decisions,
-                                               const int16_t* coeffs, const int8_t* mb_segment,
-                                               const uint8_t* token_prob_updates, uint8_t* out,
-                                               uint64_t out_capacity, uint64_t* out_size) {
-  if (!h || !decisions || !coeffs || !out_size) return VP8A_E_INVALID_ARGUMENT;
-  *out_size = 0;
+vp8a_status check_header(const vp8a_frame_header* h, const int8_t* mb_segment) {
   if (h->width == 0 || h->width > 0x3FFF || h->height == 0 || h->height > 0x3FFF) return VP8A_E_INVALID_DIMENSIONS;
   if (h->quant.y_ac_qi > 127) return VP8A_E_QUANT_INDEX_OUT_OF_RANGE;
   if (h->loop_filter_level > 63) return VP8A_E_LOOP_FILTER_LEVEL_OUT_OF_RANGE;
@@ -360,50 +380,64 @@ extern "C" vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* h, const 
       if (std::abs((int)h->segment_quant[k]) > 127 || std::abs((int)h->segment_lf[k]) > 63)
         return VP8A_E_INVALID_ARGUMENT;
   }
-  const int cols = (int)((h->width + 15) / 16), rows = (int)((h->height + 15) / 16);
-  const size_t n_mbs = (size_t)cols * rows;
+  return VP8A_OK;
+}
 
-  // Probabilities the tokens are coded against: the §13.5 defaults with the
-  // caller's updates laid over them (merge_default_token_probs).
-  Probs probs;
-  std::memcpy(probs, kDefaultCoeffProbs, sizeof probs);
-  if (token_prob_updates) {
-    uint8_t* flat = &probs[0][0][0][0];
-    for (int i = 0; i < 1056; i++)
-      if (token_prob_updates[i]) flat[i] = token_prob_updates[i];
-  }
-
+vp8a_status scan_frame(const vp8a_frame_header* h, const vp8a_mb_decision* decisions, const int16_t* coeffs,
+                       const int8_t* mb_segment, FrameTokens& t) {
+  const size_t n_mbs = (size_t)((h->width + 15) / 16) * ((h->height + 15) / 16);
   // Per MB: the wire segment, skip flag (no nonzero block among those the
   // MB codes, src/encoder.rs:8746-8769) and the per-block nonzero flags.
-  std::vector<uint8_t> skip(n_mbs), seg(n_mbs, 0);
-  std::vector<uint32_t> nzmask(n_mbs);  // bit b: coding-order block b has a coded nonzero
-  uint32_t n_skip = 0, n_ref[4] = {0, 0, 0, 0}, seg_count[4] = {0, 0, 0, 0};
+  t.skip.resize(n_mbs);
+  t.seg.assign(n_mbs, 0);
+  t.nzmask.resize(n_mbs);
   for (size_t i = 0; i < n_mbs; i++) {
     const vp8a_mb_decision& d = decisions[i];
     if (d.ref_frame < VP8A_REF_LAST || d.ref_frame > VP8A_REF_ALTREF || d.mode > VP8A_MODE_SPLIT)
       return VP8A_E_INVALID_ARGUMENT;  // intra MBs are not produced by the device analysis
     if (d.mode == VP8A_MODE_SPLIT && d.partition > VP8A_PART_MV16) return VP8A_E_INVALID_ARGUMENT;
-    BlockRef blk[25];
-    const int nb = mb_blocks(coeffs + 400 * i, d.mode != VP8A_MODE_SPLIT, blk);
-    uint32_t mask = 0;
-    for (int b = 0; b < nb; b++) {
-      if (!block_nonzero(blk[b])) continue;
-      mask |= 1u << b;
-      for (int k = blk[b].first; k < 16; k++)
-        if (std::abs((int)blk[b].c[k]) > 2114) return VP8A_E_COEFFICIENT_OUT_OF_RANGE;
+    // Coding-order block b: with a Y2 block, Y2 first and the Y blocks without
+    // their DC. The range check takes all 400 coefficients; only one outside is
+    // looked at block by block.
+    const int16_t* mb = coeffs + 400 * i;
+    const bool has_y2 = d.mode != VP8A_MODE_SPLIT;
+    uint32_t all = 0, bad = 0;
+    for (int b = 0; b < 25; b++) {
+      uint64_t w[4];
+      std::memcpy(w, mb + 16 * b, sizeof w);
+      if (has_y2 && b >= 1 && b <= 16) w[0] &= ~(uint64_t)0xFFFF;
+      all |= (uint32_t)((w[0] | w[1] | w[2] | w[3]) != 0) << b;
     }
-    nzmask[i] = mask;
-    skip[i] = mask == 0;
-    n_skip += skip[i];
-    n_ref[d.ref_frame]++;
+    for (int k = 0; k < 400; k++) bad |= (uint32_t)((uint16_t)(mb[k] + 2114) > 2u * 2114);
+    const uint32_t mask = has_y2 ? all : all >> 1;
+    if (bad) {
+      BlockRef blk[25];
+      const int nb = mb_blocks(mb, has_y2, blk);
+      for (int b = 0; b < nb; b++)
+        for (int k = blk[b].first; k < 16; k++)
+          if (std::abs((int)blk[b].c[k]) > 2114) return VP8A_E_COEFFICIENT_OUT_OF_RANGE;
+    }
+    t.nzmask[i] = mask;
+    t.skip[i] = mask == 0;
+    t.n_skip += t.skip[i];
+    t.n_ref[d.ref_frame]++;
     if (h->segmentation) {
       const int s = mb_segment[i] < 0 ? 0 : mb_segment[i];
       if (s > 3) return VP8A_E_INVALID_ARGUMENT;
-      seg[i] = (uint8_t)s;
-      seg_count[s]++;
+      t.seg[i] = (uint8_t)s;
+      t.seg_count[s]++;
     }
   }
+  return VP8A_OK;
+}
 
+vp8a_status first_partition(const vp8a_frame_header* h, const vp8a_mb_decision* decisions,
+                            const uint8_t* token_prob_updates, const FrameTokens& t, std::vector<uint8_t>& out) {
+  const int cols = (int)((h->width + 15) / 16), rows = (int)((h->height + 15) / 16), np = h->n_partitions;
+  const size_t n_mbs = (size_t)cols * rows;
+  const int8_t* qd = &h->quant.y_dc_delta;
+  const std::vector<uint8_t>&skip = t.skip, &seg = t.seg;
+  const uint32_t n_skip = t.n_skip, *n_ref = t.n_ref, *seg_count = t.seg_count;
   // ---- §19.2 first partition: the frame header
   BoolWriter hdr;
   uint8_t seg_probs[3] = {0, 0, 0};
@@ -548,8 +582,25 @@ extern "C" vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* h, const 
       above[c] = cur;
     }
   }
-  const std::vector<uint8_t> first = hdr.finish();
-  if (first.size() > 0x7FFFF) return VP8A_E_FIRST_PARTITION_TOO_LARGE;
+  out = hdr.finish();
+  return out.size() > 0x7FFFF ? VP8A_E_FIRST_PARTITION_TOO_LARGE : VP8A_OK;
+}
+
+void code_tokens(const vp8a_frame_header* h, const vp8a_mb_decision* decisions, const int16_t* coeffs,
+                 const uint8_t* token_prob_updates, FrameTokens& t) {
+  const int cols = (int)((h->width + 15) / 16), rows = (int)((h->height + 15) / 16), np = h->n_partitions;
+  const size_t n_mbs = (size_t)cols * rows;
+  const std::vector<uint8_t>& skip = t.skip;
+  const std::vector<uint32_t>& nzmask = t.nzmask;
+  // Probabilities the tokens are coded against: the §13.5 defaults with the
+  // caller's updates laid over them (merge_default_token_probs).
+  Probs probs;
+  std::memcpy(probs, kDefaultCoeffProbs, sizeof probs);
+  if (token_prob_updates) {
+    uint8_t* flat = &probs[0][0][0][0];
+    for (int i = 0; i < 1056; i++)
+      if (token_prob_updates[i]) flat[i] = token_prob_updates[i];
+  }
 
   // ---- §13 residual tokens. The §13.3 contexts: one above record per
   // column for the whole frame, one left record per row; a skipped MB
@@ -583,13 +634,18 @@ extern "C" vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* h, const 
       }
     }
   }
-  std::vector<std::vector<uint8_t>> parts(np);
+  auto& parts = t.parts;
+  parts.assign(np, {});
   auto code_partition = [&](int p) {
-    BoolWriter w;
+    // A token is at most 7 tree bits, 11 extra ones and a sign, 7 shifts each.
+    constexpr size_t kMbBytes = 25 * 16 * 19;
+    Bytes bytes(kMbBytes + 64 * n_mbs / np);
+    BoolCoder w(bytes.data.get());
     for (int r = p; r < rows; r += np)
       for (int c = 0; c < cols; c++) {
         const size_t i = (size_t)r * cols + c;
         if (skip[i]) continue;
+        bytes.room(w, kMbBytes + 8);
         BlockRef blk[25];
         const int nb = mb_blocks(coeffs + 400 * i, decisions[i].mode != VP8A_MODE_SPLIT, blk);
         for (int b = 0; b < nb; b++) {
@@ -600,7 +656,9 @@ extern "C" vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* h, const 
             w.put(probs[blk[b].plane][kBands[blk[b].first]][ctx][0], false);
         }
       }
-    parts[p] = w.finish();
+    bytes.room(w, 8);
+    w.flush();
+    parts[p].assign(w.begin, w.p);
   };
   if (np == 1 || n_mbs < 4096) {
     for (int p = 0; p < np; p++) code_partition(p);
@@ -609,7 +667,12 @@ extern "C" vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* h, const 
     for (int p = 0; p < np; p++) th.emplace_back(code_partition, p);
     for (auto& t : th) t.join();
   }
+}
 
+vp8a_status assemble(const std::vector<uint8_t>& first, const FrameTokens& t, uint8_t* out, uint64_t out_capacity,
+                     uint64_t* out_size) {
+  const auto& parts = t.parts;
+  const int np = (int)parts.size();
   // ---- §9.1 frame tag (inter, version 0, shown), first partition, the
   // §9.5 size table (3-byte little-endian sizes of all but the last
   // partition) and the partitions.
@@ -635,4 +698,24 @@ extern "C" vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* h, const 
     o += p.size();
   }
   return VP8A_OK;
+}
+
+}  // namespace vp8a_emit
+
+using namespace vp8a_emit;
+
+extern "C" vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* h, const vp8a_mb_decision* decisions,
+                                               const int16_t* coeffs, const int8_t* mb_segment,
+                                               const uint8_t* token_prob_updates, uint8_t* out,
+                                               uint64_t out_capacity, uint64_t* out_size) {
+  if (!h || !decisions || !coeffs || !out_size) return VP8A_E_INVALID_ARGUMENT;
+  *out_size = 0;
+  FrameTokens t;
+  std::vector<uint8_t> first;
+  vp8a_status s = check_header(h, mb_segment);
+  if (s == VP8A_OK) s = scan_frame(h, decisions, coeffs, mb_segment, t);
+  if (s == VP8A_OK) s = first_partition(h, decisions, token_prob_updates, t, first);
+  if (s != VP8A_OK) return s;
+  code_tokens(h, decisions, coeffs, token_prob_updates, t);
+  return assemble(first, t, out, out_capacity, out_size);
 }

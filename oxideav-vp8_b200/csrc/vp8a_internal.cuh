@@ -35,6 +35,14 @@ struct vp8a_ctx {
   uint8_t* up_host = nullptr;
   cudaEvent_t up_ev[UP_SLOTS] = {};
   unsigned up_next = 0;
+  // Second stream of the whole-frame encode, the event that orders the two, and
+  // pinned memory for one frame's results (created on first use, at most
+  // DOWN_MAX bytes, given back with the context).
+  static constexpr size_t DOWN_MAX = 64 << 20;
+  cudaStream_t aux = nullptr;
+  cudaEvent_t aux_ev = nullptr;
+  uint8_t* down_host = nullptr;
+  size_t down_bytes = 0;
   // The loop-filter sweep's launch shape is chosen by rule (lf.cu); a forced
   // layout (tests) overrides it. last_layout: the last sweep's (passes per
   // CTA, threads, prefetch, CTAs per SM).

@@ -333,8 +333,14 @@ def encode_p_frame(ctx, frame, refs, ref_ids, y_ac_qi, loop_filter_level=0, shar
     coefficients, flags, the loop-filter records and the chosen level and
     sharpness). `proposals` (optional) are second NEWMV candidates for the
     analysis (vp8a_analyse_inter_frame_proposals)."""
-    dec = analyse_inter_frame(ctx, frame, refs, ref_ids, rd_lambda(y_ac_qi), proposals=proposals).reshape(-1)
     quant = abi.quant_indices(y_ac_qi)
+    if _host_frame(frame, refs, ref_ids, y_ac_qi, loop_filter_level, sharpness_level, n_partitions):
+        # One call: the planes go up once, the bitstream is coded beside the device.
+        hdr = abi.frame_header(frame[0].shape[1], frame[0].shape[0], quant, n_partitions=n_partitions,
+                               refresh_last=refresh_last, filter_type=int(simple),
+                               loop_filter_level=loop_filter_level, sharpness_level=sharpness_level)
+        return _encode_host_frame(ctx, frame, refs, ref_ids, rd_lambda(y_ac_qi), hdr, auto_lf, proposals)
+    dec = analyse_inter_frame(ctx, frame, refs, ref_ids, rd_lambda(y_ac_qi), proposals=proposals).reshape(-1)
     recon = tuple(np.zeros_like(p) for p in refs[0])
     lf = np.zeros(dec.size, abi.MB_LF_INFO_DTYPE)
     cf, fl = reconstruct_inter_frame(ctx, frame, refs, ref_ids, dec, quant, recon, lf_info=lf)
@@ -350,6 +356,57 @@ def encode_p_frame(ctx, frame, refs, ref_ids, y_ac_qi, loop_filter_level=0, shar
     bits = write_inter_frame(hdr, dec, cf)
     return bits, out, dict(decisions=dec, coeffs=cf, flags=fl, lf_info=lf, recon=recon, level=level,
                            sharpness=sharp)
+
+
+def _host_frame(frame, refs, ref_ids, y_ac_qi, level, sharpness, n_partitions):
+    """Whether vp8a_encode_inter_frame takes the frame as it is: numpy planes of
+    matching sizes (up to 3840x2160's macroblocks, whose results the call's
+    pinned block holds) and arguments in range. Anything else goes stage by
+    stage, where each stage reports what it refuses."""
+    def plane(p):
+        return isinstance(p, np.ndarray) and p.dtype == np.uint8 and p.ndim == 2 and p.strides[1] == 1 \
+            and p.strides[0] >= p.shape[1]
+    if not (1 <= len(refs) <= 3 and len(refs) == len(ref_ids) and len(frame) == 3
+            and all(plane(p) for f in (frame, *refs) for p in f)):
+        return False
+    h, w = frame[0].shape
+    mbr, mbc = (h + 15) // 16, (w + 15) // 16
+    if not (0 < h <= 0x3FFF and 0 < w <= 0x3FFF and mbr * mbc <= 32400
+            and all(p.shape == ((h + 1) // 2, (w + 1) // 2) and p.strides[0] == frame[1].strides[0] for p in frame[1:])
+            and all(len(r) == 3 and r[0].shape == (16 * mbr, 16 * mbc)
+                    and all(p.shape == (8 * mbr, 8 * mbc) and p.strides[0] == r[1].strides[0] for p in r[1:])
+                    for r in refs)):
+        return False
+    return (all(k in (abi.REF_LAST, abi.REF_GOLDEN, abi.REF_ALTREF) for k in ref_ids) and 0 <= y_ac_qi <= 127
+            and 0 <= level <= 63 and 0 <= sharpness <= 7 and n_partitions in (1, 2, 4, 8))
+
+
+def _encode_host_frame(ctx, frame, refs, ref_ids, lam, hdr, auto_lf, proposals):
+    """encode_p_frame over host planes in one vp8a_encode_inter_frame call."""
+    prs = [planes(*p) for p in refs]
+    parr = (abi.Planes * len(prs))(*prs)
+    ids = np.ascontiguousarray(np.asarray(ref_ids, np.uint8))
+    n = prs[0].mb_cols * prs[0].mb_rows
+    props = proposals if proposals is None or hasattr(proposals, "data_ptr") \
+        else np.ascontiguousarray(proposals, abi.MV_DTYPE)
+    dec, lf = np.empty(n, abi.MB_DECISION_DTYPE), np.empty(n, abi.MB_LF_INFO_DTYPE)
+    cf, fl = np.empty((n, 400), np.int16), np.empty(n, np.uint8)
+    recon, filt = (tuple(np.empty(p.shape, np.uint8) for p in refs[0]) for _ in range(2))
+    out = np.empty(1024 + 600 * n, np.uint8)
+    level, sharp, size = C.c_uint8(), C.c_uint8(), C.c_uint64(0)
+    st = ctx._lib.vp8a_encode_inter_frame(
+        ctx.handle, C.byref(i420(*frame)), C.cast(parr, C.c_void_p), ptr(ids), len(prs),
+        C.byref(abi.default_mv_contexts()), lam, ptr(props), C.byref(hdr), int(bool(auto_lf)), ptr(dec), ptr(cf),
+        ptr(fl), ptr(lf), C.byref(planes(*recon)), C.byref(planes(*filt)), C.byref(level), C.byref(sharp), ptr(out),
+        out.size, C.byref(size))
+    hdr.loop_filter_level, hdr.sharpness_level = level.value, sharp.value
+    if st == abi.E_INVALID_ARGUMENT and size.value > out.size:
+        bits = write_inter_frame(hdr, dec, cf)
+    else:
+        check(st, "vp8a_encode_inter_frame")
+        bits = out[:size.value].tobytes()
+    return bits, filt if level.value else recon, dict(decisions=dec, coeffs=cf, flags=fl, lf_info=lf, recon=recon,
+                                                      level=level.value, sharpness=sharp.value)
 
 
 def reconstruct_inter_frame(ctx, frame, refs, ref_ids, decisions, quant, recon, mb_segment=None,

@@ -71,6 +71,10 @@ PROTOTYPES = {
     "vp8a_dequant_factors": (None, [C.POINTER(abi.QuantIndices), U32, C.c_int32, U32, P]),
     "vp8a_write_inter_frame": (C.c_int, [C.POINTER(abi.FrameHeader), P, P, P, P, P, C.c_uint64,
                                          C.POINTER(C.c_uint64)]),
+    "vp8a_encode_inter_frame": (C.c_int, [P, C.POINTER(abi.I420), P, P, C.c_uint32, C.POINTER(abi.MvContexts),
+                                          C.c_double, P, C.POINTER(abi.FrameHeader), C.c_uint32, P, P, P, P,
+                                          C.POINTER(abi.Planes), C.POINTER(abi.Planes), P, P, P, C.c_uint64,
+                                          C.POINTER(C.c_uint64)]),
     "vp8a_reconstruct_inter_frame": (
         C.c_int,
         [P, C.POINTER(abi.I420), P, P, U32, P, C.POINTER(abi.QuantIndices), P, P, U32, U32, U32,
