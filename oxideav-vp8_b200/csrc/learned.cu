@@ -631,26 +631,6 @@ __device__ __forceinline__ bool out_or(bool p) {
   return r != 0;
 }
 
-// Named barrier 1 over the 256 epilogue threads; the OR of `p` over them.
-__device__ __forceinline__ bool epi_or(bool p) {
-  uint32_t r;
-  __syncwarp();
-  asm volatile(
-      "{\n\t.reg .pred q, r;\n\t"
-      "setp.ne.b32 q, %1, 0;\n\t"
-      "bar.red.or.pred r, 1, 256, q;\n\t"
-      "selp.b32 %0, 1, 0, r;\n\t}\n"
-      : "=r"(r)
-      : "r"((uint32_t)p)
-      : "memory");
-  return r != 0;
-}
-
-__device__ __forceinline__ void epi_sync() {
-  __syncwarp();
-  asm volatile("bar.sync 1, 256;" ::: "memory");
-}
-
 // 16 consecutive 32-bit TMEM columns of this warp's 32 lanes.
 __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
   asm volatile(
@@ -1018,10 +998,13 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
 // context's status word and the abort word, and the CTA leaves once its own
 // copies and MMAs are in (bounded again).
 //
+// Sums grow in the element-wise kernels' order, so results differ from theirs only
+// in the order of the atomics (dW of the last layer: in the order of its chain).
+//
 // Measured at 2048 images, us a launch, with the element-wise kernels and a
 // one-image-a-CTA tcgen05 forward, then with these: 2 -> 32 forward 87 -> 55, 32 ->
-// 32 forward 129 -> 73, dX 943 -> 86, dW 1397 -> 126, 32 -> 1 forward 115 -> 25, dX
-// 153 -> 48, dW 954 -> 28, dW of 2 -> 32 549 -> 48; the training step 6.85 -> 0.85 ms.
+// 32 forward 129 -> 73, dX 943 -> 86, dW 1397 -> 126, 32 -> 1 forward 115 -> 39, dX
+// 153 -> 57, dW 954 -> 28, dW of 2 -> 32 549 -> 75; the training step 6.85 -> 0.90 ms.
 namespace lptrain {
 using lpnet::arrive;
 using lpnet::mma;
@@ -1072,12 +1055,6 @@ __device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
                : "r"(addr)
                : "memory");
 }
-__device__ __forceinline__ void ldsm2t(uint32_t addr, uint32_t (&r)[2]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
-               : "=r"(r[0]), "=r"(r[1])
-               : "r"(addr)
-               : "memory");
-}
 __device__ __forceinline__ float bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 // Two channels of `v` where the same channels of x are above zero (the ReLU's
@@ -1090,6 +1067,32 @@ __device__ __forceinline__ uint32_t relu_mask(uint32_t v, uint32_t x) {
 // consecutive pixels' groups lie on distinct banks.
 __device__ __forceinline__ uint32_t swz(int p, int cg) { return (uint32_t)(p * 64 + (((cg ^ (p >> 1)) & 3) << 4)); }
 
+// db over half an image of dY in a stage at `tile`: lane = channel, pixel after
+// pixel. One FP32 chain a group of LP_WCPB halves, the element-wise kernel's: a
+// bias gradient is a small difference of large sums, and another order of them
+// moves it by up to 2e-4. 512 dependent additions take less time than a stage's
+// MMAs, on a warp of their own.
+__device__ __forceinline__ void db_chain(uint32_t tile, int lane, float& sum) {
+  uint32_t at[4];
+#pragma unroll
+  for (int r = 0; r < 4; r++) at[r] = tile + (uint32_t)((((lane >> 3) ^ r) & 3) << 4) + (lane & 7) * 2;
+  uint32_t v[2][16];
+  auto load = [&](int p, uint32_t (&to)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      asm volatile("ld.shared.u16 %0, [%1];" : "=r"(to[i]) : "r"(at[(i >> 1) & 3] + (uint32_t)(p + i) * 64));
+  };
+  load(0, v[0]);
+#pragma unroll 1
+  for (int p = 0; p < 512; p += 32) {
+    load(p + 16, v[1]);
+#pragma unroll
+    for (int i = 0; i < 16; i++) sum += __uint_as_float(v[0][i] << 16);
+    if (p + 32 < 512) load(p + 32, v[0]);
+#pragma unroll
+    for (int i = 0; i < 16; i++) sum += __uint_as_float(v[1][i] << 16);
+  }
+}
 }  // namespace lptrain
 
 // The 32 -> 32 convolution, forward or (BWD) the gradient of its input. An
@@ -1324,14 +1327,16 @@ __global__ void __launch_bounds__(lptc3::THREADS, 1)
 // adds a group's sums with one atomic per weight: the FP32 chains (512 MMA steps)
 // are lp_conv_bwd_w_smem_kernel's, pixel by pixel, so the partial sums are the
 // same bits (four shorter chains a warp each measured 20 % less time and gradients
-// 2e-5 apart). That fixes K, so the twelve warps split N: warp w holds 8 input
+// 2e-5 apart). That fixes K, so six warps split N: warp w holds 16 input
 // channels (w / 3) and (ROWS = 3) kernel row w % 3, or (ROWS = 1: few groups, one
-// kernel row a CTA) kernel column w % 3.
+// kernel row a CTA) kernel column w % 3. Two more load the stages and add up db.
+// (Twelve warps of 8 channels each keep shared memory busier than the tensor
+// cores: 126 us at 2048 images without db and 175 with it, 126 with it so.)
 constexpr int LP_WCPB = 16;  // half images whose gradients one FP32 chain adds up
 namespace lpdw {
 constexpr int X_BYTES = 18 * 34 * 64, X_SPACE = (X_BYTES + 511) / 512 * 512;
 constexpr int STAGE = X_SPACE + lptrain::HALF_BYTES;
-constexpr int STAGES = 3, WARPS = 12, THREADS = (WARPS + 1) * 32;
+constexpr int STAGES = 3, WARPS = 6, THREADS = (WARPS + 2) * 32;  // + db, + loads
 constexpr int OFF_BAR = STAGES * STAGE;
 constexpr int SMEM = OFF_BAR + 2 * STAGES * 8 + 8 + 512;  // + the abort word, + alignment
 }  // namespace lpdw
@@ -1353,7 +1358,7 @@ __global__ void __launch_bounds__(lpdw::THREADS, 1)
   if (tid == 0) {
     for (int i = 0; i < STAGES; i++) {
       bar_init(full(i), 1);
-      bar_init(empty(i), WARPS);
+      bar_init(empty(i), WARPS + 1);
     }
     *abort_w = 0;
     asm volatile("fence.mbarrier_init.release.cluster;");
@@ -1362,7 +1367,7 @@ __global__ void __launch_bounds__(lpdw::THREADS, 1)
   const int items = 2 * n, first = blockIdx.x * LP_WCPB, stride = gridDim.x * LP_WCPB;
   bool ok = true;
   int j = 0;  // half images so far
-  if (warp == WARPS) {
+  if (warp == WARPS + 1) {
     if (lane == 0) {
       for (int i0 = first; i0 < items && ok; i0 += stride)
         for (int it = i0; it < items && it < i0 + LP_WCPB; it++, j++) {
@@ -1377,16 +1382,28 @@ __global__ void __launch_bounds__(lpdw::THREADS, 1)
       for (int k = j > STAGES ? j - STAGES : 0; k < j; k++)
         mbar_wait(full(k % STAGES), (uint32_t)(k / STAGES) & 1u, LIMIT);
     }
-  } else {
-    const int ky = ROWS == 3 ? warp % 3 : (int)blockIdx.y, kx0 = ROWS == 3 ? 0 : warp % 3, cg = warp / 3;
-    // This lane's row of the 8 x 8 matrices a load takes: of dY (pixels 0-7 and
-    // 8-15, channel groups 0 and 1; 2 and 3 for co 16-31), of X (pixels 0-15 of
-    // group cg, at two kernel columns).
-    const int pa = (lane & 7) + ((lane >> 4) & 1) * 8, ca = (lane >> 3) & 1;
-    const int pb = (lane & 15) + kx0 + (ROWS == 3 ? lane >> 4 : 0) + ky * 34;
-    float bs[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+  } else if (warp == WARPS) {
     for (int i0 = first; i0 < items && ok; i0 += stride) {
-      float acc[KX][2][4] = {};
+      float sum = 0.f;
+      for (int it = i0; it < items && it < i0 + LP_WCPB; it++, j++) {
+        const int s = j % STAGES;
+        ok = __all_sync(FULL, wait(full(s), (uint32_t)(j / STAGES) & 1u, abort_w));
+        if (!ok) break;
+        db_chain(base + (uint32_t)(s * STAGE + X_SPACE), lane, sum);
+        __syncwarp();
+        if (lane == 0) arrive(empty(s));
+      }
+      if (ok && (ROWS == 3 || blockIdx.y == 0)) atomicAdd(db + lane, sum);
+    }
+  } else {
+    const int ky = ROWS == 3 ? warp % 3 : (int)blockIdx.y, kx0 = ROWS == 3 ? 0 : warp % 3, ch = warp / 3;
+    // This lane's row of the 8 x 8 matrices a load takes: of dY (pixels 0-7 and
+    // 8-15, channel groups 0 and 1; 2 and 3 for co 16-31), of X (the same pixels,
+    // groups 2 ch and 2 ch + 1).
+    const int pa = (lane & 7) + ((lane >> 4) & 1) * 8, ca = (lane >> 3) & 1;
+    const int pb = (lane & 15) + kx0 + ky * 34, cb = 2 * ch + (lane >> 4);
+    for (int i0 = first; i0 < items && ok; i0 += stride) {
+      float acc[KX][2][2][4] = {};  // [kernel column][8 ci][16 co][fragment]
       for (int it = i0; it < items && it < i0 + LP_WCPB; it++, j++) {
         const int s = j % STAGES;
         ok = __all_sync(FULL, wait(full(s), (uint32_t)(j / STAGES) & 1u, abort_w));
@@ -1396,32 +1413,27 @@ __global__ void __launch_bounds__(lpdw::THREADS, 1)
         // % 2) on. The swizzle depends on that row's place in four (a 34-pixel
         // pitch): four base addresses, the rest is immediate. The next step's
         // fragments load while this one's MMAs run.
-        uint32_t xb[4];
+        uint32_t xb[KX == 3 ? 2 : 1][4];  // kernel columns 0 and 1; 2 is two pixels on
 #pragma unroll
-        for (int r = 0; r < 4; r++)
-          xb[r] = xs + (uint32_t)(pb * 64 + (((cg ^ (r + (pb >> 1))) & 3) << 4));
+        for (int x = 0; x < (KX == 3 ? 2 : 1); x++)
+#pragma unroll
+          for (int r = 0; r < 4; r++)
+            xb[x][r] = xs + (uint32_t)((pb + x) * 64 + (((cb ^ (r + ((pb + x) >> 1))) & 3) << 4));
         uint32_t aa = ds + swz(pa, ca), ab = aa ^ 32u;
-        uint32_t a[2][2][4], b[2][3][2];
+        uint32_t a[2][2][4], b[2][KX][4];
         auto load = [&](int i) {
           const int u = i & 1, r = i >> 1, q = (r * 34 + (i & 1) * 16) * 64;
           ldsm4t(aa + i * 1024, a[u][0]);
           ldsm4t(ab + i * 1024, a[u][1]);
-          if (ROWS == 3) {
-            uint32_t f[4];
-            ldsm4t(xb[r & 3] + q, f);
-            ldsm2t(xb[(r + 1) & 3] + q + 128, b[u][2]);
-            b[u][0][0] = f[0];
-            b[u][0][1] = f[1];
-            b[u][1][0] = f[2];
-            b[u][1][1] = f[3];
-          } else {
-            ldsm2t(xb[r & 3] + q, b[u][0]);
+          ldsm4t(xb[0][r & 3] + q, b[u][0]);
+          if (KX == 3) {
+            ldsm4t(xb[KX == 3 ? 1 : 0][r & 3] + q, b[u][KX / 2]);
+            ldsm4t(xb[0][(r + 1) & 3] + q + 128, b[u][KX - 1]);
           }
         };
         load(0);
 #pragma unroll 1
         for (int o = 0; o < 4; o++) {
-          const bool sums = cg == o;  // db: each warp takes a twelfth of the pixels
 #pragma unroll
           for (int i = 0; i < 8; i++) {
             const int u = i & 1;
@@ -1432,21 +1444,16 @@ __global__ void __launch_bounds__(lpdw::THREADS, 1)
               aa += 8 * 1024;
               ab += 8 * 1024;
 #pragma unroll
-              for (int r = 0; r < 4; r++) xb[r] += 4 * 34 * 64;
+              for (int r = 0; r < (KX == 3 ? 8 : 4); r++) xb[r >> 2][r & 3] += 4 * 34 * 64;
               load(0);
             }
 #pragma unroll
             for (int m = 0; m < 2; m++)
 #pragma unroll
-              for (int x = 0; x < KX; x++) mma_bf16(acc[x][m], a[u][m], b[u][x]);
-            if (sums && i % 3 == warp % 3) {
-#pragma unroll
-              for (int m = 0; m < 2; m++)
-#pragma unroll
-                for (int e = 0; e < 2; e++)
-                  bs[m][e] +=
-                      (bf_lo(a[u][m][e]) + bf_hi(a[u][m][e])) + (bf_lo(a[u][m][e + 2]) + bf_hi(a[u][m][e + 2]));
-            }
+              for (int x = 0; x < KX; x++) {
+                mma_bf16(acc[x][0][m], a[u][m], {b[u][x][0], b[u][x][1]});
+                mma_bf16(acc[x][1][m], a[u][m], {b[u][x][2], b[u][x][3]});
+              }
           }
         }
         __syncwarp();
@@ -1454,24 +1461,11 @@ __global__ void __launch_bounds__(lpdw::THREADS, 1)
       }
       if (!ok) break;
 #pragma unroll
-      for (int x = 0; x < KX; x++)
-#pragma unroll
-        for (int m = 0; m < 2; m++)
-#pragma unroll
-          for (int f = 0; f < 4; f++)
-            atomicAdd(dW + (m * 16 + g + 8 * (f >> 1)) * 288 + (ky * 3 + kx0 + x) * 32 + cg * 8 + 2 * t + (f & 1),
-                      acc[x][m][f]);
-    }
-    if (ok && (ROWS == 3 || blockIdx.y == 0)) {
-#pragma unroll
-      for (int m = 0; m < 2; m++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          float v = bs[m][e];
-          v += __shfl_xor_sync(FULL, v, 1);
-          v += __shfl_xor_sync(FULL, v, 2);
-          if (t == 0) atomicAdd(db + m * 16 + 8 * e + g, v);
-        }
+      for (int q = 0; q < KX * 16; q++) {
+        const int x = q >> 4, i = (q >> 3) & 1, m = (q >> 2) & 1, f = q & 3;
+        atomicAdd(dW + (m * 16 + g + 8 * (f >> 1)) * 288 + (ky * 3 + kx0 + x) * 32 + ch * 16 + i * 8 + 2 * t + (f & 1),
+                  acc[x][i][m][f]);
+      }
     }
   }
   if (!ok) {
@@ -1496,10 +1490,12 @@ constexpr int OFF_BAR = STAGES * STAGE;
 constexpr int SMEM = OFF_BAR + 2 * STAGES * 8 + 8 + 512;
 template <int C>
 constexpr int WARPS_OF = 2 * ((9 * C + 7) / 8);  // 16 x 8 tiles of dW
+template <int C>
+constexpr int THREADS_OF = 32 * (WARPS_OF<C> + C);  // + loads, + db (C = 2)
 }  // namespace lpdws
 
 template <int C>
-__global__ void __launch_bounds__(32 * lpdws::WARPS_OF<C> + 32, 2)
+__global__ void __launch_bounds__(lpdws::THREADS_OF<C>, 2)
     lp_conv_bwd_w_edge_kernel(const __grid_constant__ CUtensorMap tm32, const __grid_constant__ CUtensorMap tms, int n,
                               float* dW, float* db, uint32_t* status) {
   using namespace lptrain;
@@ -1516,7 +1512,7 @@ __global__ void __launch_bounds__(32 * lpdws::WARPS_OF<C> + 32, 2)
   if (tid == 0) {
     for (int i = 0; i < STAGES; i++) {
       bar_init(full(i), 1);
-      bar_init(empty(i), WARPS);
+      bar_init(empty(i), C == 2 ? WARPS + 1 : WARPS);
     }
     *abort_w = 0;
     asm volatile("fence.mbarrier_init.release.cluster;");
@@ -1539,13 +1535,26 @@ __global__ void __launch_bounds__(32 * lpdws::WARPS_OF<C> + 32, 2)
       for (int k = j > STAGES ? j - STAGES : 0; k < j; k++)
         mbar_wait(full(k % STAGES), (uint32_t)(k / STAGES) & 1u, LIMIT);
     }
+  } else if (C == 2 && warp == WARPS + 1) {
+    for (int i0 = first; i0 < items && ok; i0 += stride) {
+      float sum = 0.f;
+      for (int it = i0; it < items && it < i0 + LP_WCPB; it++, j++) {
+        const int s = j % STAGES;
+        ok = __all_sync(FULL, wait(full(s), (uint32_t)(j / STAGES) & 1u, abort_w));
+        if (!ok) break;
+        db_chain(base + (uint32_t)(s * STAGE), lane, sum);
+        __syncwarp();
+        if (lane == 0) arrive(empty(s));
+      }
+      if (ok) atomicAdd(db + lane, sum);
+    }
   } else {
     const int m = warp & 1, i = warp >> 1;  // 16 channels, 8 columns
     const int pa = (lane & 7) + ((lane >> 4) & 1) * 8, ca = ((lane >> 3) & 1) + 2 * m;
     // This lane's column's element at pixel 2 t of a row's first 16.
     const int nn = i * 8 + g < N ? i * 8 + g : 0, tap = nn / C;
     const int nb = (1 + S * (tap / 3 - 1)) * RP + 8 + (2 * t + S * (tap % 3 - 1)) * C + nn % C;
-    float bs[2] = {0.f, 0.f};
+    float bs = 0.f;  // C = 1: db
     for (int i0 = first; i0 < items && ok; i0 += stride) {
       float acc[4] = {};
       for (int it = i0; it < items && it < i0 + LP_WCPB; it++, j++) {
@@ -1575,14 +1584,8 @@ __global__ void __launch_bounds__(32 * lpdws::WARPS_OF<C> + 32, 2)
           for (int w = 0; w < 4; w++) {
             mma_bf16(acc, a[u][w], b[u][w]);
             const int k = v * 4 + w;
-            if (C == 2) {
-              if (i == w % 3)
-#pragma unroll
-                for (int h = 0; h < 2; h++)
-                  bs[h] += (bf_lo(a[u][w][h]) + bf_hi(a[u][w][h])) + (bf_lo(a[u][w][h + 2]) + bf_hi(a[u][w][h + 2]));
-            } else if (lane < 16 && warp == w) {
-              bs[0] += __uint_as_float((uint32_t)small[((k >> 1) + 1) * RP + 8 + (k & 1) * 16 + lane] << 16);
-            }
+            if (C == 1 && lane < 16 && warp == w)
+              bs += __uint_as_float((uint32_t)small[((k >> 1) + 1) * RP + 8 + (k & 1) * 16 + lane] << 16);
           }
         }
         __syncwarp();
@@ -1595,14 +1598,10 @@ __global__ void __launch_bounds__(32 * lpdws::WARPS_OF<C> + 32, 2)
         if (c < N) atomicAdd(dW + (C == 2 ? ch * N + c : c * 32 + ch), acc[f]);
       }
     }
-    if (ok) {
+    if (C == 1 && ok) {
 #pragma unroll
-      for (int h = 0; h < (C == 2 ? 2 : 1); h++) {
-        float v = bs[h];
-#pragma unroll
-        for (int o = 1; o < (C == 2 ? 4 : 32); o <<= 1) v += __shfl_xor_sync(FULL, v, o);
-        if (C == 2 ? t == 0 : lane == 0) atomicAdd(db + (C == 2 ? m * 16 + 8 * h + g : 0), v);
-      }
+      for (int o = 1; o < 32; o <<= 1) bs += __shfl_xor_sync(FULL, bs, o);
+      if (lane == 0) atomicAdd(db, bs);
     }
   }
   if (!ok) {
@@ -1685,9 +1684,10 @@ __global__ void __launch_bounds__(256) lp_conv_first_kernel(const uint16_t* X, c
   }
 }
 
-// The gradient of the last layer's input, 1 -> 32: K = the 9 taps of dY around a
-// pixel (one K = 16 step a tile), masked by the ReLU of X; weights in registers
-// in lp_conv_first_kernel's column order. Bound by reading X and writing dX.
+// The gradient of the last layer's input, 1 -> 32: one K = 8 step a tap (its first
+// column is dY's pixel), the sums growing tap by tap as the element-wise kernel's;
+// masked by the ReLU of X; weights in registers in lp_conv_first_kernel's column
+// order. Bound by reading X and writing dX.
 __global__ void __launch_bounds__(256) lp_conv_bwd_last_kernel(const uint16_t* dY, const uint16_t* W,
                                                                const uint16_t* Xa, uint16_t* dX) {
   using lptrain::relu_mask;
@@ -1705,18 +1705,14 @@ __global__ void __launch_bounds__(256) lp_conv_bwd_last_kernel(const uint16_t* d
     const int p = 2 * (tid + 256 * i);
     *reinterpret_cast<uint32_t*>(&ys[((p >> 5) + 1) * RP + 4 + (p & 31)]) = v[i];
   }
-  uint32_t b[4][2];
+  uint32_t b[4][9];
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const uint16_t* w = W + 8 * (g >> 1) + 2 * j + (g & 1);
-    b[j][0] = pack_raw(w[2 * t * 32], w[(2 * t + 1) * 32]);
-    b[j][1] = t == 0 ? (uint32_t)w[8 * 32] : 0u;
-  }
-  // dY at p - off(tap).
-  auto off = [&](int tap) { return (2 - tap / 3) * RP + 2 - tap % 3 + 3; };
-  const int o0 = off(2 * t), o1 = off(2 * t + 1), o2 = off(8);
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int tap = 0; tap < 9; tap++)
+      b[j][tap] = t == 0 ? (uint32_t)W[tap * 32 + 8 * (g >> 1) + 2 * j + (g & 1)] : 0u;
   __syncthreads();
-#pragma unroll 4
+#pragma unroll 2
   for (int u = 0; u < 8; u++) {
     const int tile = warp * 8 + u, y = tile >> 1, xb = (tile & 1) * 16;
     const size_t at = (img * LP_P + y * 32 + xb + g) * 32 + 8 * t;
@@ -1725,14 +1721,15 @@ __global__ void __launch_bounds__(256) lp_conv_bwd_last_kernel(const uint16_t* d
       xm[0] = *reinterpret_cast<const uint4*>(Xa + at);
       xm[1] = *reinterpret_cast<const uint4*>(Xa + at + 8 * 32);
     }
-    const uint16_t* r = ys + y * RP + xb + g;
-    const uint32_t a[4] = {pack_raw(r[o0], r[o1]), pack_raw(r[8 + o0], r[8 + o1]), t == 0 ? (uint32_t)r[o2] : 0u,
-                           t == 0 ? (uint32_t)r[8 + o2] : 0u};
-    float d[4][4];
+    // dY at p - off(tap).
+    const uint16_t* r = ys + y * RP + xb + g + 3;
+    float d[4][4] = {};
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.f;
-      mma_bf16(d[j], a, b[j]);
+    for (int tap = 0; tap < 9; tap++) {
+      const uint16_t* q = r + (2 - tap / 3) * RP + 2 - tap % 3;
+      const uint32_t a0 = t == 0 ? (uint32_t)q[0] : 0u, a1 = t == 0 ? (uint32_t)q[8] : 0u;
+#pragma unroll
+      for (int j = 0; j < 4; j++) mma_bf16_k8(d[j], a0, a1, b[j][tap]);
     }
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -1750,16 +1747,16 @@ __global__ void __launch_bounds__(256) lp_conv_bwd_last_kernel(const uint16_t* d
   }
 }
 
-// The last layer, 32 -> 1: z[p][tap] = X[p] . W[tap], a contraction of K = 32
-// with the taps as N (4 MMAs a tile of 16 pixels, the weights in registers), then
-// y[p] = sum over taps of z[p + off(tap)][tap] + bias from shared memory. Half an
-// image a stage by TMA; bound by reading X.
+// The last layer, 32 -> 1: an implicit GEMM over a staged image with its halo,
+// one column of N = 8 in use, A through ldmatrix. The sums grow tap by tap and
+// channel half by half as in lp_conv_fwd_smem_kernel, so the scores are the same
+// bits. (A contraction with the taps as N takes 4 MMAs a tile instead of 18 and the
+// same time, 25 us at 2048 images, but scores 3e-7 away, which the softmax's
+// BF16 gradient passes on.) Bound by reading X.
 namespace lplast {
-constexpr int STAGES = 4, WARPS = 8, THREADS = (WARPS + 1) * 32, ZP = 34;  // z row pitch with its halo
-constexpr int OFF_Z = STAGES * lptrain::HALF_BYTES;
-constexpr int OFF_BAR = OFF_Z + 9 * 34 * ZP * 4;
+constexpr int SPACE = (34 * 34 * 64 + 511) / 512 * 512, STAGES = 3, WARPS = 8, THREADS = (WARPS + 1) * 32;
+constexpr int OFF_BAR = STAGES * SPACE;
 constexpr int SMEM = OFF_BAR + 2 * STAGES * 8 + 8 + 512;
-static_assert(OFF_BAR % 8 == 0, "barrier alignment");
 }  // namespace lplast
 
 __global__ void __launch_bounds__(lplast::THREADS, 1)
@@ -1771,7 +1768,6 @@ __global__ void __launch_bounds__(lplast::THREADS, 1)
   uint8_t* sm = sm_raw + ((512u - ((uint32_t)__cvta_generic_to_shared(sm_raw) & 511u)) & 511u);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
-  float* z = reinterpret_cast<float*>(sm + OFF_Z);  // [9][34][34]
   auto full = [&](int i) { return base + (uint32_t)(OFF_BAR + 8 * i); };
   auto empty = [&](int i) { return base + (uint32_t)(OFF_BAR + 8 * (STAGES + i)); };
   volatile uint32_t* abort_w = reinterpret_cast<volatile uint32_t*>(sm + OFF_BAR + 16 * STAGES);
@@ -1783,84 +1779,67 @@ __global__ void __launch_bounds__(lplast::THREADS, 1)
     *abort_w = 0;
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
-  for (int q = tid; q < 9 * 34 * ZP; q += THREADS) z[q] = 0.f;
   __syncthreads();
   const int first = blockIdx.x, stride = gridDim.x;
   bool ok = true;
+  int j = 0;
   if (warp == WARPS) {
     if (lane == 0) {
-      int j = 0;
-      for (int img = first; img < n && ok; img += stride)
-        for (int h = 0; h < 2; h++, j++) {
-          const int s = j % STAGES;
-          if (j >= STAGES) ok = wait(empty(s), (uint32_t)(j / STAGES - 1) & 1u, abort_w);
-          if (!ok) break;
-          expect(full(s), HALF_BYTES);
-          tma4(base + (uint32_t)(s * HALF_BYTES), &tmx, 0, 0, h * 16, img, full(s));
-        }
+      for (int img = first; img < n; img += stride, j++) {
+        const int s = j % STAGES;
+        if (j >= STAGES) ok = wait(empty(s), (uint32_t)(j / STAGES - 1) & 1u, abort_w);
+        if (!ok) break;
+        expect(full(s), 34 * 34 * 64);
+        tma4(base + (uint32_t)(s * SPACE), &tmx, 0, -1, -1, img, full(s));
+      }
       for (int k = j > STAGES ? j - STAGES : 0; k < j; k++)
         mbar_wait(full(k % STAGES), (uint32_t)(k / STAGES) & 1u, LIMIT);
     }
   } else {
     const int pa = (lane & 7) + ((lane >> 3) & 1) * 8, ca = (lane >> 4) & 1;
-    uint32_t b[2][2][2];  // [16 channels][8 taps][fragment]
+    uint32_t b[18][2];  // [tap, 16 channels][fragment]: column 0 only
 #pragma unroll
-    for (int k = 0; k < 2; k++)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int tap = i * 8 + g;
-        const uint16_t* w = W + (tap < 9 ? tap : 0) * 32 + k * 16 + 2 * t;
-        b[k][i][0] = tap < 9 ? pack_raw(w[0], w[1]) : 0u;
-        b[k][i][1] = tap < 9 ? pack_raw(w[8], w[9]) : 0u;
-      }
+    for (int k = 0; k < 18; k++) {
+      const uint16_t* w = W + k * 16 + 2 * t;
+      b[k][0] = g == 0 ? pack_raw(w[0], w[1]) : 0u;
+      b[k][1] = g == 0 ? pack_raw(w[8], w[9]) : 0u;
+    }
     const float bv = bias[0];
-    int j = 0;
-    for (int img = first; img < n && ok; img += stride) {
-      for (int h = 0; h < 2; h++, j++) {
-        const int s = j % STAGES;
-        ok = __all_sync(FULL, wait(full(s), (uint32_t)(j / STAGES) & 1u, abort_w));
-        if (!ok) break;
-        const uint32_t xs = base + (uint32_t)(s * HALF_BYTES);
+    for (int img = first; img < n; img += stride, j++) {
+      const int s = j % STAGES;
+      ok = __all_sync(FULL, wait(full(s), (uint32_t)(j / STAGES) & 1u, abort_w));
+      if (!ok) break;
+      const uint32_t xs = base + (uint32_t)(s * SPACE);
+#pragma unroll 1
+      for (int h = 0; h < 2; h++) {
+        // Four tiles of 16 pixels: rows 4 warp + 2 h and the next.
+        const int y = 4 * warp + 2 * h;
+        float d[4][4] = {};
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int y = 2 * warp + (u >> 1), xb = (u & 1) * 16;
-          uint32_t a[2][4];
-          const uint32_t aa = xs + swz(y * 32 + xb + pa, ca);
-          ldsm4(aa, a[0]);
-          ldsm4(aa ^ 32u, a[1]);
-          float d[2][4] = {};
+        for (int tap = 0; tap < 9; tap++) {
 #pragma unroll
-          for (int i = 0; i < 2; i++) {
-            mma_bf16(d[i], a[0], b[0][i]);
-            mma_bf16(d[i], a[1], b[1][i]);
-          }
-          float* zr = z + (h * 16 + y + 1) * ZP + xb + 1 + g;
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            zr[(2 * t + e) * 34 * ZP] = d[0][e];
-            zr[(2 * t + e) * 34 * ZP + 8] = d[0][2 + e];
-          }
-          if (t == 0) {
-            zr[8 * 34 * ZP] = d[1][0];
-            zr[8 * 34 * ZP + 8] = d[1][2];
+          for (int u = 0; u < 4; u++) {
+            const int p = (y + (u >> 1) + tap / 3) * 34 + (u & 1) * 16 + tap % 3 + pa;
+            const uint32_t aa = xs + swz(p, ca);
+            uint32_t a[2][4];
+            ldsm4(aa, a[0]);
+            ldsm4(aa ^ 32u, a[1]);
+            mma_bf16(d[u], a[0], b[2 * tap]);
+            mma_bf16(d[u], a[1], b[2 * tap + 1]);
           }
         }
-        __syncwarp();
-        if (lane == 0) arrive(empty(s));
-      }
-      ok = !lpnet::epi_or(!ok);  // the eight warps leave together
-      if (!ok) break;
+        if (t == 0) {
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int p = tid + 256 * i;
-        const float* zr = z + (p >> 5) * ZP + (p & 31);
-        float v = 0.f;
+          for (int u = 0; u < 4; u++)
 #pragma unroll
-        for (int tap = 0; tap < 9; tap++) v += zr[(tap * 34 + tap / 3) * ZP + tap % 3];
-        v += bv;
-        Y[(size_t)img * LP_P + p] = relu ? fmaxf(v, 0.f) : v;
+            for (int e = 0; e < 2; e++) {
+              const float v = d[u][2 * e] + bv;
+              Y[(size_t)img * LP_P + (y + (u >> 1)) * 32 + (u & 1) * 16 + g + 8 * e] = relu ? fmaxf(v, 0.f) : v;
+            }
+        }
       }
-      lpnet::epi_sync();
+      __syncwarp();
+      if (lane == 0) arrive(empty(s));
     }
   }
   if (!ok) {
@@ -1951,7 +1930,7 @@ vp8a_status conv_tc(vp8a_ctx* ctx, const uint16_t* a, const uint16_t* W, const f
 vp8a_status conv_last(vp8a_ctx* ctx, const uint16_t* X, const uint16_t* W, const float* bias, int n, int relu,
                       float* Y) {
   CUtensorMap tm;
-  vp8a_status s = image_map(X, (uint32_t)n, 32, 32, 16, &tm);
+  vp8a_status s = image_map(X, (uint32_t)n, 32, 34, 34, &tm);
   if (s == VP8A_OK) s = use_smem(lp_conv_last_kernel, lplast::SMEM);
   if (s != VP8A_OK) return s;
   lp_conv_last_kernel<<<std::min(n, ctx->sm_count), lplast::THREADS, lplast::SMEM, ctx->stream>>>(
@@ -1989,7 +1968,7 @@ vp8a_status conv_bwd_w_edge(vp8a_ctx* ctx, const uint16_t* t32, const uint16_t* 
   if (s == VP8A_OK) s = use_smem(lp_conv_bwd_w_edge_kernel<C>, lpdws::SMEM);
   if (s != VP8A_OK) return s;
   lp_conv_bwd_w_edge_kernel<C>
-      <<<std::min(groups, 2 * ctx->sm_count), 32 * lpdws::WARPS_OF<C> + 32, lpdws::SMEM, ctx->stream>>>(tm, tms, n, dW, db,
+      <<<std::min(groups, 2 * ctx->sm_count), lpdws::THREADS_OF<C>, lpdws::SMEM, ctx->stream>>>(tm, tms, n, dW, db,
                                                                                                 ctx->d_status);
   VP8A_CUDA(cudaGetLastError());
   ctx->launches++;

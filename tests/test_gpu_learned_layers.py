@@ -75,3 +75,30 @@ def test_layers_match_64_bit_convolutions(ctx, n, cin, cout, offset):
     assert bool(((gx.double() - dx).abs() <= SUM * sx + HALF * dx.abs()).all())
     assert bool(((gw.double().view(dw.shape) - 2 * dw).abs() <= 2 * SUM * sw).all())
     assert bool(((gb.double() - 2 * db).abs() <= 2 * SUM * sb).all())
+
+
+@pytest.mark.parametrize("n", [1, 3, 8])
+@pytest.mark.parametrize("cin,cout", [(2, 32), (32, 32), (32, 1)])
+def test_both_routes_round_alike(ctx, n, cin, cout):
+    # Up to 8 images are one FP32 chain: aligned and unaligned tensors then give
+    # the same bits (but for dW and db of the last layer, whose chain runs over the
+    # other tensor's pixels).
+    g = torch.Generator(device="cuda").manual_seed(n + cin)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g)  # noqa: E731
+    x, w = rnd(n, 32, 32, cin).bfloat16(), (rnd(cout, 9, cin) * 0.2).bfloat16()
+    b, dy, lib, last = rnd(cout), (rnd(n, 32, 32, cout) * 0.05).bfloat16(), ctx._lib, cout == 1
+    got = []
+    for offset in (0, 2):
+        xs, dys = shifted(x, offset), shifted(dy, offset)
+        y = shifted(torch.zeros((n, 32, 32, cout), dtype=torch.float32 if last else torch.bfloat16, device="cuda"), offset)
+        gx, gw, gb = shifted(torch.zeros_like(x), offset), torch.zeros(cout * 9 * cin, device="cuda"), torch.zeros(
+            cout, device="cuda")
+        torch.cuda.synchronize()
+        if cin != 32 or last:
+            assert lib.vp8a_lp_conv_forward(ctx.handle, xs.data_ptr(), cin, w.data_ptr(), b.data_ptr(), cout, n, 1,
+                                            None if last else y.data_ptr(), y.data_ptr() if last else None) == abi.OK
+        assert lib.vp8a_lp_conv_backward(ctx.handle, xs.data_ptr(), cin, w.data_ptr(), cout, n, dys.data_ptr(), 1,
+                                         gx.data_ptr(), gw.data_ptr(), gb.data_ptr()) == abi.OK
+        ctx.synchronize()
+        got.append((y, *(() if cin == 2 else (gx,)), *(() if last else (gw, gb))))
+    assert all(torch.equal(p, q) for p, q in zip(*got))
