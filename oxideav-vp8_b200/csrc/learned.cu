@@ -1004,7 +1004,7 @@ __global__ void __launch_bounds__(lpnet::THREADS, 1) lp_net_kernel(const uint16_
 // Measured at 2048 images, us a launch, with the element-wise kernels and a
 // one-image-a-CTA tcgen05 forward, then with these: 2 -> 32 forward 87 -> 55, 32 ->
 // 32 forward 129 -> 73, dX 943 -> 86, dW 1397 -> 126, 32 -> 1 forward 115 -> 39, dX
-// 153 -> 57, dW 954 -> 28, dW of 2 -> 32 549 -> 75; the training step 6.85 -> 0.90 ms.
+// 153 -> 57, dW 954 -> 28, dW of 2 -> 32 549 -> 69; the training step 6.85 -> 0.89 ms.
 namespace lptrain {
 using lpnet::arrive;
 using lpnet::mma;
@@ -1076,22 +1076,22 @@ __device__ __forceinline__ void db_chain(uint32_t tile, int lane, float& sum) {
   uint32_t at[4];
 #pragma unroll
   for (int r = 0; r < 4; r++) at[r] = tile + (uint32_t)((((lane >> 3) ^ r) & 3) << 4) + (lane & 7) * 2;
-  uint32_t v[2][16];
-  auto load = [&](int p, uint32_t (&to)[16]) {
-#pragma unroll
-    for (int i = 0; i < 16; i++)
-      asm volatile("ld.shared.u16 %0, [%1];" : "=r"(to[i]) : "r"(at[(i >> 1) & 3] + (uint32_t)(p + i) * 64));
+  // Each addition sits between the loads of the pixels 32 on.
+  uint32_t v[32];
+  auto load = [&](int p, int i) {
+    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v[i]) : "r"(at[(i >> 1) & 3] + (uint32_t)(p + i) * 64));
   };
-  load(0, v[0]);
+#pragma unroll
+  for (int i = 0; i < 32; i++) load(0, i);
 #pragma unroll 1
-  for (int p = 0; p < 512; p += 32) {
-    load(p + 16, v[1]);
+  for (int p = 32; p < 512; p += 32)
 #pragma unroll
-    for (int i = 0; i < 16; i++) sum += __uint_as_float(v[0][i] << 16);
-    if (p + 32 < 512) load(p + 32, v[0]);
+    for (int i = 0; i < 32; i++) {
+      sum += __uint_as_float(v[i] << 16);
+      load(p, i);
+    }
 #pragma unroll
-    for (int i = 0; i < 16; i++) sum += __uint_as_float(v[1][i] << 16);
-  }
+  for (int i = 0; i < 32; i++) sum += __uint_as_float(v[i] << 16);
 }
 }  // namespace lptrain
 
