@@ -983,6 +983,8 @@ struct Feed {
   alignas(16) MbInfoDev left, none;
   uint64_t dec_bar[DEC_RING], in_bar[2];
   int stop;  // the helper met a wait that ran out
+  // For leaving: MBs whose decisions every CTA has sent, and the helper's count.
+  unsigned sent[MAX_REFS], n_pub;
 };
 static_assert(offsetof(Feed, src) % 16 == 0 && offsetof(Feed, above) % 16 == 0, "Feed alignment");
 
@@ -1063,7 +1065,8 @@ __device__ void run_helper(Feed& F, const AnArgs& a0, const AnArgs* jobs, const 
   unsigned n_pre = 0, n_pub = 0;
   unsigned long long polls = 0;
   unsigned idle = 0;
-  while (pub.job) {
+  bool stop = false;
+  while (pub.job && !stop) {
     bool moved = false;
     // MB n_pub decided everywhere?
     if (__all_sync(FULL, bar_done(&F.dec_bar[n_pub % DEC_RING], n_pub / DEC_RING & 1u))) {
@@ -1132,11 +1135,33 @@ __device__ void run_helper(Feed& F, const AnArgs& a0, const AnArgs* jobs, const 
       }
     }
     if (!moved) {
-      if ((++idle & 15u) == 0 && __any_sync(FULL, *(volatile unsigned*)pub.job->status != 0u)) {
-        if (lane == 0) *(volatile int*)&F.stop = 1;
-        return;
-      }
+      stop = (++idle & 15u) == 0 && __any_sync(FULL, *(volatile unsigned*)pub.job->status != 0u);
+      if (stop && lane == 0) *(volatile int*)&F.stop = 1;
       __nanosleep(40);
+    }
+  }
+  if (lane == 0) F.n_pub = n_pub;
+}
+
+// Leaving. A cluster barrier does not order asynchronous stores, and a CTA's shared
+// memory must not go away under one. A cluster that took all its MBs has awaited
+// every decision (the helpers ended at the last). One that stops has not: so each
+// CTA tells the others how many MBs' decisions it has sent (plain stores, which the
+// barrier orders) and waits for what was sent to it. A decision that a CTA never
+// sent is taken off the phase by hand. MB m's decisions are sent only once every
+// helper has taken in MB m - 4's, so the phases are armed (tests/
+// test_cluster_leave.py runs this under random interleavings). One thread.
+__device__ __forceinline__ void await_decisions(Feed& F, int csize) {
+  unsigned most = 0;
+  for (int q = 0; q < csize; q++) most = max(most, F.sent[q]);
+  for (unsigned m = F.n_pub; m < most; m++) {
+    uint64_t* bar = &F.dec_bar[m % DEC_RING];
+    unsigned missing = 0;
+    for (int q = 0; q < csize; q++) missing += F.sent[q] <= m ? (unsigned)sizeof(RefDec) : 0u;
+    if (missing)
+      asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_at(bar)), "r"(missing)
+                   : "memory");
+    for (int polls = 0; polls < 1 << 20 && !bar_done(bar, m / DEC_RING & 1u); polls++) {
     }
   }
 }
@@ -1211,10 +1236,11 @@ __global__ void __launch_bounds__(AN_THREADS + 32, 2)
   if (warp == NW) {
     run_helper<BATCH>(feed, a0, jobs, items, n_it, cid, n_clusters, k, lane);
     __syncwarp();
-    cl.sync();  // no CTA leaves while another may write to it
+    cl.sync();
     return;
   }
-  for (int it = cid; it < n_it; it += n_clusters) {
+  bool stopped = false;
+  for (int it = cid; it < n_it && !stopped; it += n_clusters) {
     int r = it, job = 0;
     if (BATCH) {
       const uint32_t w = items[it];
@@ -1326,8 +1352,8 @@ __global__ void __launch_bounds__(AN_THREADS + 32, 2)
       }
       search_sync();
       if (s_stop) {
-        cl.sync();
-        return;
+        stopped = true;
+        break;
       }
       stage_ref(P, R, plan, mbx, mby, a.words, tid, AN_THREADS);
       search_sync();
@@ -1638,7 +1664,9 @@ __global__ void __launch_bounds__(AN_THREADS + 32, 2)
       }
     }
   }
-  cl.sync();  // no CTA leaves while another may write to it
+  if (tid < csize) *cl.map_shared_rank(&feed.sent[k], tid) = n;
+  cl.sync();
+  if (tid == 0) await_decisions(feed, csize);
 }
 
 }  // namespace
