@@ -880,13 +880,21 @@ __device__ __forceinline__ uint64_t run_pass(const LfArgs& a, const Limits* lim,
 // 900, and reads of a neighbour's memory are slow). Two messages are in flight
 // at most: message c is sent at column c + 1, after column c - 2's return has
 // been waited for.
+//
+// A wait that runs out closes the link for its eight lanes: they send and wait no
+// more, so the messages sent are the first so many of each link. Before the CTAs
+// leave, each tells its neighbours how many it has sent (a plain store, which the
+// cluster barrier orders; it does not order asynchronous ones) and waits for those
+// sent to it that it has not taken in (tests/test_cluster_leave.py runs this under
+// random interleavings).
 
 constexpr unsigned LINK_POLLS = 1u << 24;  // about a second; a message takes microseconds
 
 struct Link {
   alignas(16) uint8_t inbox[2][64];  // message c in entry c & 1
   uint64_t in_bar[2], ret_bar[2];
-  int dead;  // a wait ran out: no further waiting
+  unsigned sent_in, sent_ret;        // messages and returns sent to this CTA, told at the end
+  int dead;                          // a wait ran out: no further waiting
 };
 
 __device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -903,30 +911,42 @@ __device__ __forceinline__ void send8(uint32_t at, uint2 v, uint32_t bar) {
                "r"(v.x), "r"(v.y), "r"(bar)
                : "memory");
 }
-// False when the wait ran out (the pass then runs on without its neighbours).
-__device__ __forceinline__ bool wait_message(const LfArgs& a, Link* k, uint64_t* bar, int parity) {
-  const uint32_t at = smem_at(bar);
+__device__ __forceinline__ bool message_in(uint32_t bar, unsigned parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// Message (or return) m, by an MB's eight lanes; false for all of them when the wait
+// of one ran out (the pass then runs on without that neighbour).
+__device__ __forceinline__ bool wait_message(const LfArgs& a, Link* k, uint64_t* bars, int m) {
+  const uint32_t at = smem_at(bars + (m & 1));
   unsigned polls = 0;
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(at), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (*(volatile int*)&k->dead) return false;
+  bool in;
+  while (!(in = message_in(at, (unsigned)(m >> 1) & 1u))) {
+    if (*(volatile int*)&k->dead) break;
     if (++polls > LINK_POLLS) {
       *(volatile int*)&k->dead = 1;
       atomicCAS(a.status, 0u, (unsigned)vp8a::DEV_TIMEOUT);
-      return false;
+      break;
     }
   }
+  return __all_sync(((1u << LPM) - 1u) << (threadIdx.x & 31 & ~(LPM - 1)), in);
+}
+// The messages `got` .. `sent` - 1, on the way out: they arrive within microseconds.
+__device__ __forceinline__ void await_messages(uint64_t* bars, unsigned got, unsigned sent) {
+  for (; got < sent; got++)
+    for (int polls = 0; polls < 1 << 20 && !message_in(smem_at(bars + (got & 1)), got >> 1 & 1u); polls++) {
+    }
 }
 
 __device__ __forceinline__ void init_link(Link* k) {
   k->dead = 0;
+  k->sent_in = k->sent_ret = 0;
   for (int i = 0; i < 2; i++) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(&k->in_bar[i])) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(&k->ret_bar[i])) : "memory");
@@ -975,6 +995,10 @@ __device__ __forceinline__ uint64_t run_split(const LfArgs& a, const Limits* lim
   }
   uint64_t total = 0;
   LaneRows<LUMA> rec, src, fin;
+  // The links as this lane's MB serves them: open; messages sent down, returns taken
+  // in; messages taken in from above, each returned.
+  bool down = hand_down, up = handed;
+  unsigned n_down = 0, n_back = 0, n_up = 0;
   unsigned info = 0;
   int slot = 0;  // c % RING
   auto fetch = [&](int c) {
@@ -994,13 +1018,13 @@ __device__ __forceinline__ uint64_t run_split(const LfArgs& a, const Limits* lim
     const int left_at = (slot ? slot - 1 : RING - 1) * SLOT;
     const Limits L = lim[info & 63];
     const uint32_t kinner = sub ? L.flat : DISABLED;
-    bool linked = hand_down, written = false;
+    bool written = false;
     if (live && c >= RING) {
       // MB (r, c - RING) is final (its last rows back from the next CTA).
       const int f = c - RING;
-      if (hand_down) {
-        linked = wait_message(a, link, &link->ret_bar[f & 1], (f >> 1) & 1);
-        if (linked && q == 0) expect_message(&link->ret_bar[f & 1]);
+      if (down && (down = wait_message(a, link, link->ret_bar, f))) {
+        if (q == 0) expect_message(&link->ret_bar[f & 1]);
+        n_back++;
       }
       if (score) {
         total += f < whole_cols ? score_mb<LUMA>(me, q, src)
@@ -1019,29 +1043,38 @@ __device__ __forceinline__ uint64_t run_split(const LfArgs& a, const Limits* lim
       else vertical_edges<LUMA, SIMPLE, false>(rec, me, set + left_at, q, c > 0, L, kleft, kinner);
     }
     __syncwarp();
-    if (linked && c >= 1 && c <= cols)
+    if (down && c >= 1 && c <= cols) {
       send8(down_inbox + ((c - 1) & 1) * 64, *(const uint2*)(set + left_at + Geo<LUMA>::tail_off(q)),
             down_bar + ((c - 1) & 1) * 8);
+      n_down++;
+    }
     fetch(c + 1);
     if (written) store_rows<LUMA>(op + (c - RING) * ROWB, out.half, a.recon_align, fin);
     __syncthreads();
     if (main) {
       uint8_t* msg = link->inbox[c & 1];
-      linked = handed && wait_message(a, link, &link->in_bar[c & 1], (c >> 1) & 1);
-      uint8_t* up = handed ? msg + Geo<LUMA>::msg_col(q) : up_set + slot * SLOT + LAST + Geo<LUMA>::col_off(q);
+      if (up) up = wait_message(a, link, link->in_bar, c);
+      uint8_t* above = handed ? msg + Geo<LUMA>::msg_col(q) : up_set + slot * SLOT + LAST + Geo<LUMA>::col_off(q);
       const uint32_t ktop = top ? L.flat : DISABLED;
-      if (full) horizontal_edges<LUMA, SIMPLE, true>(me, up, q, top, L, ktop, kinner);
-      else horizontal_edges<LUMA, SIMPLE, false>(me, up, q, top, L, ktop, kinner);
+      if (full) horizontal_edges<LUMA, SIMPLE, true>(me, above, q, top, L, ktop, kinner);
+      else horizontal_edges<LUMA, SIMPLE, false>(me, above, q, top, L, ktop, kinner);
       if (handed) __syncwarp((1u << LPM) - 1u);
-      if (handed && linked) {
+      if (up) {
         const uint2 v = *(const uint2*)(msg + q * 8);
         if (q == 0) expect_message(&link->in_bar[c & 1]);
         send8(up_rings + slot * SLOT, v, up_bar + (c & 1) * 8);
+        n_up++;
       }
     }
     slot = c < 0 ? 0 : (slot == RING - 1 ? 0 : slot + 1);
     __syncthreads();
   }
+  cg::cluster_group cl = cg::this_cluster();
+  if (hand_down && q == 0) *cl.map_shared_rank(&link->sent_in, rank + 1) = n_down;
+  if (handed && q == 0) *cl.map_shared_rank(&link->sent_ret, rank - 1) = n_up;
+  cl.sync();
+  if (handed && q == 0) await_messages(link->in_bar, n_up, link->sent_in);
+  if (hand_down && q == 0) await_messages(link->ret_bar, n_back, link->sent_ret);
   return total;
 }
 
@@ -1109,8 +1142,6 @@ __device__ __forceinline__ void sweep_body(const LfArgs& a, int cta, int np) {
       PlanePass<false, SIMPLE, TILED> c(a, rings, q);
       v = run_pass<PRE>(a, lim, lim, taken, (int)blockIdx.x, c, none);
     }
-    // No CTA of a cluster leaves while another may write to it.
-    if constexpr (CL) cg::this_cluster().sync();
     if (!a.ssd_out) continue;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);

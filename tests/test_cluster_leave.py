@@ -7,7 +7,11 @@ and their ring depths, are read from their source.
 
 The analysis (csrc/analysis.cu): CTA k sends MB m's decision to every CTA onto the
 mbarrier m % ring, armed for one message a CTA; its helper takes the phases in
-order, arming each again, and prepares MB m while m < taken + 2."""
+order, arming each again, and prepares MB m while m < taken + 2.
+
+The split loop-filter pass (csrc/lf.cu): the CTA above sends column c's rows at
+column c + 1, once column c - 2's are back; the CTA below takes them in at column c
+and returns them. A wait that runs out closes its end of the link."""
 import os
 import random
 import re
@@ -124,3 +128,102 @@ def test_a_barrier_alone_is_not_enough():
     with pytest.raises(Violation):
         for seed in range(400):
             analysis(2, 12, 5, seed, False, 4)
+
+
+def split_pass(n_ctas, rows, cols, seed, awaits):
+    """CTA k holds `rows` rows; row s of all runs column t - s at step t."""
+    rnd = random.Random(seed)
+    patience = rnd.choice([0, 1, 3, 30])  # tries of a wait before it runs out
+    pace = rnd.choice([0.4, 0.1, 0.02])  # of the messages' arrival
+    depth = 3  # columns from an MB to the one that takes its slot
+    ins = [[Phases(1, 1) for _ in range(2)] for _ in range(n_ctas)]
+    rets = [[Phases(1, 1) for _ in range(2)] for _ in range(n_ctas)]
+    n_in, n_back, n_down = [0] * n_ctas, [0] * n_ctas, [0] * n_ctas
+    dead = [False] * n_ctas
+    flying = []
+    inside = set(range(n_ctas))
+
+    def land():
+        box, k, m = flying.pop(rnd.randrange(len(flying)))
+        if k not in inside:
+            raise Violation("a message arrived after its target had left")
+        assert box[k][m & 1].armed == m // 2 + 1, "a message ahead of its phase"
+        box[k][m & 1].add(m // 2)
+
+    def waits(box, k, m):
+        assert box[k][m & 1].armed == m // 2 + 1, "an unarmed phase is awaited"
+        tries = 0
+        while not box[k][m & 1].done(m // 2):
+            if dead[k]:
+                return False
+            tries += 1
+            if tries > patience:
+                dead[k] = True
+                return False
+            yield
+        return True
+
+    def cta(k):
+        up, down = k > 0, k + 1 < n_ctas
+        for t in range(n_ctas * rows + cols + depth):
+            c = t - (k + 1) * rows + 1  # the last row's column
+            if down and depth <= c < cols + depth:
+                down = yield from waits(rets, k, c - depth)
+                if down:
+                    rets[k][c - depth & 1].armed += 1
+                    n_back[k] += 1
+            if down and 1 <= c <= cols:
+                flying.append((ins, k + 1, c - 1))
+                n_down[k] += 1
+            yield
+            c = t - k * rows  # the first row's
+            if up and 0 <= c < cols:
+                up = yield from waits(ins, k, c)
+                if up:
+                    ins[k][c & 1].armed += 1
+                    flying.append((rets, k - 1, c))
+                    n_in[k] += 1
+            yield
+
+    agents = {k: cta(k) for k in range(n_ctas)}
+    while agents:
+        if flying and rnd.random() < pace:
+            land()
+        k = rnd.choice(sorted(agents))
+        if next(agents[k], 0) == 0:
+            del agents[k]
+    owed = {k: [(ins, m) for m in range(n_in[k], n_down[k - 1] if k else 0)] +
+               [(rets, m) for m in range(n_back[k], n_in[k + 1] if k + 1 < n_ctas else 0)] for k in range(n_ctas)}
+    step = 0
+    while inside:
+        step += 1
+        assert step < 100000, "a wait on the way out does not end"
+        if flying and rnd.random() < 0.5:
+            land()
+            continue
+        k = rnd.choice(sorted(inside))
+        assert all(box[k][m & 1].armed == m // 2 + 1 for box, m in owed[k]), "an unarmed phase is awaited"
+        if not awaits or all(box[k][m & 1].done(m // 2) for box, m in owed[k]):
+            inside.remove(k)
+    if flying:
+        raise Violation("a message was on its way when its target left")
+    return any(dead)
+
+
+def split_awaits():
+    text = source("lf.cu")
+    body = text[text.index("uint64_t run_split("):text.index("class_limits(")]
+    return body.count("await_messages(") == 2 and body.index("cl.sync();") < body.index("await_messages(")
+
+
+@pytest.mark.parametrize("n_ctas,rows", [(2, 1), (2, 3), (4, 1), (5, 2)])
+def test_split_pass_ctas_leave_after_their_messages(n_ctas, rows):
+    awaits = split_awaits()
+    gave_up = sum(split_pass(n_ctas, rows, 9, seed, awaits) for seed in range(400))
+    assert 0 < gave_up
+
+
+def test_a_barrier_alone_is_not_enough_for_a_split_pass():
+    with pytest.raises(Violation):
+        for seed in range(400):
+            split_pass(4, 1, 9, seed, False)
