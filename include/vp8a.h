@@ -260,12 +260,13 @@ vp8a_status vp8a_ctx_synchronize(vp8a_ctx* ctx);
 /* Kernel launches issued by this context since creation. */
 uint64_t vp8a_ctx_launch_count(const vp8a_ctx* ctx);
 /* No counterpart in the reference (its threads join instead of polling).
- * Sets how many times a wavefront wait of the inter analysis (an MB row
- * waiting for the row above it) may poll before it gives up: the call then
+ * Sets how many times a wait between CTAs may poll before it gives up: in
+ * the inter analysis an MB row's for the row above it, in a loop-filter pass
+ * split over several CTAs one's for its neighbour's rows. The call then
  * returns VP8A_E_DEVICE_TIMEOUT, every CTA leaves, and the context stays
  * usable. Default 2^24 polls (seconds). 0 gives up at the first poll that
- * finds the row above behind, which makes the timeout path testable without
- * hanging or faulting anything. Applies to calls issued after it. */
+ * finds nothing yet, which makes the timeout path testable without hanging
+ * or faulting anything. Applies to calls issued after it. */
 vp8a_status vp8a_ctx_set_wait_limit(vp8a_ctx* ctx, uint64_t polls);
 /* No counterpart in the reference (launch shapes of the device kernels).
  * The loop-filter sweep's launch shape follows rules on the picture's size
@@ -513,7 +514,16 @@ vp8a_status vp8a_build_arnr_altref(vp8a_ctx* ctx, const vp8a_i420* frames, uint3
 vp8a_status vp8a_build_arnr_altref_planes(vp8a_ctx* ctx, const vp8a_i420* frames, uint32_t n,
                                           uint32_t center, uint32_t strength, const vp8a_planes* out);
 
-/* ------------------------------------------------------- §15 loop filter */
+/* ------------------------------------------------------- §15 loop filter
+ *
+ * A pass over a picture may be split over several CTAs (by a rule on the
+ * picture's size and the number of candidates) whose waits for one another
+ * are bounded (vp8a_ctx_set_wait_limit). When one runs out, the calls below
+ * but vp8a_reconstruction_ssd and vp8a_filter_sweep_noalloc, whose passes are
+ * never split, return VP8A_E_DEVICE_TIMEOUT if any buffer was host memory;
+ * otherwise the next vp8a_ctx_synchronize returns it. The selection walks
+ * wait for their results and always return it themselves. The planes that
+ * vp8a_filter_frame was filtering and the tables are then not to be used. */
 
 /* filter_inter_frame_flags (src/loop_filter.rs:1364) / filter_frame_flags
  * (src/loop_filter.rs:2506) in place on `planes`. Key frames pass every MB

@@ -142,6 +142,7 @@ struct LfArgs {
   // segment overrides and deltas can still filter MBs at base level 0.
   int level0_unfiltered;
   unsigned* status;  // set to DEV_TIMEOUT when a wait between a split pass's CTAs runs out
+  unsigned long long spin_limit;  // polls of such a wait (about 60 ns each; a message takes microseconds)
 };
 
 __host__ __device__ __forceinline__ int clamp63(int v) { return v < 0 ? 0 : (v > 63 ? 63 : v); }
@@ -888,8 +889,6 @@ __device__ __forceinline__ uint64_t run_pass(const LfArgs& a, const Limits* lim,
 // sent to it that it has not taken in (tests/test_cluster_leave.py runs this under
 // random interleavings).
 
-constexpr unsigned LINK_POLLS = 1u << 24;  // about a second; a message takes microseconds
-
 struct Link {
   alignas(16) uint8_t inbox[2][64];  // message c in entry c & 1
   uint64_t in_bar[2], ret_bar[2];
@@ -925,11 +924,11 @@ __device__ __forceinline__ bool message_in(uint32_t bar, unsigned parity) {
 // of one ran out (the pass then runs on without that neighbour).
 __device__ __forceinline__ bool wait_message(const LfArgs& a, Link* k, uint64_t* bars, int m) {
   const uint32_t at = smem_at(bars + (m & 1));
-  unsigned polls = 0;
+  unsigned long long polls = 0;
   bool in;
   while (!(in = message_in(at, (unsigned)(m >> 1) & 1u))) {
     if (*(volatile int*)&k->dead) break;
-    if (++polls > LINK_POLLS) {
+    if (++polls > a.spin_limit) {
       *(volatile int*)&k->dead = 1;
       atomicCAS(a.status, 0u, (unsigned)vp8a::DEV_TIMEOUT);
       break;
@@ -1284,6 +1283,7 @@ vp8a_status stage_lf(vp8a_ctx* ctx, vp8a::Stager& st, const vp8a_planes* planes,
   a.mbs = (const vp8a_mb_lf_info*)d;
   a.base = *base;
   a.status = ctx->d_status;
+  a.spin_limit = ctx->wait_limit;
   if (src) {
     if (src->width == 0 || src->height == 0 || src->width > (uint32_t)cols * 16 ||
         src->height > (uint32_t)rows * 16) {

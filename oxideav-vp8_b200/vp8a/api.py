@@ -78,7 +78,8 @@ class Context:
         return tuple(int(x) for x in out)
 
     def set_wait_limit(self, polls):
-        """Poll budget of the analysis wavefront waits (default 2**24)."""
+        """Poll budget of the waits between CTAs: the analysis's wavefront and
+        the split loop-filter passes (default 2**24)."""
         check(self._lib.vp8a_ctx_set_wait_limit(self.handle, int(polls)), "vp8a_ctx_set_wait_limit")
 
 
