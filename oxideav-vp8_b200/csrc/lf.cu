@@ -1422,7 +1422,9 @@ vp8a_status launch_variant(vp8a_ctx* ctx, const Shape& S, unsigned grid, size_t 
   const auto one = lf_sweep_kernel<SIMPLE, CL, BOTH, PRE, TILED>;
   const auto many = lf_sweep_batch_kernel<SIMPLE, CL, BOTH, PRE, true>;
   const void* k = dj ? (const void*)many : (const void*)one;
-  VP8A_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // The kernel's limit, shared by every context's launches on the device: always the
+  // most that any takes, so that no thread lowers it between another's two calls.
+  VP8A_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_RING_BYTES));
   if (split > MAX_CLUSTER) VP8A_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
