@@ -266,7 +266,8 @@ uint64_t vp8a_ctx_launch_count(const vp8a_ctx* ctx);
  * returns VP8A_E_DEVICE_TIMEOUT, every CTA leaves, and the context stays
  * usable. Default 2^24 polls (seconds). 0 gives up at the first poll that
  * finds nothing yet, which makes the timeout path testable without hanging
- * or faulting anything. Applies to calls issued after it. */
+ * or faulting anything. (A loop-filter pass counts all waits of a CTA
+ * together, by the 1024 polls.) Applies to calls issued after it. */
 vp8a_status vp8a_ctx_set_wait_limit(vp8a_ctx* ctx, uint64_t polls);
 /* No counterpart in the reference (launch shapes of the device kernels).
  * The loop-filter sweep's launch shape follows rules on the picture's size

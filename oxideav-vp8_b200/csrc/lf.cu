@@ -141,8 +141,8 @@ struct LfArgs {
   // mode runs the pass with the base level as given, since per-MB
   // segment overrides and deltas can still filter MBs at base level 0.
   int level0_unfiltered;
-  unsigned* status;  // set to DEV_TIMEOUT when a wait between a split pass's CTAs runs out
-  unsigned long long spin_limit;  // polls of such a wait (about 60 ns each; a message takes microseconds)
+  unsigned spin_limit;  // polls of the waits between a split pass's CTAs (microseconds each message)
+  unsigned* status;     // set to DEV_TIMEOUT when they run out
 };
 
 __host__ __device__ __forceinline__ int clamp63(int v) { return v < 0 ? 0 : (v > 63 ? 63 : v); }
@@ -882,19 +882,21 @@ __device__ __forceinline__ uint64_t run_pass(const LfArgs& a, const Limits* lim,
 // at most: message c is sent at column c + 1, after column c - 2's return has
 // been waited for.
 //
-// A wait that runs out closes the link for its eight lanes: they send and wait no
-// more, so the messages sent are the first so many of each link. Before the CTAs
-// leave, each tells its neighbours how many it has sent (a plain store, which the
-// cluster barrier orders; it does not order asynchronous ones) and waits for those
-// sent to it that it has not taken in (tests/test_cluster_leave.py runs this under
-// random interleavings).
+// A lane whose wait runs out closes its end of the link: it sends and waits no more,
+// so its shares sent are the first so many messages'. Before the CTAs leave
+// (leave_split), each tells its neighbours how many that was and waits for what was
+// sent to it and not taken in.
 
 struct Link {
   alignas(16) uint8_t inbox[2][64];  // message c in entry c & 1
   uint64_t in_bar[2], ret_bar[2];
-  unsigned sent_in, sent_ret;        // messages and returns sent to this CTA, told at the end
-  int dead;                          // a wait ran out: no further waiting
+  // By lane: messages sent down, returns taken in, messages taken in and returned;
+  // what the neighbours have sent, told at the end.
+  unsigned n_down[LPM], n_back[LPM], n_up[LPM], sent_in[LPM], sent_ret[LPM];
+  int turns;  // polls left for this CTA's waits, in thousands (POLL_TURN)
+  int dead;   // they have run out: a wait's first poll that fails ends it
 };
+constexpr int POLL_TURN = 1024;
 
 __device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint32_t cluster_at(uint32_t at, int rank) {
@@ -910,6 +912,9 @@ __device__ __forceinline__ void send8(uint32_t at, uint2 v, uint32_t bar) {
                "r"(v.x), "r"(v.y), "r"(bar)
                : "memory");
 }
+__device__ __forceinline__ void store_cluster(uint32_t at, unsigned v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
+}
 __device__ __forceinline__ bool message_in(uint32_t bar, unsigned parity) {
   uint32_t done;
   asm volatile(
@@ -920,32 +925,44 @@ __device__ __forceinline__ bool message_in(uint32_t bar, unsigned parity) {
       : "memory");
   return done != 0;
 }
-// Message (or return) m, by an MB's eight lanes; false for all of them when the wait
-// of one ran out (the pass then runs on without that neighbour).
+// Message (or return) m; false when the wait ran out (the pass then runs on without
+// that neighbour). The limit is counted outside the polls' way, in turns: a load of it
+// and a comparison a poll made a 1280x720 pass 162 us instead of 155.
 __device__ __forceinline__ bool wait_message(const LfArgs& a, Link* k, uint64_t* bars, int m) {
   const uint32_t at = smem_at(bars + (m & 1));
-  unsigned long long polls = 0;
-  bool in;
-  while (!(in = message_in(at, (unsigned)(m >> 1) & 1u))) {
+  const unsigned parity = (unsigned)(m >> 1) & 1u;
+#pragma unroll 1
+  for (int polls = 0;;) {
+    if (message_in(at, parity)) return true;
     if (*(volatile int*)&k->dead) break;
-    if (++polls > a.spin_limit) {
-      *(volatile int*)&k->dead = 1;
-      atomicCAS(a.status, 0u, (unsigned)vp8a::DEV_TIMEOUT);
-      break;
+    if (++polls > POLL_TURN) {
+      polls = 0;
+      if (atomicSub(&k->turns, 1) <= 1) *(volatile int*)&k->dead = 1;
     }
   }
-  return __all_sync(((1u << LPM) - 1u) << (threadIdx.x & 31 & ~(LPM - 1)), in);
+  atomicCAS(a.status, 0u, (unsigned)vp8a::DEV_TIMEOUT);
+  return false;
 }
-// The messages `got` .. `sent` - 1, on the way out: they arrive within microseconds.
-__device__ __forceinline__ void await_messages(uint64_t* bars, unsigned got, unsigned sent) {
-  for (; got < sent; got++)
-    for (int polls = 0; polls < 1 << 20 && !message_in(smem_at(bars + (got & 1)), got >> 1 & 1u); polls++) {
+// On the way out: the messages from `got` on of which a lane sent its share (lane q
+// those of the first sent[q]). They arrive within microseconds.
+__device__ __forceinline__ void await_messages(uint64_t* bars, unsigned got, const unsigned* sent) {
+  unsigned most = 0;
+  for (int q = 0; q < LPM; q++) most = max(most, sent[q]);
+  for (; got < most; got++) {
+    const uint32_t at = smem_at(bars + (got & 1));
+    unsigned missing = 0;
+    for (int q = 0; q < LPM; q++) missing += sent[q] <= got ? 8u : 0u;
+    if (missing)
+      asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(at), "r"(missing) : "memory");
+    for (int polls = 0; polls < 1 << 20 && !message_in(at, got >> 1 & 1u); polls++) {
     }
+  }
 }
 
-__device__ __forceinline__ void init_link(Link* k) {
-  k->dead = 0;
-  k->sent_in = k->sent_ret = 0;
+__device__ __forceinline__ void init_link(Link* k, unsigned limit) {
+  k->turns = (int)(limit / POLL_TURN) + 1;
+  k->dead = limit == 0;
+  for (int q = 0; q < LPM; q++) k->sent_in[q] = k->sent_ret[q] = 0;
   for (int i = 0; i < 2; i++) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(&k->in_bar[i])) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(&k->ret_bar[i])) : "memory");
@@ -994,10 +1011,9 @@ __device__ __forceinline__ uint64_t run_split(const LfArgs& a, const Limits* lim
   }
   uint64_t total = 0;
   LaneRows<LUMA> rec, src, fin;
-  // The links as this lane's MB serves them: open; messages sent down, returns taken
-  // in; messages taken in from above, each returned.
-  bool down = hand_down, up = handed;
-  unsigned n_down = 0, n_back = 0, n_up = 0;
+  bool down = hand_down, up = handed;  // this lane's ends of the links are open
+  if (down) link->n_down[q] = link->n_back[q] = cols;
+  if (up) link->n_up[q] = cols;
   unsigned info = 0;
   int slot = 0;  // c % RING
   auto fetch = [&](int c) {
@@ -1021,9 +1037,14 @@ __device__ __forceinline__ uint64_t run_split(const LfArgs& a, const Limits* lim
     if (live && c >= RING) {
       // MB (r, c - RING) is final (its last rows back from the next CTA).
       const int f = c - RING;
-      if (down && (down = wait_message(a, link, link->ret_bar, f))) {
-        if (q == 0) expect_message(&link->ret_bar[f & 1]);
-        n_back++;
+      if (down) {
+        if (!wait_message(a, link, link->ret_bar, f)) {
+          down = false;
+          link->n_down[q] = min(c - 1, cols);
+          link->n_back[q] = f;
+        } else if (q == 0) {
+          expect_message(&link->ret_bar[f & 1]);
+        }
       }
       if (score) {
         total += f < whole_cols ? score_mb<LUMA>(me, q, src)
@@ -1042,17 +1063,18 @@ __device__ __forceinline__ uint64_t run_split(const LfArgs& a, const Limits* lim
       else vertical_edges<LUMA, SIMPLE, false>(rec, me, set + left_at, q, c > 0, L, kleft, kinner);
     }
     __syncwarp();
-    if (down && c >= 1 && c <= cols) {
+    if (down && c >= 1 && c <= cols)
       send8(down_inbox + ((c - 1) & 1) * 64, *(const uint2*)(set + left_at + Geo<LUMA>::tail_off(q)),
             down_bar + ((c - 1) & 1) * 8);
-      n_down++;
-    }
     fetch(c + 1);
     if (written) store_rows<LUMA>(op + (c - RING) * ROWB, out.half, a.recon_align, fin);
     __syncthreads();
     if (main) {
       uint8_t* msg = link->inbox[c & 1];
-      if (up) up = wait_message(a, link, link->in_bar, c);
+      if (up && !wait_message(a, link, link->in_bar, c)) {
+        up = false;
+        link->n_up[q] = c;
+      }
       uint8_t* above = handed ? msg + Geo<LUMA>::msg_col(q) : up_set + slot * SLOT + LAST + Geo<LUMA>::col_off(q);
       const uint32_t ktop = top ? L.flat : DISABLED;
       if (full) horizontal_edges<LUMA, SIMPLE, true>(me, above, q, top, L, ktop, kinner);
@@ -1062,19 +1084,33 @@ __device__ __forceinline__ uint64_t run_split(const LfArgs& a, const Limits* lim
         const uint2 v = *(const uint2*)(msg + q * 8);
         if (q == 0) expect_message(&link->in_bar[c & 1]);
         send8(up_rings + slot * SLOT, v, up_bar + (c & 1) * 8);
-        n_up++;
       }
     }
     slot = c < 0 ? 0 : (slot == RING - 1 ? 0 : slot + 1);
     __syncthreads();
   }
-  cg::cluster_group cl = cg::this_cluster();
-  if (hand_down && q == 0) *cl.map_shared_rank(&link->sent_in, rank + 1) = n_down;
-  if (handed && q == 0) *cl.map_shared_rank(&link->sent_ret, rank - 1) = n_up;
-  cl.sync();
-  if (handed && q == 0) await_messages(link->in_bar, n_up, link->sent_in);
-  if (hand_down && q == 0) await_messages(link->ret_bar, n_back, link->sent_ret);
   return total;
+}
+
+// The end of a split pass. A CTA's shared memory must not go away under a message on
+// its way to it, and a cluster barrier does not order asynchronous stores: it orders
+// the plain ones that tell each neighbour how many messages it was sent. Nothing is
+// left to wait for unless a wait ran out (tests/test_cluster_leave.py runs this under
+// random interleavings). Written with the instructions themselves and apart from
+// run_split: through cooperative groups' remote pointer and barrier a 1280x720 pass
+// took 170 us instead of 158, every step of it slower.
+__device__ __forceinline__ void leave_split(const LfArgs& a, Link* link, int rank) {
+  const Rows R(a, 2);
+  const int g = threadIdx.x / LPM, q = threadIdx.x & (LPM - 1);
+  const int s0 = rank_row(a.n_scored, a.split, rank), s1 = rank_row(a.n_scored, a.split, rank + 1);
+  const bool handed = g == 0 && s0 < s1 && R.top(s0);
+  const bool hand_down = s0 + g == s1 - 1 && s1 < a.n_scored && R.top(s1);
+  if (hand_down) store_cluster(cluster_at(smem_at(&link->sent_in[q]), rank + 1), link->n_down[q]);
+  if (handed) store_cluster(cluster_at(smem_at(&link->sent_ret[q]), rank - 1), link->n_up[q]);
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (handed && q == 0) await_messages(link->in_bar, link->n_up[0], link->sent_in);
+  if (hand_down && q == 0) await_messages(link->ret_bar, link->n_back[0], link->sent_ret);
 }
 
 // LoopFilterParams::derive (src/loop_filter.rs:99-148) for every filter
@@ -1121,7 +1157,7 @@ __device__ __forceinline__ void sweep_body(const LfArgs& a, int cta, int np) {
     if constexpr (BOTH && SIMPLE) class_limits<SIMPLE>(a, lv, sh, false, lim_c);
     if (threadIdx.x == 0) {
       taken[0] = blockDim.x >> 5;
-      if constexpr (CL) init_link(&link);
+      if constexpr (CL) init_link(&link, a.spin_limit);
     }
     if constexpr (CL) cg::this_cluster().sync();
     else __syncthreads();
@@ -1130,6 +1166,7 @@ __device__ __forceinline__ void sweep_body(const LfArgs& a, int cta, int np) {
     if constexpr (CL) {
       v = luma ? run_split<true, SIMPLE>(a, lim, rings, &link, rank)
                : run_split<false, SIMPLE>(a, lim, rings, &link, rank);
+      leave_split(a, &link, rank);
     } else if constexpr (BOTH) {
       PlanePass<true, SIMPLE, TILED> y(a, rings, q);
       PlanePass<false, SIMPLE, TILED> c(a, rings + a.n_sets * Geo<true>::SET, q);
@@ -1283,7 +1320,7 @@ vp8a_status stage_lf(vp8a_ctx* ctx, vp8a::Stager& st, const vp8a_planes* planes,
   a.mbs = (const vp8a_mb_lf_info*)d;
   a.base = *base;
   a.status = ctx->d_status;
-  a.spin_limit = ctx->wait_limit;
+  a.spin_limit = (unsigned)std::min<uint64_t>(ctx->wait_limit, 0xffffffffu);
   if (src) {
     if (src->width == 0 || src->height == 0 || src->width > (uint32_t)cols * 16 ||
         src->height > (uint32_t)rows * 16) {
