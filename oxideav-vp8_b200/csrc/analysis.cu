@@ -967,6 +967,12 @@ __device__ __forceinline__ void main_sync() { asm volatile("bar.sync 1, %0;" ::"
 __device__ __forceinline__ void search_sync() { asm volatile("bar.sync 2, %0;" ::"n"(AN_THREADS) : "memory"); }
 static_assert(MAIN_THREADS >= 16 * FN, "one thread per field task");
 
+// The cluster's barrier for leaving.
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // What a CTA's helper warp and its cluster hand it, MB by MB (n counts the
 // MBs the cluster has taken): the source MB and the census record of the MB
 // above, fetched two MBs ahead, and every reference's decision. The decisions
@@ -1065,8 +1071,7 @@ __device__ void run_helper(Feed& F, const AnArgs& a0, const AnArgs* jobs, const 
   unsigned n_pre = 0, n_pub = 0;
   unsigned long long polls = 0;
   unsigned idle = 0;
-  bool stop = false;
-  while (pub.job && !stop) {
+  while (pub.job) {
     bool moved = false;
     // MB n_pub decided everywhere?
     if (__all_sync(FULL, bar_done(&F.dec_bar[n_pub % DEC_RING], n_pub / DEC_RING & 1u))) {
@@ -1135,8 +1140,13 @@ __device__ void run_helper(Feed& F, const AnArgs& a0, const AnArgs* jobs, const 
       }
     }
     if (!moved) {
-      stop = (++idle & 15u) == 0 && __any_sync(FULL, *(volatile unsigned*)pub.job->status != 0u);
-      if (stop && lane == 0) *(volatile int*)&F.stop = 1;
+      if ((++idle & 15u) == 0 && __any_sync(FULL, *(volatile unsigned*)pub.job->status != 0u)) {
+        if (lane == 0) {
+          F.n_pub = n_pub;
+          *(volatile int*)&F.stop = 1;
+        }
+        return;
+      }
       __nanosleep(40);
     }
   }
@@ -1235,12 +1245,21 @@ __global__ void __launch_bounds__(AN_THREADS + 32, 2)
 
   if (warp == NW) {
     run_helper<BATCH>(feed, a0, jobs, items, n_it, cid, n_clusters, k, lane);
-    __syncwarp();
-    cl.sync();
+    cluster_sync();
     return;
   }
-  bool stopped = false;
-  for (int it = cid; it < n_it && !stopped; it += n_clusters) {
+  // A copy of its own at both ways out: with one that both run into, a 1920x1080
+  // analysis took 1.68 ms instead of 1.66.
+  auto leave = [&]() {
+    if (tid < csize) {
+      uint32_t at;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_at(&feed.sent[k])), "r"(tid));
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(n) : "memory");
+    }
+    cluster_sync();
+    if (tid == 0) await_decisions(feed, csize);
+  };
+  for (int it = cid; it < n_it; it += n_clusters) {
     int r = it, job = 0;
     if (BATCH) {
       const uint32_t w = items[it];
@@ -1352,8 +1371,8 @@ __global__ void __launch_bounds__(AN_THREADS + 32, 2)
       }
       search_sync();
       if (s_stop) {
-        stopped = true;
-        break;
+        leave();
+        return;
       }
       stage_ref(P, R, plan, mbx, mby, a.words, tid, AN_THREADS);
       search_sync();
@@ -1664,9 +1683,7 @@ __global__ void __launch_bounds__(AN_THREADS + 32, 2)
       }
     }
   }
-  if (tid < csize) *cl.map_shared_rank(&feed.sent[k], tid) = n;
-  cl.sync();
-  if (tid == 0) await_decisions(feed, csize);
+  leave();
 }
 
 }  // namespace

@@ -113,9 +113,11 @@ def analysis(n_ctas, mbs, cols, seed, awaits, ring):
 def analysis_constants():
     text = source("analysis.cu")
     kernel = text[text.index("analysis_kernel(const __grid_constant__"):]
-    barrier = kernel.rindex("cl.sync();", 0, kernel.index("kDefaultMvContexts"))
-    tail = kernel[barrier:kernel.index("kDefaultMvContexts")]
-    return "await_decisions(" in tail, int(re.search(r"DEC_RING = (\d+);", text).group(1))
+    leave = kernel[kernel.index("auto leave = ["):kernel.index("  };")]
+    awaits = leave.index("cluster_sync();") < leave.index("await_decisions(")
+    # Both ways out: stopping, and the end of the kernel.
+    awaits = awaits and kernel.count("leave();") == 2 and "leave();\n}" in kernel and "leave();\n        return;" in kernel
+    return awaits, int(re.search(r"DEC_RING = (\d+);", text).group(1))
 
 
 @pytest.mark.parametrize("n_ctas", [1, 2, 3])
