@@ -1494,6 +1494,30 @@ template <int C>
 constexpr int THREADS_OF = 32 * (WARPS_OF<C> + C);  // + loads, + db (C = 2)
 }  // namespace lpdws
 
+// One half image of dW of the last layer at (channel, tap), pixel by pixel, added to
+// `sum`. A matrix instruction multiplies every X of its tile with every column's dY, a
+// halo's zeros among them, which an infinity or NaN in X would turn into NaN where
+// that pixel and tap have no pixel of dY between them; and a pixel of dY whose own X
+// lies outside does not count there, where the element-wise kernel multiplies it with
+// a zero. So a half image that leaves a tile's sums not finite is summed this way
+// instead, as the element-wise kernel's zeros have it.
+__device__ __noinline__ float lp_edge_sum(const uint8_t* xt, const uint16_t* small, int half, int ch, int tap,
+                                          float sum) {
+  constexpr int RP = 32 + 16;
+  const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+  auto in = [](int v) { return v >= 0 && v < 32; };
+  auto value = [](uint16_t b) { return __uint_as_float((uint32_t)b << 16); };
+#pragma unroll 1
+  for (int p = 0; p < 512; p++) {
+    const int r = p >> 5, x = p & 31, y = half * 16 + r;
+    if (in(y - dy) && in(x - dx))
+      sum += value(*reinterpret_cast<const uint16_t*>(xt + lptrain::swz(p, ch >> 3) + (ch & 7) * 2)) *
+             value(small[(r + 1 - dy) * RP + 8 + x - dx]);
+    if (!in(y + dy) || !in(x + dx)) sum += value(small[(r + 1) * RP + 8 + x]) * 0.f;
+  }
+  return sum;
+}
+
 template <int C>
 __global__ void __launch_bounds__(lpdws::THREADS_OF<C>, 2)
     lp_conv_bwd_w_edge_kernel(const __grid_constant__ CUtensorMap tm32, const __grid_constant__ CUtensorMap tms, int n,
@@ -1551,8 +1575,9 @@ __global__ void __launch_bounds__(lpdws::THREADS_OF<C>, 2)
   } else {
     const int m = warp & 1, i = warp >> 1;  // 16 channels, 8 columns
     const int pa = (lane & 7) + ((lane >> 4) & 1) * 8, ca = ((lane >> 3) & 1) + 2 * m;
-    // This lane's column's element at pixel 2 t of a row's first 16.
-    const int nn = i * 8 + g < N ? i * 8 + g : 0, tap = nn / C;
+    // This lane's column's element at pixel 2 t of a row's first 16 (columns past N,
+    // not stored, take the middle tap's).
+    const int nn = i * 8 + g < N ? i * 8 + g : N / 2, tap = nn / C;
     const int nb = (1 + S * (tap / 3 - 1)) * RP + 8 + (2 * t + S * (tap % 3 - 1)) * C + nn % C;
     float bs = 0.f;  // C = 1: db
     for (int i0 = first; i0 < items && ok; i0 += stride) {
@@ -1563,6 +1588,7 @@ __global__ void __launch_bounds__(lpdws::THREADS_OF<C>, 2)
         if (!ok) break;
         const uint32_t as = base + (uint32_t)(s * STAGE);
         const uint16_t* small = reinterpret_cast<const uint16_t*>(sm + s * STAGE + HALF_BYTES);
+        const float before[4] = {acc[0], acc[1], acc[2], acc[3]};
         // Four steps' fragments load while the four before run.
         uint32_t a[2][4][4], b[2][4][2];
         auto load = [&](int v) {
@@ -1586,6 +1612,19 @@ __global__ void __launch_bounds__(lpdws::THREADS_OF<C>, 2)
             const int k = v * 4 + w;
             if (C == 1 && lane < 16 && warp == w)
               bs += __uint_as_float((uint32_t)small[((k >> 1) + 1) * RP + 8 + (k & 1) * 16 + lane] << 16);
+          }
+        }
+        if (C == 1) {
+          // Every not finite element reaches the sums of its channel's row or, through
+          // the middle tap, a column of every tile.
+          const float most = fmaxf(fmaxf(fabsf(acc[0]), fabsf(acc[1])), fmaxf(fabsf(acc[2]), fabsf(acc[3])));
+          const bool nan = acc[0] != acc[0] || acc[1] != acc[1] || acc[2] != acc[2] || acc[3] != acc[3];
+          if (__any_sync(FULL, nan || most == INFINITY)) {
+#pragma unroll
+            for (int f = 0; f < 4; f++) {
+              const int c = i * 8 + 2 * t + (f & 1);
+              acc[f] = lp_edge_sum(sm + s * STAGE, small, it & 1, m * 16 + g + 8 * (f >> 1), c < N ? c : N / 2, before[f]);
+            }
           }
         }
         __syncwarp();
