@@ -11,7 +11,7 @@
 
 #include "../../include/vp8a.h"
 
-#define VP8A_ABI_VERSION ((1u << 16) | 1u)  /* 1.1: the bitstream writer */
+#define VP8A_ABI_VERSION ((1u << 16) | 2u)  /* 1.1: the bitstream writer; 1.2: vp8a_encode_inter_frame */
 
 // ----------------------------------------------------------------- context
 struct vp8a_ctx {
