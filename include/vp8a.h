@@ -884,9 +884,11 @@ vp8a_status vp8a_write_inter_frame(const vp8a_frame_header* header,
  * `proposals`, optional, as vp8a_analyse_inter_frame_proposals takes them),
  * vp8a_reconstruct_inter_frame, with `auto_lf` vp8a_select_filter_params (else
  * the header's level and sharpness), vp8a_filter_frame into `filtered` when the
- * level is not 0, and vp8a_write_inter_frame, with the same results. Every
- * buffer but `proposals` is host memory, no output overlaps an input;
- * segmentation is off. Returns
+ * level is not 0, and vp8a_write_inter_frame, with the same results. The
+ * header's loop-filter deltas, when enabled, are the ones in effect: the
+ * filter applies them whether they are sent or not. Every buffer but
+ * `proposals` is host memory, no output overlaps an input and nothing is
+ * written between the rows of an output plane; segmentation is off. Returns
  * VP8A_E_INVALID_ARGUMENT with *out_size > out_capacity when `out` is too small
  * (the other outputs are written). */
 vp8a_status vp8a_encode_inter_frame(vp8a_ctx* ctx, const vp8a_i420* frame, const vp8a_planes* refs,

@@ -252,6 +252,16 @@ vp8a_status encode(vp8a_ctx* ctx, const vp8a_i420* frame, const vp8a_planes* ref
   cfg.loop_filter_level = h.loop_filter_level;
   cfg.sharpness_level = h.sharpness_level;
   cfg.simple = h.filter_type;
+  // The header's deltas, as a decoder of the frame adds them.
+  cfg.delta_enabled = h.lf_delta_enabled;
+  cfg.ref_delta_current = h.lf_ref_delta[0];
+  cfg.ref_delta_last = h.lf_ref_delta[1];
+  cfg.ref_delta_golden = h.lf_ref_delta[2];
+  cfg.ref_delta_altref = h.lf_ref_delta[3];
+  cfg.bpred_mode_delta = h.lf_mode_delta[0];
+  cfg.zero_mv_mode_delta = h.lf_mode_delta[1];
+  cfg.other_mv_mode_delta = h.lf_mode_delta[2];
+  cfg.split_mv_mode_delta = h.lf_mode_delta[3];
   if (auto_lf) {
     vp8a_filter_config base = cfg;
     base.loop_filter_level = 0;

@@ -20,13 +20,13 @@ def surfaces(ref, pad):
     return whole, [s[:, :p.shape[1]] for s, p in zip(whole, ref)]
 
 
-def encode(ctx, frame, refs, qi, level, auto_lf, recon, filtered, out, capacity):
+def encode(ctx, frame, refs, qi, level, auto_lf, recon, filtered, out, capacity, **header):
     n = refs[0][0].size // 256
     dec, lf = np.zeros(n, abi.MB_DECISION_DTYPE), np.zeros(n, abi.MB_LF_INFO_DTYPE)
     cf, fl = np.zeros((n, 400), np.int16), np.zeros(n, np.uint8)
     pl = (abi.Planes * len(refs))(*[vp8a.planes(*r) for r in refs])
     ids = np.array([1, 2, 3][:len(refs)], np.uint8)
-    hdr = abi.frame_header(frame[0].shape[1], frame[0].shape[0], abi.quant_indices(qi), loop_filter_level=level)
+    hdr = abi.frame_header(frame[0].shape[1], frame[0].shape[0], abi.quant_indices(qi), loop_filter_level=level, **header)
     lv, sh, size = C.c_uint8(), C.c_uint8(), C.c_uint64()
     st = ctx._lib.vp8a_encode_inter_frame(
         ctx.handle, C.byref(vp8a.i420(*frame)), C.cast(pl, C.c_void_p), ids.ctypes.data, len(refs),
@@ -71,3 +71,29 @@ def test_a_short_buffer_is_not_overrun(ctx, capacity):
     st, size, lv, _ = encode(ctx, frame, refs, 4, 0, True, recon, filtered, out, capacity)
     assert st == abi.E_INVALID_ARGUMENT and size == len(want_bits) and (out[capacity:] == FILL).all()
     assert lv == d["level"] and all(np.array_equal(a, b) for a, b in zip(recon, d["recon"]))
+
+
+@pytest.mark.parametrize("level,auto_lf", [(30, False), (0, True)])
+def test_the_headers_filter_deltas_are_applied(ctx, level, auto_lf):
+    # What a decoder of the frame adds to its levels, the call's own filter adds.
+    deltas = dict(lf_delta_enabled=1, lf_delta_update=1, lf_ref_delta_present=15, lf_mode_delta_present=15,
+                  lf_ref_delta=[2, 9, -14, 6], lf_mode_delta=[4, -12, -2, 11])
+    frame, refs = case(208, 144, 3)
+    (_, recon), (_, filtered) = surfaces(refs[0], 0), surfaces(refs[0], 0)
+    out = np.zeros(60000, np.uint8)
+    st, size, lv, (dec, cf, fl, lf) = encode(ctx, frame, refs, 60, level, auto_lf, recon, filtered, out, out.size,
+                                             **deltas)
+    assert st == abi.OK
+    r, m = deltas["lf_ref_delta"], deltas["lf_mode_delta"]
+    cfg = lambda lv, sh: abi.filter_config(  # noqa: E731
+        lv, sh, delta_enabled=1, ref_delta_current=r[0], ref_delta_last=r[1], ref_delta_golden=r[2],
+        ref_delta_altref=r[3], bpred_mode_delta=m[0], zero_mv_mode_delta=m[1], other_mv_mode_delta=m[2],
+        split_mv_mode_delta=m[3])
+    sh = 0
+    if auto_lf:
+        level, sh = vp8a.select_filter_params(ctx, recon, lf, cfg(0, 0), frame)
+    assert lv == level > 0
+    for got, want in zip(filtered, vp8a.filter_frame(ctx, recon, lf, cfg(level, sh))):
+        assert np.array_equal(got, want)
+    hdr = abi.frame_header(208, 144, abi.quant_indices(60), loop_filter_level=level, sharpness_level=sh, **deltas)
+    assert out[:size].tobytes() == vp8a.write_inter_frame(hdr, dec, cf)
