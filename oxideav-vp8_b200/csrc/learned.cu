@@ -1927,13 +1927,12 @@ vp8a_status encode_map(const uint16_t* x, int rank, const cuuint64_t* dim, const
 }
 
 // The TMA map of n NHWC [32][32][32] BF16 images: a 4-D tensor (channel, x, y,
-// image) with boxes of `ch` channels (8 unswizzled, 32 with the 64-byte
-// swizzle) x w x h x 1.
-vp8a_status image_map(const uint16_t* x, uint32_t n, uint32_t ch, uint32_t w, uint32_t h, CUtensorMap* tm) {
+// image) with boxes of 32 channels x w x h x 1 in the 64-byte swizzle.
+vp8a_status image_map(const uint16_t* x, uint32_t n, uint32_t w, uint32_t h, CUtensorMap* tm) {
   const cuuint64_t dim[4] = {32, 32, 32, n};
   const cuuint64_t stride[3] = {32 * 2, 32 * 32 * 2, 32 * 32 * 32 * 2};  // bytes, dims 1..3
-  const cuuint32_t box[4] = {ch, w, h, 1};
-  return encode_map(x, 4, dim, stride, box, ch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE, tm);
+  const cuuint32_t box[4] = {32, w, h, 1};
+  return encode_map(x, 4, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_64B, tm);
 }
 
 // The TMA map of n NHWC [32][32][C] images as (x * C + c, y, image): boxes of 18
@@ -1956,7 +1955,7 @@ template <bool BWD>
 vp8a_status conv_tc(vp8a_ctx* ctx, const uint16_t* a, const uint16_t* W, const float* bias, int n, int relu,
                     const uint16_t* Xa, uint16_t* Y) {
   CUtensorMap tm;
-  vp8a_status s = image_map(a, (uint32_t)n, 32, 34, 34, &tm);
+  vp8a_status s = image_map(a, (uint32_t)n, 34, 34, &tm);
   if (s == VP8A_OK) s = use_smem(lp_conv_tc_kernel<BWD>, lptc3::SMEM);
   if (s != VP8A_OK) return s;
   lp_conv_tc_kernel<BWD><<<std::min(n, ctx->sm_count), lptc3::THREADS, lptc3::SMEM, ctx->stream>>>(
@@ -1969,7 +1968,7 @@ vp8a_status conv_tc(vp8a_ctx* ctx, const uint16_t* a, const uint16_t* W, const f
 vp8a_status conv_last(vp8a_ctx* ctx, const uint16_t* X, const uint16_t* W, const float* bias, int n, int relu,
                       float* Y) {
   CUtensorMap tm;
-  vp8a_status s = image_map(X, (uint32_t)n, 32, 34, 34, &tm);
+  vp8a_status s = image_map(X, (uint32_t)n, 34, 34, &tm);
   if (s == VP8A_OK) s = use_smem(lp_conv_last_kernel, lplast::SMEM);
   if (s != VP8A_OK) return s;
   lp_conv_last_kernel<<<std::min(n, ctx->sm_count), lplast::THREADS, lplast::SMEM, ctx->stream>>>(
@@ -1987,8 +1986,8 @@ vp8a_status conv_bwd_w_32(vp8a_ctx* ctx, const uint16_t* dY, const uint16_t* X, 
   const int groups = (2 * n + LP_WCPB - 1) / LP_WCPB;
   const bool split = 3 * groups <= ctx->sm_count;
   const auto kernel = split ? lp_conv_bwd_w_kernel<1> : lp_conv_bwd_w_kernel<3>;
-  vp8a_status s = image_map(X, (uint32_t)n, 32, 34, 18, &tmx);
-  if (s == VP8A_OK) s = image_map(dY, (uint32_t)n, 32, 32, 16, &tmd);
+  vp8a_status s = image_map(X, (uint32_t)n, 34, 18, &tmx);
+  if (s == VP8A_OK) s = image_map(dY, (uint32_t)n, 32, 16, &tmd);
   if (s == VP8A_OK) s = use_smem(kernel, lpdw::SMEM);
   if (s != VP8A_OK) return s;
   kernel<<<dim3(std::min(groups, ctx->sm_count), split ? 3 : 1), lpdw::THREADS, lpdw::SMEM, ctx->stream>>>(
@@ -2002,7 +2001,7 @@ template <int C>
 vp8a_status conv_bwd_w_edge(vp8a_ctx* ctx, const uint16_t* t32, const uint16_t* small, int n, float* dW, float* db) {
   CUtensorMap tm, tms;
   const int groups = (2 * n + LP_WCPB - 1) / LP_WCPB;
-  vp8a_status s = image_map(t32, (uint32_t)n, 32, 32, 16, &tm);
+  vp8a_status s = image_map(t32, (uint32_t)n, 32, 16, &tm);
   if (s == VP8A_OK) s = row_map(small, (uint32_t)n, C, &tms);
   if (s == VP8A_OK) s = use_smem(lp_conv_bwd_w_edge_kernel<C>, lpdws::SMEM);
   if (s != VP8A_OK) return s;

@@ -61,9 +61,11 @@ __device__ __forceinline__ uint32_t pk16(int v) { return (uint32_t)(uint16_t)(in
 // Bytes 1 and 3 as fields.
 __device__ __forceinline__ uint32_t odd_bytes(uint32_t x) { return __byte_perm(x, 0u, 0x4341); }
 // (t >> 7) - 64 clamped to 0..255, per field: t is the filter's sum plus 64 + 64 *
-// 128, which keeps every field in 0..65535 (the taps' negative sums exceed -19 *
-// 255, the positive ones stay below 160 * 255).
+// 128. The taps' negative sums reach -32 * 255 and the positive ones 160 * 255 (the
+// half-pel taps both), so every field lies in 96 .. 49056 and takes nothing from its
+// neighbour.
 constexpr int TAP_BIAS = 64 + 64 * 128;
+static_assert(TAP_BIAS - 32 * 255 >= 0 && TAP_BIAS + 160 * 255 <= 0xffff, "sums stay in their fields");
 __device__ __forceinline__ uint32_t tap_result(uint32_t t) {
   return __viaddmin_s16x2_relu((t >> 7) & 0x01ff01ffu, pk16(-64), pk16(255));
 }
