@@ -717,9 +717,9 @@ typedef struct vp8a_sweep_job {
   uint64_t* ssd_out;  /* 512 entries, level * 8 + sharpness */
 } vp8a_sweep_job;
 
-/* vp8a_filter_sweep for every job: the (job, candidate) pairs of all jobs
- * in one launch when every job's slot rings fit in shared memory (the
- * larger pictures otherwise run as their own launches). */
+/* vp8a_filter_sweep for every job: the (job, candidate) pairs of the jobs
+ * of one launch shape and size class in one launch, the largest pictures
+ * first. */
 vp8a_status vp8a_filter_sweeps(vp8a_ctx* ctx, const vp8a_sweep_job* jobs, uint32_t n_jobs);
 
 /* select_filter_params (src/loop_filter.rs:2047) for every job: the

@@ -9,9 +9,11 @@
 // on a second stream while it runs), the caller's output pages are touched
 // meanwhile, decisions, coefficients and the reconstruction come down on the second
 // stream while the device chooses the loop-filter level, and a thread codes the
-// token partitions, which do not depend on that level. Measured at 640x360
-// (QI 56, three references): stage by stage through host buffers 2.51 ms, 1.35 ms
-// so; 1920x1080 9.6 and 4.7 ms, 3840x2160 25.7 and 14.0 ms.
+// token partitions, which do not depend on that level. Measured through
+// encode_p_frame (QI 56, three references, the same planes again and again): stage
+// by stage through host buffers 2.5 ms at 640x360, 1.43 ms so; 1920x1080 12.8 and
+// 5.9-6.6 ms, 3840x2160 40 and 21.6 ms. (On a faster host 9.6 and 4.7, 25.7 and 14.0;
+// the first frames from planes never seen before take 0.2 ms longer at 640x360.)
 #include <algorithm>
 #include <cstring>
 #include <exception>
