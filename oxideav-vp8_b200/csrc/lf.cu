@@ -1380,27 +1380,33 @@ size_t ring_bytes(const LfArgs& a, bool both) {
 constexpr size_t MAX_RING_BYTES = 220 << 10, CTA_SMEM = 2304;
 
 // What a launch of `candidates` per picture takes, in seconds, whole or split
-// (fits of measured launches, 176x144 to 3840x2160). Whole passes: 0.36 ns per
-// MB and candidate, but no less than one pass's chain of steps, whose step
-// grows with the MBs that the CTA's warps take one after another (one pass
-// alone, 1080p: 0.76 ms for 257 steps). Split passes: a step of 1.1 us whatever
-// the picture (0.22 ms), and 2.7 times the work (half of the lanes wait for
-// inner edges that their own MB does not have).
+// (fits of measured launches, 176x144 to 3840x2160 and 32x4096 to 4096x128). Whole
+// passes: 0.36 ns per MB and candidate, but no less than one pass's chain of steps,
+// whose step grows with the rows that are busy at once and so with the MBs that the
+// CTA's warps take one after another (one pass alone, 1080p: 0.76 ms for 257 steps).
+// Split passes: a step of 1.1 us whatever the picture (0.22 ms), 2.7 times the work
+// (half of the lanes wait for inner edges that their own MB does not have), and
+// every CTA stays for all the steps, 16 threads a row of the 512 that an SM holds,
+// though in a tall and narrow picture few steps have work for it (128x4096, the whole
+// grid: 6.6 ms split, 0.8 ms whole; one frame's filter 0.3 and 0.8).
 double whole_time(const std::vector<LfArgs*>& jobs, double candidates) {
   double chain = 0, mbs = 0;
   for (const LfArgs* a : jobs) {
-    chain = std::max(chain, (skew_of(1) * a->max_t0 + a->mb_cols) * (0.9e-6 + 0.027e-6 * a->n_scored));
+    chain = std::max(chain, (skew_of(1) * a->max_t0 + a->mb_cols) * (0.9e-6 + 0.0296e-6 * active_rows(*a, 1)));
     mbs += (double)a->n_scored * a->mb_cols;
   }
   return std::max(chain, 0.36e-9 * candidates * mbs);
 }
 double split_time(const std::vector<LfArgs*>& jobs, double candidates) {
-  double chain = 0, mbs = 0;
+  constexpr double THREADS = 148 * max_threads(true, false);
+  double chain = 0, mbs = 0, stay = 0;
   for (const LfArgs* a : jobs) {
-    chain = std::max(chain, (skew_of(2) * a->max_t0 + a->mb_cols) * 1.1e-6);
+    const double c = (skew_of(2) * a->max_t0 + a->mb_cols) * 1.1e-6;
+    chain = std::max(chain, c);
     mbs += (double)a->n_scored * a->mb_cols;
+    stay += c * 2 * LPM * a->n_scored;
   }
-  return std::max(chain, 0.97e-9 * candidates * mbs);
+  return std::max({chain, 0.97e-9 * candidates * mbs, candidates * stay / THREADS});
 }
 
 // CTAs per pass for a call whose largest launch has `candidates` per picture:
