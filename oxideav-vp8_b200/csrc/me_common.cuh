@@ -114,8 +114,10 @@ __device__ __forceinline__ bool word_plane(const MePlane& P) {
 }
 
 // Fill a WS x WS window whose top-left is plane pixel (x0, y0), clamping
-// every coordinate into the plane: word by word where a row's words lie
-// inside it, byte by byte at the edges.
+// every coordinate into the plane: words where they lie inside it, at the edges
+// too. (Byte loads for a whole window at an edge, a row at a time, made a
+// three-reference search of a 16x16 frame at the fastest effort 62 us instead of 54,
+// and of a 1920x1080 frame at the middle effort 161 instead of 149.)
 __device__ __forceinline__ void load_window(const MePlane& P, uint8_t* win, int x0, int y0, int lane) {
   if (word_plane(P) && x0 >= 0 && (x0 & ~3) + WS + 4 <= P.width) {
     const int sh = x0 & 3, xa = x0 - sh;
@@ -127,10 +129,21 @@ __device__ __forceinline__ void load_window(const MePlane& P, uint8_t* win, int 
     __syncwarp();
     return;
   }
-  for (int r = 0; r < WS; r++) {
-    int y = clampi(y0 + r, 0, P.height - 1);
-    const uint8_t* row = P.plane + (size_t)y * P.stride;
-    for (int c = lane; c < WS; c += 32) win[r * WS + c] = row[clampi(x0 + c, 0, P.width - 1)];
+  // Four words a lane in flight.
+  const bool words = word_plane(P);
+#pragma unroll 4
+  for (int t = lane; t < WS * (WS / 4); t += 32) {
+    const int r = t / (WS / 4), w = t - r * (WS / 4), x = x0 + 4 * w, sh = x & 3;
+    const uint8_t* row = P.plane + (size_t)clampi(y0 + r, 0, P.height - 1) * P.stride;
+    uint32_t v = 0;
+    if (words && x >= 0 && x - sh + 8 <= P.width) {
+      const uint32_t* p = (const uint32_t*)(row + (x - sh));
+      v = __funnelshift_r(__ldg(p), __ldg(p + 1), 8u * (unsigned)sh);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++) v |= (uint32_t)row[clampi(x + k, 0, P.width - 1)] << (8 * k);
+    }
+    *(uint32_t*)(win + r * WS + 4 * w) = v;
   }
   __syncwarp();
 }
